@@ -1,0 +1,71 @@
+"""The native call path of bound layers: what it serves itself and what it hands to the Python callable."""
+
+from __future__ import annotations
+
+import gc
+import weakref
+
+import pytest
+import torch
+
+from conftest import seeded
+from xqt_b200 import quantize
+from xqt_b200.errors import XQTBackendError
+from xqt_b200.ops import w8a8
+from xqt_b200.ops.mlp import W4A16SwiGLUMLP
+from xqt_b200.ops.w4a16 import bind_w4a16_decode, prepare_decode
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda", 0)
+
+
+def _layer(n, k, seed):
+    return quantize.quantize_w4_asymmetric((torch.randn((n, k), generator=seeded(seed)) * 0.02).to(DEV), group_size=128)
+
+
+@pytest.mark.parametrize("m", [1, 16])
+def test_decode_call_forms(m):
+    n, k = 264, 256
+    w = _layer(n, k, 1)
+    run = bind_w4a16_decode(prepare_decode(w.qweight, w.scales, w.zero_points, group_size=128, nibble_signed=False), rows=m, dtype=torch.bfloat16)
+    x = torch.randn((m, k), generator=seeded(2)).to(DEV, torch.bfloat16)
+    residual = torch.randn((m, n), generator=seeded(3)).to(DEV, torch.bfloat16)
+    plain = run(x)
+    out = torch.empty_like(plain)
+    assert run(x, out) is out and torch.equal(out, plain)
+    assert torch.equal(run(x, out=out), plain) and torch.equal(run(x, None, residual), run.slow(x, None, residual))
+    other = torch.cuda.Stream(DEV)
+    other.wait_stream(torch.cuda.current_stream(DEV))
+    with torch.cuda.stream(other):
+        again = run(x)
+    torch.cuda.current_stream(DEV).wait_stream(other)
+    assert torch.equal(again, plain)
+    for bad in (x.to(torch.float16), x[:, :128], x.cpu(), torch.empty((m + 1, k), device=DEV, dtype=torch.bfloat16),
+                torch.empty((k, m), device=DEV, dtype=torch.bfloat16).t()[:, :k] if m > 1 else x.reshape(1, 1, k)):
+        with pytest.raises(XQTBackendError):
+            run(bad)
+    for bad_out in (torch.empty((m, n + 8), device=DEV, dtype=torch.bfloat16), torch.empty((m, n), device=DEV)):
+        with pytest.raises(XQTBackendError):
+            run(x, bad_out)
+    with pytest.raises(XQTBackendError):
+        run(x, None, residual.to(torch.float16))
+
+
+def test_leading_dimensions_and_lifetime():
+    n, k, m = 256, 512, 6
+    codes, scale = quantize.quantize_w8_per_channel(torch.randn((n, k), generator=seeded(4)).to(DEV))
+    run = w8a8.bind_convrot_w8a8_linear(w8a8.pack_convrot_w8a8_linear(codes.t().contiguous(), scale), rows=m)
+    x = torch.randn((2, 3, k), generator=seeded(5)).to(DEV, torch.bfloat16)
+    assert tuple(run(x).shape) == (2, 3, n) and torch.equal(run(x).reshape(m, n), run(x.reshape(m, k)))
+    # a block that has bound its calls is freed with its last reference, without the garbage collector's help
+    block = W4A16SwiGLUMLP(_layer(256, 256, 6), _layer(256, 256, 7), _layer(256, 256, 8), device=DEV)
+    y = torch.randn((40, 256), generator=seeded(9)).to(DEV, torch.bfloat16)
+    for rows in (1, 17, 40):
+        assert torch.equal(block(y[:rows]), block._forward(y[:rows]))
+    gone = weakref.ref(block)
+    gc.disable()
+    try:
+        del block
+        assert gone() is None
+    finally:
+        gc.enable()

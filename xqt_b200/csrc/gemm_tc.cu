@@ -315,13 +315,6 @@ int make_tile_map(CUtensorMap* map, const void* base, CUtensorMapDataType dtype,
   return make_tile_map_ld(map, base, dtype, esize, rows, cols, cols, box_rows);
 }
 
-static int sm_count_now() {
-  int dev = 0, v = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return 148;
-  if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0) return 148;
-  return v;
-}
-
 template <int BN, typename OutT, int KIND>
 static int launch_tc(const void* a, long long lda, const void* b, long long ldb, GemmTcParams p, cudaStream_t stream) {
   using namespace gemm;
@@ -341,8 +334,8 @@ static int launch_tc(const void* a, long long lda, const void* b, long long ldb,
   const size_t smem_bytes = (size_t)p.stages * stage_bytes + 1024;
   void (*kern)(const CUtensorMap, const CUtensorMap, const GemmTcParams) =
       I8 ? gemm_i8_kernel<BN, OutT> : (KIND == 1 ? gemm_f16_kernel<BN, OutT> : gemm_bf16_kernel<BN, OutT>);
-  XQT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget));
-  int grid = sm_count_now();
+  XQT_SMEM_OPT_IN(kern, kSmemBudget);
+  int grid = sm_count();
   if (grid > p.mtiles * p.ntiles) grid = p.mtiles * p.ntiles;
   kern<<<grid, kThreads, smem_bytes, stream>>>(tm_a, tm_b, p);
   return launch_status();

@@ -512,8 +512,7 @@ static W4FusedPlan w4f_plan(int m, int n, int k, int sms) {
 static size_t w4f_align(size_t v) { return (v + 255) & ~(size_t)255; }
 constexpr size_t kW4FTicketBytes = 16384;
 size_t w4a16_gemm_fused_workspace_bytes(int m, int n, int k) {
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = sm_count();
   const W4FusedPlan pl = w4f_plan(m, n, k, sms);
   size_t bytes = 256 + kW4FTicketBytes + w4f_align((size_t)m * k * 2);
   if (pl.splits > 1) bytes += (size_t)pl.mchunks * pl.ntiles * pl.splits * pl.mt * w4f::kBM * w4f::kBN * sizeof(float);
@@ -550,8 +549,7 @@ int w4a16_gemm_fused_launch(const void* x, const void* qw, const void* scales, c
   XQT_REQUIRE(workspace != nullptr && workspace_bytes >= w4a16_gemm_fused_workspace_bytes(m, n, k) && ((uintptr_t)workspace & 255) == 0);
   XQT_REQUIRE(((uintptr_t)out & 15) == 0 && ((uintptr_t)qw & 15) == 0 && ((uintptr_t)x & 15) == 0);
   XQT_REQUIRE(!out_f32 || residual == nullptr);
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = sm_count();
   const W4FusedPlan pl = w4f_plan(m, n, k, sms);
   unsigned char* base = reinterpret_cast<unsigned char*>(workspace);
   unsigned int* status = reinterpret_cast<unsigned int*>(base);

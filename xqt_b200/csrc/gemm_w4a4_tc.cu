@@ -493,9 +493,8 @@ static int launch_w4a4(const void* a_codes, const void* b_bytes, W4A4Params p, c
   const size_t smem_bytes = w4a4_smem_bytes(p.stages);
   auto kern = gemm_w4a4_kernel<OutT>;
   XQT_SMEM_OPT_IN(kern, kSmemBudget);
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  int grid = sms > 0 ? sms : 148;
+  const int sms = sm_count();
+  int grid = sms;
   if (grid > p.mtiles * p.ntiles) grid = p.mtiles * p.ntiles;
   kern<<<grid, kThreads, smem_bytes, stream>>>(tm_a, tm_b, p);
   return launch_status();
@@ -511,8 +510,7 @@ int w4a4_expand_weight_launch(const void* qweight, void* weight_bytes, int n, in
   XQT_REQUIRE(qweight != nullptr && weight_bytes != nullptr && n > 0 && k > 0 && k % 32 == 0);
   XQT_REQUIRE(((uintptr_t)qweight & 15) == 0 && ((uintptr_t)weight_bytes & 15) == 0);
   const size_t chunks = (size_t)n * k / 32;
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = sm_count();
   const size_t want = (chunks + 255) / 256;
   w44_expand_kernel<<<(unsigned)(want < (size_t)sms * 8 ? want : (size_t)sms * 8), 256, 0, stream>>>(
       reinterpret_cast<const uint4*>(qweight), reinterpret_cast<uint4*>(weight_bytes), chunks);

@@ -1,0 +1,363 @@
+// Native call path of the bound layers: a `Bound` object holds everything one layer call needs -- the checks of its
+// input, the shape of its output, its scratch, and the library calls to make with their resolved arguments -- and a
+// call goes from the Python argument to the kernel launches without running Python code.
+//
+// What bounds it: a decode projection's kernel runs 4 us, and the same call made by a Python closure (attribute checks,
+// torch.empty, a 19-argument ctypes call) cost 12-17 us of host time, so every small call ran at the host's pace.
+//
+// The object checks what it must in order to pass a raw pointer on (dtype, device, shape, contiguity, current device).
+// Whatever it does not take on itself -- keyword arguments, a failed check, an output or residual that does not fit --
+// goes to the Python callable it was built with, which raises the layer's own error or serves the call.
+#include <torch/csrc/autograd/python_variable.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAStream.h>
+#include <structmember.h>
+
+#include <vector>
+
+#include "../../include/xqt_b200.h"
+
+namespace {
+
+// Where a pointer argument comes from; `value` is an address or a byte offset.
+enum Source : int { kConst = 0, kInput = 1, kOutput = 2, kResidual = 3, kScratch = 4, kWorkspace = 5 };
+struct Pointer {
+  int source;
+  intptr_t value;
+};
+
+// The library entry of a step.  Its arguments are its pointers, then its integers, in the order of the C prototype;
+// workspace address and size (where the entry takes them) and the stream come last.
+enum Op : int { kDecodeLanes, kW4A16Run, kSwiglu, kRotateQuantize, kW8A8Gemm, kLowrankDown, kW4A4Gemm, kOpCount };
+constexpr int kPointerCount[kOpCount] = {8, 7, 2, 5, 7, 4, 8};
+constexpr int kIntCount[kOpCount] = {9, 11, 3, 7, 4, 3, 5};
+constexpr int kMaxPointers = 8;
+struct Step {
+  int op;
+  void* fn;
+  std::vector<Pointer> ptrs;
+  std::vector<int> ints;
+  Pointer ws;
+  size_t ws_bytes;
+};
+
+// The workspace of a stream.  The reference keeps the buffer alive even where the pool it came from has since replaced
+// it by a larger one.
+struct StreamSpace {
+  cudaStream_t stream;
+  PyObject* tensor;
+  char* data;
+};
+
+struct Bound {
+  PyObject_HEAD
+  vectorcallfunc vectorcall;
+  PyObject* slow;        // the Python callable with the same signature
+  PyObject* on_error;    // called with (code, step) when a library call fails: raises
+  PyObject* workspace;   // None, or called without arguments: the current stream's workspace tensor
+  PyObject* keep;
+  at::ScalarType dtype, out_dtype;
+  int device;
+  int64_t rows, k, n;
+  bool any_rank;         // the input may have any leading dimensions that multiply to `rows`
+  bool takes_residual;   // a third positional argument, [rows, n] in the input dtype
+  int64_t scratch_bytes;
+  std::vector<Step>* steps;
+  std::vector<StreamSpace>* spaces;
+};
+
+int run_step(const Step& s, void* const* p, void* ws, cudaStream_t stream) {
+  const int* i = s.ints.data();
+  xqt_b200_stream_t st = (xqt_b200_stream_t)stream;
+  switch (s.op) {
+    case kDecodeLanes:
+      return reinterpret_cast<decltype(&xqt_b200_w4a16_decode_lanes)>(s.fn)(
+          p[0], p[1], p[2], p[3], (const float*)p[4], p[5], p[6], i[0], i[1], i[2], i[3], i[4], i[5], i[6], i[7], i[8],
+          (unsigned int*)p[7], st);
+    case kW4A16Run:
+      return reinterpret_cast<decltype(&xqt_b200_w4a16_run)>(s.fn)(
+          p[0], p[1], p[2], p[3], (const float*)p[4], p[5], p[6], i[0], i[1], i[2], i[3], i[4], i[5], i[6], i[7], i[8], i[9], ws,
+          s.ws_bytes, i[10], st);
+    case kSwiglu:
+      return reinterpret_cast<decltype(&xqt_b200_swiglu)>(s.fn)(p[0], p[1], i[0], i[1], i[2], st);
+    case kRotateQuantize:
+      return reinterpret_cast<decltype(&xqt_b200_rotate_quantize)>(s.fn)(p[0], (const float*)p[1], p[2], (float*)p[3], p[4], i[0],
+                                                                         i[1], i[2], i[3], i[4], i[5], i[6], st);
+    case kW8A8Gemm:
+      return reinterpret_cast<decltype(&xqt_b200_w8a8_gemm_addend)>(s.fn)(p[0], p[1], (const float*)p[2], (const float*)p[3],
+                                                                          (const float*)p[4], (const float*)p[5], p[6], i[0], i[1],
+                                                                          i[2], i[3], ws, s.ws_bytes, st);
+    case kLowrankDown:
+      return reinterpret_cast<decltype(&xqt_b200_lowrank_down)>(s.fn)(p[0], p[1], (float*)p[2], p[3], i[0], i[1], i[2], st);
+    case kW4A4Gemm:
+      return reinterpret_cast<decltype(&xqt_b200_w4a4_gemm)>(s.fn)(p[0], (const float*)p[1], p[2], p[3], p[4], (const float*)p[5],
+                                                                   (const float*)p[6], p[7], i[0], i[1], i[2], i[3], i[4], ws,
+                                                                   s.ws_bytes, st);
+  }
+  return (int)cudaErrorInvalidValue;
+}
+
+char* stream_space(Bound* b, cudaStream_t stream, PyObject** held) {
+  for (const StreamSpace& s : *b->spaces)
+    if (s.stream == stream) {
+      Py_INCREF(s.tensor);
+      *held = s.tensor;
+      return s.data;
+    }
+  PyObject* t = PyObject_CallNoArgs(b->workspace);
+  if (t == nullptr) return nullptr;
+  if (!THPVariable_Check(t)) {
+    Py_DECREF(t);
+    PyErr_SetString(PyExc_TypeError, "Bound: workspace() must return a tensor");
+    return nullptr;
+  }
+  char* data = static_cast<char*>(THPVariable_Unpack(t).data_ptr());
+  if (b->spaces->size() >= 16) {                 // a program that keeps making streams: forget the oldest
+    Py_DECREF(b->spaces->front().tensor);
+    b->spaces->erase(b->spaces->begin());
+  }
+  Py_INCREF(t);
+  b->spaces->push_back({stream, t, data});
+  *held = t;
+  return data;
+}
+
+bool plain(const at::Tensor& t, at::ScalarType dtype, int device) {
+  return t.scalar_type() == dtype && t.is_cuda() && t.device().index() == device && t.layout() == at::kStrided && t.is_contiguous();
+}
+
+PyObject* bound_call(PyObject* self, PyObject* const* args, size_t nargsf, PyObject* kwnames) {
+  Bound* b = reinterpret_cast<Bound*>(self);
+  const Py_ssize_t nargs = PyVectorcall_NARGS(nargsf);
+  auto slow = [&]() { return PyObject_Vectorcall(b->slow, args, nargsf, kwnames); };
+  if (kwnames != nullptr || nargs < 1 || nargs > 3 || !THPVariable_Check(args[0])) return slow();
+  const at::Tensor& x = THPVariable_Unpack(args[0]);
+  if (!plain(x, b->dtype, b->device) || c10::cuda::current_device() != b->device) return slow();
+  const auto shape = x.sizes();
+  const int64_t dim = (int64_t)shape.size();
+  if (dim < 1 || shape[dim - 1] != b->k || x.numel() != b->rows * b->k || (!b->any_rank && dim != 2)) return slow();
+
+  at::Tensor out;
+  PyObject* result = nullptr;
+  if (nargs >= 2 && args[1] != Py_None) {
+    if (!THPVariable_Check(args[1])) return slow();
+    const at::Tensor& o = THPVariable_Unpack(args[1]);
+    if (b->any_rank || !plain(o, b->out_dtype, b->device) || o.dim() != 2 || o.size(0) != b->rows || o.size(1) != b->n) return slow();
+    result = args[1];
+    Py_INCREF(result);
+  }
+  const void* residual = nullptr;
+  if (nargs == 3 && args[2] != Py_None) {
+    bool fits = b->takes_residual && THPVariable_Check(args[2]);
+    if (fits) {
+      const at::Tensor& r = THPVariable_Unpack(args[2]);
+      fits = plain(r, b->dtype, b->device) && r.dim() == 2 && r.size(0) == b->rows && r.size(1) == b->n;
+      if (fits) residual = r.data_ptr();
+    }
+    if (!fits) {
+      Py_XDECREF(result);
+      return slow();
+    }
+  }
+  PyObject* held = nullptr;
+  int code = 0;
+  size_t at_step = 0;
+  try {
+    const c10::Device device(c10::kCUDA, (c10::DeviceIndex)b->device);
+    void* out_data;
+    if (result == nullptr) {
+      if (dim == 2) {
+        out = at::detail::empty_cuda({b->rows, b->n}, b->out_dtype, device, c10::nullopt);
+      } else {
+        std::vector<int64_t> oshape(shape.begin(), shape.end());
+        oshape.back() = b->n;
+        out = at::detail::empty_cuda(oshape, b->out_dtype, device, c10::nullopt);
+      }
+      out_data = out.data_ptr();
+    } else {
+      out_data = THPVariable_Unpack(result).data_ptr();
+    }
+    at::Tensor scratch;
+    if (b->scratch_bytes > 0) scratch = at::detail::empty_cuda({b->scratch_bytes}, at::kByte, device, c10::nullopt);
+    const cudaStream_t stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)b->device).stream();
+    char* base[6] = {nullptr, static_cast<char*>(x.data_ptr()), static_cast<char*>(out_data),
+                     static_cast<char*>(const_cast<void*>(residual)),
+                     scratch.defined() ? static_cast<char*>(scratch.data_ptr()) : nullptr, nullptr};
+    if (b->workspace != Py_None) {
+      base[kWorkspace] = stream_space(b, stream, &held);
+      if (base[kWorkspace] == nullptr) {
+        Py_XDECREF(result);
+        return nullptr;
+      }
+    }
+    Py_BEGIN_ALLOW_THREADS
+    for (; at_step < b->steps->size(); ++at_step) {
+      const Step& s = (*b->steps)[at_step];
+      void* p[kMaxPointers];
+      for (size_t i = 0; i < s.ptrs.size(); ++i) {
+        char* from = base[s.ptrs[i].source];
+        p[i] = s.ptrs[i].source == kResidual && from == nullptr ? nullptr : from + s.ptrs[i].value;
+      }
+      code = run_step(s, p, base[s.ws.source] + s.ws.value, stream);
+      if (code != 0) break;
+    }
+    Py_END_ALLOW_THREADS
+  } catch (const std::exception& e) {
+    Py_XDECREF(held);
+    Py_XDECREF(result);
+    PyErr_SetString(PyExc_RuntimeError, e.what());
+    return nullptr;
+  }
+  Py_XDECREF(held);
+  if (code != 0) {
+    Py_XDECREF(result);
+    PyObject* r = PyObject_CallFunction(b->on_error, "in", code, (Py_ssize_t)at_step);
+    if (r != nullptr) {
+      Py_DECREF(r);
+      PyErr_SetString(PyExc_RuntimeError, "Bound: library call failed");
+    }
+    return nullptr;
+  }
+  return result != nullptr ? result : THPVariable_Wrap(std::move(out));
+}
+
+bool parse_pointer(PyObject* o, Pointer* p) {
+  long long value = 0;
+  int source = 0;
+  if (PyTuple_Check(o)) {
+    if (!PyArg_ParseTuple(o, "iL", &source, &value)) return false;
+  } else {
+    value = PyLong_AsLongLong(o);
+    if (value == -1 && PyErr_Occurred()) return false;
+  }
+  if (source < kConst || source > kWorkspace) {
+    PyErr_SetString(PyExc_ValueError, "Bound: unknown pointer source");
+    return false;
+  }
+  p->source = source;
+  p->value = (intptr_t)value;
+  return true;
+}
+
+bool parse_step(PyObject* o, Step* s) {
+  PyObject *ptrs, *ints, *ws;
+  unsigned long long fn;
+  Py_ssize_t ws_bytes;
+  if (!PyArg_ParseTuple(o, "iKO!O!On", &s->op, &fn, &PyTuple_Type, &ptrs, &PyTuple_Type, &ints, &ws, &ws_bytes)) return false;
+  if (s->op < 0 || s->op >= kOpCount || fn == 0 || PyTuple_GET_SIZE(ptrs) != kPointerCount[s->op] || PyTuple_GET_SIZE(ints) != kIntCount[s->op]) {
+    PyErr_SetString(PyExc_ValueError, "Bound: a step does not have the arguments of its library entry");
+    return false;
+  }
+  s->fn = reinterpret_cast<void*>(fn);
+  s->ws_bytes = (size_t)ws_bytes;
+  s->ptrs.resize((size_t)PyTuple_GET_SIZE(ptrs));
+  for (size_t i = 0; i < s->ptrs.size(); ++i)
+    if (!parse_pointer(PyTuple_GET_ITEM(ptrs, (Py_ssize_t)i), &s->ptrs[i])) return false;
+  for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(ints); ++i) {
+    const long v = PyLong_AsLong(PyTuple_GET_ITEM(ints, i));
+    if (v == -1 && PyErr_Occurred()) return false;
+    s->ints.push_back((int)v);
+  }
+  return parse_pointer(ws, &s->ws);
+}
+
+int bound_traverse(PyObject* self, visitproc visit, void* arg) {
+  Bound* b = reinterpret_cast<Bound*>(self);
+  Py_VISIT(b->slow);
+  Py_VISIT(b->on_error);
+  Py_VISIT(b->workspace);
+  Py_VISIT(b->keep);
+  return 0;
+}
+int bound_clear(PyObject* self) {
+  Bound* b = reinterpret_cast<Bound*>(self);
+  Py_CLEAR(b->slow);
+  Py_CLEAR(b->on_error);
+  Py_CLEAR(b->workspace);
+  Py_CLEAR(b->keep);
+  return 0;
+}
+void bound_dealloc(PyObject* self) {
+  Bound* b = reinterpret_cast<Bound*>(self);
+  PyObject_GC_UnTrack(self);
+  bound_clear(self);
+  if (b->spaces != nullptr)
+    for (const StreamSpace& s : *b->spaces) Py_DECREF(s.tensor);
+  delete b->spaces;
+  delete b->steps;
+  Py_TYPE(self)->tp_free(self);
+}
+
+PyObject* bound_new(PyTypeObject* type, PyObject* args, PyObject* kwargs) {
+  static const char* names[] = {"steps", "slow", "on_error", "dtype", "out_dtype", "device", "rows", "k", "n", "any_rank",
+                                "takes_residual", "scratch_bytes", "workspace", "keep", nullptr};
+  PyObject *steps, *slow, *on_error, *dtype, *out_dtype, *workspace = Py_None, *keep = Py_None;
+  int device, any_rank = 0, takes_residual = 0;
+  long long rows, k, n, scratch_bytes = 0;
+  if (!PyArg_ParseTupleAndKeywords(args, kwargs, "O!OOOOiLLL|ppLOO", const_cast<char**>(names), &PyTuple_Type, &steps, &slow, &on_error,
+                                   &dtype, &out_dtype, &device, &rows, &k, &n, &any_rank, &takes_residual, &scratch_bytes, &workspace,
+                                   &keep))
+    return nullptr;
+  if (!THPDtype_Check(dtype) || !THPDtype_Check(out_dtype)) {
+    PyErr_SetString(PyExc_TypeError, "Bound: dtype and out_dtype must be torch dtypes");
+    return nullptr;
+  }
+  auto parsed = new std::vector<Step>((size_t)PyTuple_GET_SIZE(steps));
+  for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(steps); ++i)
+    if (!parse_step(PyTuple_GET_ITEM(steps, i), &(*parsed)[(size_t)i])) {
+      delete parsed;
+      return nullptr;
+    }
+  Bound* b = reinterpret_cast<Bound*>(type->tp_alloc(type, 0));
+  if (b == nullptr) {
+    delete parsed;
+    return nullptr;
+  }
+  b->vectorcall = bound_call;
+  b->steps = parsed;
+  b->spaces = new std::vector<StreamSpace>();
+  Py_INCREF(slow); b->slow = slow;
+  Py_INCREF(on_error); b->on_error = on_error;
+  Py_INCREF(workspace); b->workspace = workspace;
+  Py_INCREF(keep); b->keep = keep;
+  b->dtype = reinterpret_cast<THPDtype*>(dtype)->scalar_type;
+  b->out_dtype = reinterpret_cast<THPDtype*>(out_dtype)->scalar_type;
+  b->device = device;
+  b->rows = rows; b->k = k; b->n = n;
+  b->any_rank = any_rank != 0;
+  b->takes_residual = takes_residual != 0;
+  b->scratch_bytes = scratch_bytes;
+  return reinterpret_cast<PyObject*>(b);
+}
+
+PyMemberDef bound_members[] = {{"keep", T_OBJECT, offsetof(Bound, keep), 0, "the objects whose memory the calls use"},
+                               {"slow", T_OBJECT, offsetof(Bound, slow), 0, "the callable that gets what the native path does not take"},
+                               {nullptr, 0, 0, 0, nullptr}};
+PyTypeObject bound_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
+PyModuleDef host_module = {PyModuleDef_HEAD_INIT, "_host", "Native call path of the bound layers.", -1, nullptr, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__host(void) {
+  bound_type.tp_name = "xqt_b200._host.Bound";
+  bound_type.tp_basicsize = sizeof(Bound);
+  bound_type.tp_flags = Py_TPFLAGS_DEFAULT | Py_TPFLAGS_HAVE_GC | Py_TPFLAGS_HAVE_VECTORCALL;
+  bound_type.tp_new = bound_new;
+  bound_type.tp_dealloc = bound_dealloc;
+  bound_type.tp_traverse = bound_traverse;
+  bound_type.tp_clear = bound_clear;
+  bound_type.tp_call = PyVectorcall_Call;
+  bound_type.tp_vectorcall_offset = offsetof(Bound, vectorcall);
+  bound_type.tp_members = bound_members;
+  if (PyType_Ready(&bound_type) < 0) return nullptr;
+  PyObject* m = PyModule_Create(&host_module);
+  if (m == nullptr) return nullptr;
+  Py_INCREF(&bound_type);
+  if (PyModule_AddObject(m, "Bound", reinterpret_cast<PyObject*>(&bound_type)) < 0) {
+    Py_DECREF(&bound_type);
+    Py_DECREF(m);
+    return nullptr;
+  }
+  return m;
+}

@@ -514,18 +514,6 @@ struct ClPlan {
   int kw, s;
 };
 
-int cl_sm_count() {
-  static int cached[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-  if (cached[dev] == 0) {
-    int v = 0;
-    if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0) v = 148;
-    cached[dev] = v;
-  }
-  return cached[dev];
-}
-
 // A plan forced through w4a16_decode_cl_set_plan (tuning runs); kw == 0 means automatic.
 int g_forced_kw = 0, g_forced_s = 0;
 
@@ -546,7 +534,7 @@ ClPlan cl_plan(int tiles, int kblocks, int m) {
   ClPlan plan;
   const int max_slice = m > 8 ? kMaxSliceBlocks16 : kMaxSliceBlocks8;
   if (!cl_plan_override(plan)) {
-    const int wave_warps = cl_sm_count() * 16;
+    const int wave_warps = sm_count() * 16;
     int pieces = 1;
     while (pieces < kMaxKW * kMaxCluster && (long long)tiles * 4 * (pieces * 2) <= wave_warps && pieces * 2 * 2 <= kblocks)
       pieces *= 2;

@@ -23,9 +23,10 @@ from torch import nn
 from . import native
 from .contracts import PackedWeight
 from .errors import XQTBackendError
+from .hostcall import INPUT, OUTPUT, WORKSPACE, bound_call, step, weak_method
 from .layout import signed_storage_to_unsigned
 from .ops import awq as awq_ops
-from .ops.w4a16 import w4a16_linear
+from .ops.w4a16 import resolve_w4a16_variant, w4a16_linear
 
 _DTYPE_NAME = {torch.float16: "fp16", torch.bfloat16: "bf16"}
 MAX_DECODE_ROWS = 16
@@ -60,6 +61,9 @@ class AWQW4A16Linear(nn.Module):
         self._prepared: dict[torch.dtype, tuple] = {}
         self._bound: dict[tuple[int, torch.dtype], Callable] = {}
         self._residual_bound: dict[tuple[int, torch.dtype], Callable] = {}
+        # (rows, dtype) -> (tensors it was built from, bound call, its execution report): calls of forward() that need no
+        # other work than the bound call
+        self._hot: dict[tuple[int, torch.dtype], tuple] = {}
         self._native_only = False
         self._native_only_rows: frozenset[int] = frozenset()
         self._native_only_dtype: torch.dtype | None = None
@@ -133,14 +137,16 @@ class AWQW4A16Linear(nn.Module):
             qweight, scales, zeros, rows=rows, input_features=self.input_features, output_features=self.output_features,
             dtype=dtype, device=device, bias=None if self.bias is None else self.bias.to(device))
         k = self.input_features
+        served = native_bound.slow
 
-        def bound(inputs: torch.Tensor) -> torch.Tensor:
+        def checked(inputs: torch.Tensor) -> torch.Tensor:
             if inputs.ndim != 2 or tuple(inputs.shape) != (rows, k) or inputs.dtype != dtype or inputs.device != device:
                 raise XQTBackendError("bound AWQ W4A16 input disagrees with the static shape/dtype/device")
-            return native_bound(inputs)
+            return served(inputs)
 
-        self._bound[key] = bound
-        return bound
+        native_bound.slow = checked
+        self._bound[key] = native_bound
+        return native_bound
 
     def bind_residual(self, *, rows: int, dtype: torch.dtype) -> Callable[[torch.Tensor, torch.Tensor], None]:
         """Decode GEMV whose epilogue adds into a residual row in place: ``residual += projection(inputs)``.
@@ -204,6 +210,7 @@ class AWQW4A16Linear(nn.Module):
             raise ValueError(f"native-only AWQ W4A16 rows must be between 1 and {MAX_DECODE_ROWS}")
         for r in frozen:
             self.bind(rows=r, dtype=dtype)
+        self._hot.clear()
         released = self.canonical_qweight.numel() * self.canonical_qweight.element_size()
         self.canonical_qweight = None
         # the execution PackedWeight dropped its canonical bytes too
@@ -215,9 +222,59 @@ class AWQW4A16Linear(nn.Module):
         return int(released)
 
     # ------------------------------------------------------------------ forward
+    def _hot_call(self, rows: int, dtype: torch.dtype) -> tuple | None:
+        """The entry of :attr:`_hot` for ``rows`` rows, built when it is missing or a buffer has been replaced since."""
+
+        buffers = self._buffers
+        zeros = buffers["weight_zero_point"]
+        made_from = (buffers["canonical_qweight"], buffers["weight_scale"], zeros, buffers["bias"])
+        hit = self._hot.get((rows, dtype))
+        if hit is not None and all(a is b for a, b in zip(hit[0], made_from)) and hit[3] == (None if zeros is None else zeros._version):
+            return hit
+        canonical, scales, _, bias = made_from
+        if self._native_only or canonical is None or not canonical.is_cuda or dtype not in _DTYPE_NAME or rows < 1 \
+                or any(t is not None and t.device != canonical.device for t in made_from):
+            return None
+        if rows <= MAX_DECODE_ROWS:
+            run, kernel = self.bind(rows=rows, dtype=dtype), "w4a16_decode_cl_kernel"
+        else:
+            n, k, padded_k, group, device = self.output_features, self.input_features, int(canonical.shape[1]) * 2, self.group_size, canonical.device
+            if any(t is not None and not t.is_contiguous() for t in made_from) or scales.dtype not in native.DTYPE_CODE \
+                    or (zeros is not None and zeros.dtype != scales.dtype):
+                return None
+            variant = resolve_w4a16_variant(rows, n, k, padded_k, group, zero_points=zeros)
+            nbytes = native.library().xqt_b200_w4a16_workspace_bytes(rows, n, k)
+            gemm = step("xqt_b200_w4a16_run", ((INPUT, 0), canonical, scales, zeros, bias, 0, (OUTPUT, 0)),
+                        (rows, n, k, padded_k, group, 0, native.DTYPE_CODE[dtype], native.DTYPE_CODE[scales.dtype], native.DTYPE_CODE[dtype],
+                         0, native.VARIANT[variant]), (WORKSPACE, 0), nbytes)
+            run = bound_call([gemm], weak_method(self._forward_flat), dtype=dtype, device=device, rows=rows, k=k, n=n,
+                             workspace=lambda: native.workspace(device, nbytes), keep=made_from, symbols="xqt_b200_w4a16_run")
+            kernel = "w4a16 tcgen05 GEMM"
+        if len(self._hot) >= 512:
+            self._hot.clear()
+        hit = (made_from, run, self._report(kernel, rows, dtype), None if zeros is None else zeros._version)
+        self._hot[(rows, dtype)] = hit
+        return hit
+
+    def _report(self, kernel: str, rows: int, dtype: torch.dtype) -> dict[str, Any]:
+        return {
+            "implementation": "b200_awq_w4a16", "native": True, "kernel": kernel, "rows": rows,
+            "input_features": self.input_features, "output_features": self.output_features, "dtype": _DTYPE_NAME[dtype],
+            "bias": self._has_bias, "layout": awq_ops.LANES_LAYOUT,
+        }
+
     def forward(self, inputs: torch.Tensor) -> torch.Tensor:
         if self.training:
             raise RuntimeError("AWQ W4A16 native path requires eval mode")
+        if inputs.ndim == 2:
+            hit = self._hot_call(inputs.shape[0], inputs.dtype)
+            if hit is not None:
+                output = hit[1](inputs)
+                self._last_execution = hit[2]
+                return output
+        return self._forward_flat(inputs)
+
+    def _forward_flat(self, inputs: torch.Tensor) -> torch.Tensor:
         if inputs.shape[-1] != self.input_features:
             raise XQTBackendError("AWQ W4A16 input trailing dimension does not match input_features")
         if inputs.dtype not in _DTYPE_NAME:
@@ -233,11 +290,7 @@ class AWQW4A16Linear(nn.Module):
             output = w4a16_linear(flat, self.canonical_qweight, self.weight_scale, self.weight_zero_point, self.bias,
                                   group_size=self.group_size, nibble_signed=False)
             kernel = "w4a16 tcgen05 GEMM"
-        self._last_execution = {
-            "implementation": "b200_awq_w4a16", "native": True, "kernel": kernel, "rows": rows,
-            "input_features": self.input_features, "output_features": self.output_features, "dtype": _DTYPE_NAME[flat.dtype],
-            "bias": self._has_bias, "layout": awq_ops.LANES_LAYOUT,
-        }
+        self._last_execution = self._report(kernel, rows, flat.dtype)
         return output.reshape(*inputs.shape[:-1], self.output_features)
 
     def execution_metadata(self) -> dict[str, Any]:

@@ -108,6 +108,22 @@ def library() -> ctypes.CDLL:
         return handle
 
 
+_host_module = None
+
+
+def host():
+    """The native call path of the bound layers (``csrc/host.cpp``), loaded once; like the library it has no fallback."""
+
+    global _host_module
+    if _host_module is None:
+        try:
+            from . import _host
+        except ImportError as exc:
+            raise NativeLibraryError(f"cannot load the native call path ({exc}): build it with `python -m xqt_b200.build`") from exc
+        _host_module = _host
+    return _host_module
+
+
 def available() -> bool:
     """True when the library loads.  Says nothing about a GPU being present."""
 
@@ -194,5 +210,5 @@ def workspace_status(device: torch.device) -> int:
 
 __all__ = [
     "ACT", "BF16", "DTYPE_CODE", "FP16", "FP32", "LIBRARY_PATH", "SIGNATURES", "VARIANT", "VARIANT_NAMES",
-    "available", "check", "library", "ptr", "status_word", "stream_handle", "version", "workspace", "workspace_status",
+    "available", "check", "host", "library", "ptr", "status_word", "stream_handle", "version", "workspace", "workspace_status",
 ]

@@ -37,6 +37,7 @@ import torch
 from .. import native, prepack
 from ..contracts import PackedWeight, PackedWeightMetadata
 from ..errors import NativeLibraryError, XQTBackendError
+from ..hostcall import INPUT, OUTPUT, bound_call, step
 from ..layout import W4_LAYOUT, validate_w4a16_packed_weight
 from ..weakid import WeakIdDict
 
@@ -203,14 +204,17 @@ def bind_awq_w4a16_decode(qweight: torch.Tensor, scales: torch.Tensor, scaled_ze
                  native.DTYPE_CODE[dtype], 0, status.data_ptr())
 
     def bound(inputs: torch.Tensor) -> torch.Tensor:
+        inputs = inputs.contiguous()
         output = torch.empty((rows, output_features), dtype=dtype, device=device)
         code = fn(inputs.data_ptr(), *args_head, output.data_ptr(), *args_tail, torch.cuda.current_stream(device).cuda_stream)
         if code != 0:
             native.check(code, "xqt_b200_w4a16_decode_lanes")
         return output
 
-    bound.keep = (qweight, scales, scaled_zeros, bias32, status)     # the raw pointers above must stay valid
-    return bound
+    keep = (qweight, scales, scaled_zeros, bias32, status)     # the raw pointers above must stay valid
+    decode = step("xqt_b200_w4a16_decode_lanes", ((INPUT, 0), *args_head, (OUTPUT, 0), status), args_tail[:-1])
+    return bound_call([decode], bound, dtype=dtype, device=device, rows=rows, k=input_features, n=output_features, keep=keep,
+                      symbols="xqt_b200_w4a16_decode_lanes")
 
 
 def awq_w4a16_decode(inputs: torch.Tensor, qweight: torch.Tensor, scales: torch.Tensor,

@@ -21,8 +21,9 @@ import torch.distributed as dist
 from .. import native
 from ..contracts import PackedWeight, PackedWeightMetadata
 from ..errors import XQTBackendError
+from ..hostcall import INPUT, OUTPUT, WORKSPACE, ScratchPlan, bound_call, step, weak_method
 from ..parallel import shard_packed_weight
-from .w4a16 import bind_w4a16_decode, glu_row_order, prepare_decode, w4a16_linear
+from .w4a16 import bind_w4a16_decode, glu_row_order, prepare_decode, resolve_w4a16_variant, w4a16_linear
 
 
 def swiglu(gate_up: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
@@ -130,6 +131,30 @@ class _Linear:
         return w4a16_linear(x, self.qweight, self.scales, self.zeros, group_size=self.group,
                             nibble_signed=self.signed, k=self.k, out_dtype=odt, out=out)
 
+    def decode_steps(self, m: int, source: tuple, target: tuple, *, glu: bool) -> list:
+        """The decode launches of ``m`` rows (one per 16) as steps of a bound call."""
+
+        lib, status, params = native.library(), native.status_word(self.qweight.device), self.tiled.params
+        if not lib.xqt_b200_w4a16_decode_lanes_supported(min(m, 16), self.n, self.k, self.group):
+            raise XQTBackendError(f"B200 W4A16 decode does not cover N={self.n}, K={self.k}, group={self.group}")
+        code, width = native.DTYPE_CODE[self.dtype], self.n // 2 if glu else self.n
+        return [step("xqt_b200_w4a16_decode_lanes",
+                     ((source[0], source[1] + 2 * r0 * self.k), self.tiled.weights, params[0], params[1] if self.tiled.has_zero_point else 0,
+                      0, 0, (target[0], target[1] + 2 * r0 * width), status),
+                     (min(16, m - r0), self.n, self.k, self.group, self.tiled.nibble_signed, code, native.DTYPE_CODE[params.dtype],
+                      code, 2 if glu else 0)) for r0 in range(0, m, 16)]
+
+    def gemm_steps(self, m: int, source: tuple, target: tuple) -> tuple[list, int]:
+        """The canonical-weight GEMM of ``m`` rows as a step of a bound call, and the workspace bytes it needs."""
+
+        lib = native.library()
+        variant = resolve_w4a16_variant(m, self.n, self.k, int(self.qweight.shape[1]) * 2, self.group, zero_points=self.zeros)
+        nbytes = lib.xqt_b200_w4a16_workspace_bytes(m, self.n, self.k)
+        code = native.DTYPE_CODE[self.dtype]
+        return [step("xqt_b200_w4a16_run", (source, self.qweight, self.scales, self.zeros, 0, 0, target),
+                     (m, self.n, self.k, int(self.qweight.shape[1]) * 2, self.group, self.signed, code,
+                      native.DTYPE_CODE[self.scales.dtype], code, 0, native.VARIANT[variant]), (WORKSPACE, 0), nbytes)], nbytes
+
     def partial_into(self, x: torch.Tensor, peer) -> None:
         """Decode-size fp32 partial sums of a K-sharded layer, written into the slot of ``peer`` (a counted
         :class:`xqt_b200.parallel.PeerAllReduce`) that its next reduction reads; the kernel picks the slot on the device."""
@@ -179,6 +204,8 @@ class W4A16SwiGLUMLP:
             up = shard_packed_weight(up, world=world, rank=rank, axis=0)
             down = shard_packed_weight(down, world=world, rank=rank, axis=1)
         self.world, self.group, self.dtype = world, group, dtype
+        self._native: dict[int, tuple] = {}       # row count -> (zero-point versions, bound call), single-GPU blocks
+        self._can_bind = world == 1 and local_linear is None and swiglu_fn is None
         self._swiglu = swiglu_fn or swiglu
         if local_linear is not None:
             self.gate_up = _InjectedLinear(_concat_rows(gate, up), local_linear)
@@ -200,6 +227,42 @@ class W4A16SwiGLUMLP:
             self._peer = PeerAllReduce(device, 16 * self.hidden, group, counted=self.down.tiled.layout == "lanes")
 
     def __call__(self, x: torch.Tensor) -> torch.Tensor:
+        if self._can_bind:
+            zeros = self._zero_versions()
+            hit = self._native.get(x.shape[0])
+            if hit is None or hit[0] != zeros:
+                if len(self._native) >= 512:
+                    self._native.clear()
+                hit = (zeros, self._bind(int(x.shape[0])))
+                self._native[x.shape[0]] = hit
+            return hit[1](x)
+        return self._forward(x)
+
+    def _zero_versions(self) -> tuple:
+        gate_up, down = self.gate_up.zeros, self.down.zeros
+        return (-1 if gate_up is None else gate_up._version, -1 if down is None else down._version)
+
+    def _bind(self, m: int):
+        """The block for ``m`` rows as one bound call: the launches of :meth:`_forward` with their arguments resolved."""
+
+        device, scratch, nbytes = self.gate_up.qweight.device, ScratchPlan(), 0
+        inter, lanes = self.inter_local, self.down.tiled.layout == "lanes"
+        if m < 1 or device.type != "cuda" or (m <= CHUNKED_DECODE_MAX_ROWS and not (self.gate_up.glu and lanes)):
+            return weak_method(self._forward)
+        h = scratch.take(2 * m * inter)
+        if m <= CHUNKED_DECODE_MAX_ROWS:
+            steps = self.gate_up.decode_steps(m, (INPUT, 0), h, glu=True) + self.down.decode_steps(m, h, (OUTPUT, 0), glu=False)
+        else:
+            both = scratch.take(4 * m * inter)
+            first, need = self.gate_up.gemm_steps(m, (INPUT, 0), both)
+            last, more = self.down.gemm_steps(m, h, (OUTPUT, 0))
+            steps = first + [step("xqt_b200_swiglu", (both, h), (m, inter, native.DTYPE_CODE[self.dtype]))] + last
+            nbytes = max(need, more)
+        return bound_call(steps, weak_method(self._forward), dtype=self.dtype, device=device, rows=m, k=self.gate_up.k, n=self.hidden,
+                          scratch_bytes=scratch.nbytes, workspace=(lambda: native.workspace(device, nbytes)) if nbytes else None,
+                          keep=(self.gate_up, self.down, native.status_word(device)), symbols="bound W4A16 SwiGLU MLP")
+
+    def _forward(self, x: torch.Tensor) -> torch.Tensor:
         h = self.gate_up.gated(x) if isinstance(self.gate_up, _Linear) else None     # decode sizes: one launch
         if h is None:
             h = self._swiglu(self.gate_up(x))

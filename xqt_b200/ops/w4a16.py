@@ -11,6 +11,7 @@ from __future__ import annotations
 import torch
 
 from .. import native
+from ..hostcall import INPUT, OUTPUT, RESIDUAL, WORKSPACE, bound_call, step
 from ..errors import XQTBackendError
 from ..weakid import WeakIdDict
 
@@ -47,6 +48,20 @@ def select_variant(m: int, n: int, k: int, padded_k: int, group_size: int, activ
     code = native.library().xqt_b200_w4a16_select_variant(
         m, n, k, padded_k, group_size, native.ACT[activation], int(has_residual))
     return native.VARIANT_NAMES[code]
+
+
+def resolve_w4a16_variant(m: int, n: int, k: int, padded_k: int, group_size: int, *, zero_points: torch.Tensor | None = None,
+                          activation: str = "none", has_residual: bool = False) -> str:
+    """The kernel :func:`w4a16_linear` takes for ``variant="auto"`` and an output in the activation dtype."""
+
+    lib = native.library()
+    variant = select_variant(m, n, k, padded_k, int(group_size), activation, has_residual)
+    if variant == "tcgen05" and not lib.xqt_b200_w4a16_two_pass(m) and not _integer_zero_points(zero_points):
+        variant = "simt"
+    # the fused single-pass form where it measures faster (17 <= M <= 512); integer zero points only
+    if variant == "tcgen05" and lib.xqt_b200_w4a16_fused_preferred(m, n, k, padded_k, int(group_size)) and _integer_zero_points(zero_points):
+        variant = "tcgen05_fused"
+    return variant
 
 
 def w4a16_linear(
@@ -119,13 +134,8 @@ def w4a16_linear(
             and _integer_zero_points(zero_points) and lib.xqt_b200_w4a16_fused_preferred(m, n, k, padded_k, int(group_size))
         variant = "tcgen05_fused" if fused_ok else "tcgen05"
     if variant == "auto":
-        variant = select_variant(m, n, k, padded_k, int(group_size), activation, residual is not None)
-        if variant == "tcgen05" and not two_pass and not _integer_zero_points(zero_points):
-            variant = "simt"
-        # the fused single-pass form where it measures faster (17 <= M <= 512); integer zero points only
-        if variant == "tcgen05" and odt != torch.float32 and lib.xqt_b200_w4a16_fused_preferred(m, n, k, padded_k, int(group_size)) \
-                and _integer_zero_points(zero_points):
-            variant = "tcgen05_fused"
+        variant = resolve_w4a16_variant(m, n, k, padded_k, int(group_size), zero_points=zero_points, activation=activation,
+                                        has_residual=residual is not None)
     if variant == "tcgen05_fused" and not _integer_zero_points(zero_points):
         raise XQTBackendError("the single-pass tcgen05 GEMM needs integer zero points")
     scratch = native.workspace(device, lib.xqt_b200_w4a16_workspace_bytes(m, n, k))
@@ -193,8 +203,9 @@ def bind_w4a16_linear(
             native.check(code, "xqt_b200_w4a16_run")
         return out
 
-    run.keep = keep          # the callable owns the tensors whose raw pointers it passes
-    return run
+    run_step = step("xqt_b200_w4a16_run", ((INPUT, 0), *static, (OUTPUT, 0)), (*tail, variant_code), (WORKSPACE, 0), nbytes)
+    return bound_call([run_step], run, dtype=dtype, device=device, rows=rows, k=kk, n=n, workspace=lambda: native.workspace(device, nbytes),
+                      keep=keep, symbols="xqt_b200_w4a16_run")          # the callable owns the tensors whose raw pointers it passes
 
 
 def decode_supported(m: int, n: int, k: int, group_size: int) -> bool:
@@ -343,8 +354,12 @@ def _bind_decode_lanes(tiled, *, rows: int, dtype: torch.dtype, bias: torch.Tens
             native.check(code, "xqt_b200_w4a16_decode_lanes")
         return out
 
-    run.keep = keep          # the callable owns the tensors whose raw pointers it passes
-    return run
+    if out_select is not None:
+        run.keep = keep          # the callable owns the tensors whose raw pointers it passes
+        return run
+    decode = step("xqt_b200_w4a16_decode_lanes", ((INPUT, 0), *head, (RESIDUAL, 0), (OUTPUT, 0), status), tail)
+    return bound_call([decode], run, dtype=dtype, device=device, rows=rows, k=k, n=n_out, out_dtype=odt,
+                      residual=not glu and odt == dtype, keep=keep, symbols="xqt_b200_w4a16_decode_lanes")
 
 
 def prepare_decode(qweight: torch.Tensor, scales: torch.Tensor, zero_points: torch.Tensor | None, *,

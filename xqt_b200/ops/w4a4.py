@@ -27,8 +27,9 @@ import torch
 
 from .. import native
 from ..errors import XQTBackendError
+from ..hostcall import INPUT, OUTPUT, WORKSPACE, bound_call, step
 from ..quantize import Rotation, quantize_residual_int4
-from .activation import rotate_quantize
+from .activation import _KIND, _column_scale, rotate_quantize
 
 GROUP = 64
 RANK_PAD = 32
@@ -328,8 +329,29 @@ def bind_svdq_w4a4_linear(packed: PackedSVDQW4A4Linear, workspace: W4A4Workspace
             raise XQTBackendError("bound SVDQ W4A4 call: input shape, dtype or device mismatch")
         return svdq_w4a4_linear(inputs, packed, workspace=workspace, lora_scale=lora_scale)
 
-    run.keep = (packed, workspace)
-    return run
+    if lora_scale != 1.0 or k % (1 if packed.rotation is None else packed.rotation.block) or rows < 1 \
+            or int(workspace.quantized_activation.shape[1]) != k or workspace.rotated_activation is None:
+        run.keep = (packed, workspace)
+        return run
+    # the calls of the unbound form with every argument resolved: prologue with tile-major scales, down projection into
+    # operand images, GEMM (flags 1 | 2).  Without a low-rank branch the images are zero bits.
+    lib, n, dcode, rot = native.library(), packed.output_features, native.DTYPE_CODE[dtype], packed.rotation
+    la = workspace.lora_activation if packed.rank else None
+    if la is None:
+        la = torch.zeros((-(-rows // TILE) * TILE, RANK_PAD), device=device, dtype=torch.float32)
+    column_scale = None if rot is None else _column_scale(rot, device)
+    codes, scales, rotated = workspace.quantized_activation, workspace.activation_scales, workspace.rotated_activation
+    steps = [step("xqt_b200_rotate_quantize", ((INPUT, 0), column_scale, codes, scales, rotated),
+                  (rows, k, _KIND[None if rot is None else rot.kind], 0 if rot is None else rot.block, 6,
+                   GROUP if packed.act_granularity == "group" else 0, dcode))]
+    if packed.rank:
+        steps.append(step("xqt_b200_lowrank_down", (rotated, packed.down, 0, la), (rows, k, dcode)))
+    nbytes = lib.xqt_b200_w4a4_workspace_bytes(rows, n, k)
+    steps.append(step("xqt_b200_w4a4_gemm", (codes, scales, packed.qweight, packed.weight_bytes, packed.aux, la, packed.bias, (OUTPUT, 0)),
+                      (rows, n, k, dcode, 3), (WORKSPACE, 0), nbytes))
+    return bound_call(steps, run, dtype=dtype, device=device, rows=rows, k=k, n=n, any_rank=True,
+                      workspace=lambda: native.workspace(device, nbytes, "gemm"), keep=(packed, workspace, la, column_scale),
+                      symbols="bound SVDQ W4A4 (xqt_b200_rotate_quantize / xqt_b200_lowrank_down / xqt_b200_w4a4_gemm)")
 
 
 __all__ = ["PackedSVDQW4A4Linear", "W4A4Workspace", "allocate_w4a4_workspace", "bind_svdq_w4a4_linear", "convrot_w4a4_linear",

@@ -19,6 +19,7 @@ import torch
 
 from .. import native
 from ..errors import XQTBackendError
+from ..hostcall import INPUT, OUTPUT, bound_call, step
 from ..quantize import Rotation, regular_rotation
 from .activation import rotate_quantize
 
@@ -324,8 +325,11 @@ def bind_convrot_w8a8_linear(packed: PackedConvRotW8A8Linear, workspace: ConvRot
             native.check(code, "bound ConvRot W8A8 (xqt_b200_rotate_quantize / xqt_b200_w8a8_gemm)")
         return out
 
-    run.keep = (packed, workspace, rot, column_scale, scratch)
-    return run
+    quantise = step("xqt_b200_rotate_quantize", ((INPUT, 0), *prologue[:4]), prologue[4:])
+    gemm = step("xqt_b200_w8a8_gemm_addend", (*gemm_head, 0, (OUTPUT, 0)), gemm_tail[:4], scratch, scratch.numel())
+    return bound_call([quantise, gemm], run, dtype=dtype, device=device, rows=rows, k=k, n=n, any_rank=True,
+                      keep=(packed, workspace, rot, column_scale, scratch),
+                      symbols="bound ConvRot W8A8 (xqt_b200_rotate_quantize / xqt_b200_w8a8_gemm)")
 
 
 __all__ = ["ConvRotW8A8Workspace", "FusedConvRotW8A8LinearGroup", "PackedConvRotW8A8Linear", "SharedConvRotW8A8Group", "allocate_convrot_w8a8_workspace", "bind_convrot_w8a8_linear",
