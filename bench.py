@@ -744,7 +744,7 @@ def measure_other_configs(device, world, rank, barrier) -> list:
     records.append(_record(
         "cfg4_w8a8_convrot", {"workload": "w8a8_convrot_linear_M2048_K4096_N4096", "rotation": "regular Hadamard 256", "world": 1},
         metric="w8a8_linear_throughput", unit="TOP/s", work=2.0 * m * n * k, us=t_full, bound="tensor", peak=i8_peak, peak_source=i8_kind,
-        kernel="gemm_i8_kernel (after rotate_quant_fast_kernel)", algorithmic="2*M*N*K over the full forward (rotate + quantise + GEMM)",
+        kernel="gemm_scaled_kernel (after act_prologue_i8_kernel)", algorithmic="2*M*N*K over the full forward (rotate + quantise + GEMM)",
         clocks=clocks, e2e=_e2e_us(x_host, full, barrier, 20, device), cpu=cpu,
         extra={"gemm_only": {"us_per_call": round(t_gemm, 2), "frac": round(2.0 * m * n * k / t_gemm / 1e6 / i8_peak, 4)}}))
     _log(f"w8a8: full {t_full:.1f} us, gemm {t_gemm:.1f} us")

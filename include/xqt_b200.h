@@ -260,6 +260,20 @@ int xqt_b200_rotate_quantize(const void* activation, const float* column_scale, 
                              float* scales, void* rotated, int m, int k, int rot_kind, int rot_block,
                              int quant_bits, int group_size, int act_dtype, xqt_b200_stream_t stream);
 
+/* The same prologue together with the down projection of a low-rank branch, one kernel: codes and scales as
+ * xqt_b200_rotate_quantize writes them in quant_bits 8, 9 or 6 (group 64), bit for bit, and from the same rotated, rounded
+ * activation la = lora_scale * x_rot * down^T (the quantise + "LoRA down" kernel of the reference,
+ * svdq_w4a4_sm89_kernel.cu:24-328, lora.cuh:110-243).
+ *   down     [32, K] act_dtype (rows past the rank zero) or NULL with la_form 0; K a multiple of 32
+ *   la_form  1: fp32 [M, 32];  2: the operand images xqt_b200_w4a4_gemm takes with flag 2 (ceil(M/128) x 16 KiB);
+ *            3: act_dtype [M, 64], columns 0..31 written (rounded once)
+ * xqt_b200_act_prologue_supported: rotation none or of 16..256 features (regular: 16, 64, 256), K a multiple of 16 (64 for
+ * mode 6), and for the int8 modes K at most about 20000. */
+int xqt_b200_act_prologue_supported(int k, int rot_kind, int rot_block, int mode);
+int xqt_b200_act_prologue(const void* activation, const float* column_scale, void* codes, float* scales, const void* down,
+                          void* la, float lora_scale, int m, int k, int rot_kind, int rot_block, int mode, int la_form,
+                          int act_dtype, xqt_b200_stream_t stream);
+
 /* Per-tensor dynamic int8 quantisation, the activation side of xqt's reference W8A8 linear Int8MmaLinear
  * (xqt/contracts/int8_mma.py:135-149,308-319): scale = max(absmax(activation), eps) / 127,
  * codes = clamp(rint(x / scale), -127, 127).  codes int8 [M,K]; row_scales fp32 [M] receives the scale
@@ -290,6 +304,12 @@ int xqt_b200_w8a8_gemm_addend(const void* act_codes, const void* weight_codes, c
                               const float* weight_scale, const float* bias, const float* addend,
                               void* output, int m, int n, int k, int out_dtype, void* workspace,
                               size_t workspace_bytes, xqt_b200_stream_t stream);
+/* The whole layer behind xqt_b200_act_prologue (mode 9, la_form 3): acc * a_s * w_s (+ bias) + la * up^T, one kernel.
+ *   la  out_dtype [M, 64], up  out_dtype [N, 64]: their first 32 columns enter, with fp32 sums */
+int xqt_b200_w8a8_gemm_lowrank(const void* act_codes, const void* weight_codes, const float* act_scale,
+                               const float* weight_scale, const float* bias, const void* la, const void* up,
+                               void* output, int m, int n, int k, int out_dtype, void* workspace,
+                               size_t workspace_bytes, xqt_b200_stream_t stream);
 int xqt_b200_lowrank_up(const void* la, const void* up, float* output, int m, int n, int rank_padded,
                         int act_dtype, void* workspace, size_t workspace_bytes, xqt_b200_stream_t stream);
 

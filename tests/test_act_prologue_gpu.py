@@ -1,0 +1,64 @@
+"""The fused activation prologue (rotation, quantisation, down projection) against the two-kernel form, whose codes and
+scales other tests hold to the oracle: codes and scales bit for bit, the down projection against fp32 torch."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+from conftest import seeded
+from xqt_b200 import native, quantize
+from xqt_b200.ops.activation import _KIND, _column_scale, rotate_quantize
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda", 0)
+ROTATIONS = {"none": None, "r16": quantize.regular_rotation(16), "r64": quantize.randomized_rotation(64, 3), "r256": quantize.regular_rotation(256),
+             "s32": quantize.randomized_rotation(32, 4), "s128": quantize.randomized_rotation(128, 5)}
+
+
+# rows: one, the remainders of a 4-row unit, and (2400, 1100) the 16- and 8-row CTAs; K: below and across a 256-feature chunk
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("m,k,rotation,mode", [
+    (1, 64, "r64", 6), (3, 320, "r64", 6), (5, 768, "s128", 6), (130, 3072, "r256", 6), (1100, 512, "s32", 6), (2400, 384, "s128", 6), (9, 192, "none", 6), (40, 8192, "s128", 6), (1400, 4096, "r64", 6),
+    (1, 64, "r16", 8), (6, 288, "s32", 8), (7, 2304, "r256", 8), (1100, 512, "s128", 8), (33, 544, "none", 8), (1300, 4096, "r256", 8), (3, 20480, "s32", 8), (2, 16384, "r64", 8),
+    (1, 32, "none", 9), (18, 4096, "none", 9), (1100, 1056, "none", 9), (2400, 640, "none", 9)])
+def test_matches_the_separate_kernels(m, k, rotation, mode, dtype):
+    rot = ROTATIONS[rotation]
+    x = torch.randn((m, k), generator=seeded(m + k)) * 3
+    x[:, ::37] *= 20
+    x[m // 2] = 0                                          # an all-zero token
+    x = x.to(DEV, dtype)
+    down = (torch.randn((32, k), generator=seeded(k)) * 0.05).to(DEV, dtype)
+    want_codes, want_scales, rotated = rotate_quantize(x, rot, bits=4 if mode == 6 else 8, sign_magnitude=mode == 6, tiled_scales=mode == 6,
+                                                       scale_in_act_dtype=mode == 9, return_rotated=True)
+    lib = native.library()
+    kind, block = _KIND[None if rot is None else rot.kind], 0 if rot is None else rot.block
+    assert lib.xqt_b200_act_prologue_supported(k, kind, block, mode)
+    column_scale = None if rot is None else _column_scale(rot, DEV)
+    want_la = 0.5 * rotated.float() @ down.float().t()
+    # the MMA's fp32 sums of K exact products: the error of a sum of K terms in fp32 is below K * 2^-24 of the sum of magnitudes
+    bound = 0.5 * k * 2.0 ** -24 * (rotated.float().abs() @ down.float().abs().t()) + 1e-30
+    for form in (0, 1, 2, 3):
+        codes = torch.full((m, k), 99, device=DEV, dtype=torch.int8)
+        scales = torch.full_like(want_scales, -1.0)
+        la = torch.zeros({0: (1,), 1: (m, 32), 2: (-(-m // 128) * 128, 32), 3: (m, 64)}[form], device=DEV, dtype=dtype if form == 3 else torch.float32)
+        native.check(lib.xqt_b200_act_prologue(
+            x.data_ptr(), native.ptr(column_scale), codes.data_ptr(), scales.data_ptr(), down.data_ptr() if form else 0, la.data_ptr() if form else 0,
+            0.5, m, k, kind, block, mode, form, native.DTYPE_CODE[dtype], native.stream_handle(DEV)), "xqt_b200_act_prologue")
+        assert torch.equal(codes, want_codes)
+        if mode == 6:                                      # tile-major: only the rows below M are written
+            order = lambda s: s.reshape(-1, k // 64, 128).permute(0, 2, 1).reshape(-1, k // 64)[:m]
+            assert torch.equal(order(scales), order(want_scales))
+        else:
+            assert torch.equal(scales, want_scales)
+        if form == 1:
+            assert ((la - want_la).abs() <= bound).all()
+            plain = la
+        elif form == 2:                                    # [hi | lo] bf16 rows, chunks swizzled by row
+            chunks = la.view(torch.bfloat16).reshape(-1, 8, 8)
+            index = torch.arange(8, device=DEV)[None] ^ (torch.arange(chunks.shape[0], device=DEV)[:, None] & 7)
+            straight = torch.gather(chunks, 1, index[:, :, None].expand_as(chunks)).reshape(-1, 64).float()[:m]
+            hi = plain.to(torch.bfloat16).float()
+            assert torch.equal(straight[:, :32], hi) and torch.equal(straight[:, 32:], (plain - hi).to(torch.bfloat16).float())
+        elif form == 3:
+            assert torch.equal(la[:, :32], plain.to(dtype)) and not la[:, 32:].any()

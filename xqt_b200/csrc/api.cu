@@ -40,10 +40,11 @@ int w4a4_expand_weight_launch(const void*, void*, int, int, cudaStream_t);
 size_t w4a4_aux_tile_bytes(int k);
 bool w4a4_gemm_supported(int m, int n, int k);
 int rotate_quant_launch(const void*, const float*, void*, float*, void*, int, int, int, int, int, int, int, cudaStream_t);
-int gemm_i8_launch(const void*, const void*, const float*, const float*, const float*, void*, int, int, int, int,
-                   unsigned int*, cudaStream_t);
-int gemm_i8_addend_launch(const void*, const void*, const float*, const float*, const float*, const float*, void*, int, int, int,
-                          int, unsigned int*, cudaStream_t);
+bool act_prologue_supported(int k, int rot_kind, int rot_block, int mode);
+int act_prologue_launch(const void*, const float*, void*, float*, const void*, void*, float, int, int, int, int, int, int, int,
+                        cudaStream_t);
+int gemm_scaled_launch(const void*, const void*, const float*, const float*, const float*, const float*, const void*, const void*, void*, int,
+                       int, int, int, unsigned int*, cudaStream_t);
 int gemm_f16_launch_strided(const void*, long long, const void*, long long, const float*, const void*, void*, int, int, int, int,
                             int, int, unsigned int*, cudaStream_t);
 size_t w4a4_dense_workspace_bytes(int m, int n, int k);
@@ -277,6 +278,19 @@ int xqt_b200_rotate_quantize(const void* activation, const float* column_scale, 
                              group_size, act_dtype, (cudaStream_t)stream);
 }
 
+int xqt_b200_act_prologue_supported(int k, int rot_kind, int rot_block, int mode) {
+  return act_prologue_supported(k, rot_kind, rot_block, mode) ? 1 : 0;
+}
+
+int xqt_b200_act_prologue(const void* activation, const float* column_scale, void* codes, float* scales, const void* down, void* la,
+                          float lora_scale, int m, int k, int rot_kind, int rot_block, int mode, int la_form, int act_dtype,
+                          xqt_b200_stream_t stream) {
+  if (m == 0) return 0;
+  XQT_REQUIRE(activation != nullptr && codes != nullptr && scales != nullptr);
+  return act_prologue_launch(activation, column_scale, codes, scales, down, la, lora_scale, m, k, rot_kind, rot_block, mode, la_form,
+                             act_dtype, (cudaStream_t)stream);
+}
+
 int xqt_b200_quantize_per_tensor(const void* activation, void* codes, float* row_scales, float* stats, int m, int k,
                                  int act_dtype, float eps, xqt_b200_stream_t stream) {
   if (m == 0) return 0;
@@ -289,8 +303,8 @@ int xqt_b200_w8a8_gemm(const void* act_codes, const void* weight_codes, const fl
                        void* workspace, size_t workspace_bytes, xqt_b200_stream_t stream) {
   if (m == 0) return 0;
   XQT_REQUIRE(workspace != nullptr && workspace_bytes >= 256);
-  return gemm_i8_launch(act_codes, weight_codes, act_scale, weight_scale, bias, output, m, n, k, out_dtype,
-                        reinterpret_cast<unsigned int*>(workspace), (cudaStream_t)stream);
+  return gemm_scaled_launch(act_codes, weight_codes, act_scale, weight_scale, bias, nullptr, nullptr, nullptr, output, m, n, k, out_dtype,
+                            reinterpret_cast<unsigned int*>(workspace), (cudaStream_t)stream);
 }
 
 int xqt_b200_w8a8_gemm_addend(const void* act_codes, const void* weight_codes, const float* act_scale,
@@ -298,8 +312,17 @@ int xqt_b200_w8a8_gemm_addend(const void* act_codes, const void* weight_codes, c
                               int k, int out_dtype, void* workspace, size_t workspace_bytes, xqt_b200_stream_t stream) {
   if (m == 0) return 0;
   XQT_REQUIRE(workspace != nullptr && workspace_bytes >= 256);
-  return gemm_i8_addend_launch(act_codes, weight_codes, act_scale, weight_scale, bias, addend, output, m, n, k, out_dtype,
-                               reinterpret_cast<unsigned int*>(workspace), (cudaStream_t)stream);
+  return gemm_scaled_launch(act_codes, weight_codes, act_scale, weight_scale, bias, addend, nullptr, nullptr, output, m, n, k, out_dtype,
+                            reinterpret_cast<unsigned int*>(workspace), (cudaStream_t)stream);
+}
+
+int xqt_b200_w8a8_gemm_lowrank(const void* act_codes, const void* weight_codes, const float* act_scale, const float* weight_scale,
+                               const float* bias, const void* la, const void* up, void* output, int m, int n, int k, int out_dtype,
+                               void* workspace, size_t workspace_bytes, xqt_b200_stream_t stream) {
+  if (m == 0) return 0;
+  XQT_REQUIRE(workspace != nullptr && workspace_bytes >= 256 && la != nullptr && up != nullptr);
+  return gemm_scaled_launch(act_codes, weight_codes, act_scale, weight_scale, bias, nullptr, la, up, output, m, n, k, out_dtype,
+                            reinterpret_cast<unsigned int*>(workspace), (cudaStream_t)stream);
 }
 
 int xqt_b200_lowrank_up(const void* la, const void* up, float* output, int m, int n, int rank_padded, int act_dtype,

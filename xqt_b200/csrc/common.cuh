@@ -52,6 +52,34 @@ inline int sm_count() {
   return cached[dev];
 }
 
+// Launch with programmatic stream serialisation: the kernel may start while the one before it in the stream drains.  It
+// has to execute griddepcontrol.wait (in every CTA) before it touches memory that an earlier kernel writes or reads.
+template <typename... Params, typename... Args>
+inline int launch_pdl_cluster(void (*kern)(Params...), dim3 grid, dim3 block, int cluster, size_t smem, cudaStream_t stream, Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cluster > 1) {
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)cluster;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.numAttrs = 2;
+  }
+  XQT_CUDA(cudaLaunchKernelEx(&cfg, kern, Params(args)...));
+  return launch_status();
+}
+template <typename... Params, typename... Args>
+inline int launch_pdl(void (*kern)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+  return launch_pdl_cluster(kern, grid, block, 1, smem, stream, args...);
+}
+
 __host__ __device__ constexpr int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
 template <typename T>

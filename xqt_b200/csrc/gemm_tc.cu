@@ -3,15 +3,13 @@
 // loop and double-buffered accumulators so the epilogue of one tile overlaps the main loop of the
 // next.  Y[M,N] = A[M,K] * B[N,K]^T with both operands K-major.
 //
-// Warp roles (192 threads, one CTA per SM):
+// Warp roles (320 threads, one CTA per SM):
 //   warp 0      TMA producer: one elected thread arms the stage barrier and issues two tiled loads
 //   warp 1      allocates tensor memory; one elected thread issues the MMAs and commits
 //   warps 2..9  epilogue: each owns one 32-lane quarter of tensor memory (quarter = warp % 4) and one
 //               half of the tile's columns (warps 2-5 the left half, 6-9 the right half)
 //
-// This file holds the int8 instantiation (W8A8: kind::i8, int32 accumulators over the whole K,
-// epilogue acc * a_scale[m] * w_scale[n] in fp32, the arithmetic of xqt's per-token int8 contract,
-// xqt/kernels/ops/gemm/reference.py:278-323 and quantize.py:60-131 written in its integer form).
+// Operands are fp16 or bf16 (both sides alike); the int8 GEMM of the W8A8 layers is gemm_scaled.cu.
 #include "common.cuh"
 #include "sm100.cuh"
 
@@ -31,12 +29,9 @@ enum Status : unsigned int { kOk = 0, kTimeout = 16 };
 struct GemmTcParams {
   int m, n, k;
   int mtiles, ntiles, kblocks, stages;
-  const float* row_scale;   // [M]  activation scale per token
-  const float* col_scale;   // [N]  weight scale per output channel
   const float* bias;        // [N] or null
-  const void* residual;     // [M, N] in the output dtype or null (fp16 kind only)
-  const float* addend;      // [M, N] fp32 or null (int8 kind only): added before the one rounding (a low-rank branch)
-  int out_f32;              // fp16 kind only: 1 = the output is fp32 (partial sums of a K-sharded layer)
+  const void* residual;     // [M, N] in the output dtype or null
+  int out_f32;              // 1 = the output is fp32 (partial sums of a K-sharded layer)
   void* out;                // [M, N]
   unsigned int* status;
 };
@@ -62,12 +57,10 @@ __device__ __forceinline__ void store8<__half>(__half* dst, const float (&v)[8])
   *reinterpret_cast<uint4*>(dst) = o;
 }
 
-// KIND 0: int8 operands, int32 accumulators, scaled epilogue.  KIND 1 / 2: fp16 / bf16 operands (both
-// sides the same format), fp32 accumulators, epilogue acc (+ bias) (+ residual).
+// KIND 1 / 2: fp16 / bf16 operands (both sides the same format), fp32 accumulators, epilogue acc (+ bias) (+ residual).
 template <int BN, typename OutT, int KIND>
 __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const GemmTcParams& p) {
   using namespace gemm;
-  constexpr bool I8 = KIND == 0;
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ __align__(8) unsigned long long bars[2 * kMaxStages + 4];
   __shared__ uint32_t s_tmem_base;
@@ -75,9 +68,8 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
 
   constexpr int kABytes = kBM * kRowBytes, kBBytes = BN * kRowBytes, kStageBytes = kABytes + kBBytes;
   constexpr uint32_t kTmemCols = 2 * BN;
-  constexpr uint32_t kIdesc = I8 ? umma_idesc(kAccS32, kFmtS8, kFmtS8, kBM, BN)
-                                 : (KIND == 1 ? umma_idesc(kAccF32, kFmtF16, kFmtF16, kBM, BN) : umma_idesc(kAccF32, kFmtBF16, kFmtBF16, kBM, BN));
-  constexpr int kElemsPerRow = I8 ? kRowBytes : kRowBytes / 2;   // K elements per 128-byte swizzle row
+  constexpr uint32_t kIdesc = KIND == 1 ? umma_idesc(kAccF32, kFmtF16, kFmtF16, kBM, BN) : umma_idesc(kAccF32, kFmtBF16, kFmtBF16, kBM, BN);
+  constexpr int kElemsPerRow = kRowBytes / 2;   // K elements per 128-byte swizzle row
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int ns = p.stages;
@@ -158,7 +150,7 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
           if (sn == ns) { sn = 0; pn ^= 1; }
           // four 32-byte K steps, the commit that frees the stage, and the poll of the next stage's
           // barrier in one go: the poll's round trip is hidden behind the MMA issue
-          ready = umma_ss_x4_commit_poll<I8>(d_tmem, adesc, bdesc, kIdesc, kb != 0 ? 1u : 0u, empty_bar(s), full_bar(sn), pn);
+          ready = umma_ss_x4_commit_poll<false>(d_tmem, adesc, bdesc, kIdesc, kb != 0 ? 1u : 0u, empty_bar(s), full_bar(sn), pn);
           if (last_tile && kb == p.kblocks - 1) ready = false;
           s = sn;
           phase = pn;
@@ -177,8 +169,6 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
       guarded_wait(tfull_bar(buf), (local >> 1) & 1);
       tc_fence_after();
       const int row = m0 + quarter * 32 + lane;
-      float rs = 0.f;
-      if (I8) rs = row < p.m ? __ldg(p.row_scale + row) : 0.f;
       const OutT* res = reinterpret_cast<const OutT*>(p.residual);
       const uint32_t taddr = tmem_base + buf * BN + ((uint32_t)(quarter * 32) << 16);
 #pragma unroll 1
@@ -192,20 +182,6 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
             const int col = n0 + c * 32 + j * 8;
             if (col < p.n) {   // N is a multiple of 8
               float v[8];
-              if (I8) {
-#pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                  v[e] = (float)(int)r[j * 8 + e] * (rs * __ldg(p.col_scale + col + e));
-                  if (p.bias != nullptr) v[e] += __ldg(p.bias + col + e);
-                }
-                if (p.addend != nullptr) {
-                  const float4* add = reinterpret_cast<const float4*>(p.addend + (size_t)row * p.n + col);
-                  const float4 a0 = __ldg(add), a1 = __ldg(add + 1);
-                  v[0] += a0.x; v[1] += a0.y; v[2] += a0.z; v[3] += a0.w;
-                  v[4] += a1.x; v[5] += a1.y; v[6] += a1.z; v[7] += a1.w;
-                }
-                store8<OutT>(out + (size_t)row * p.n + col, v);
-              } else {
 #pragma unroll
                 for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(r[j * 8 + e]);
                 if (p.bias != nullptr) {
@@ -225,7 +201,6 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
                 } else {
                   store8<OutT>(out + (size_t)row * p.n + col, v);
                 }
-              }
             }
           }
         }
@@ -238,12 +213,6 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
   tc_fence_before();
   __syncthreads();
   if (warp == 1) tmem_dealloc(tmem_base, kTmemCols);
-}
-
-template <int BN, typename OutT>
-__global__ void __launch_bounds__(gemm::kThreads, 1)
-gemm_i8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b, const GemmTcParams p) {
-  gemm_tc_body<BN, OutT, 0>(tm_a, tm_b, p);
 }
 
 // fp16 x fp16 -> fp32: the second pass of the W4A16 linear at large M (weights dequantised once per
@@ -319,10 +288,8 @@ template <int BN, typename OutT, int KIND>
 static int launch_tc(const void* a, long long lda, const void* b, long long ldb, GemmTcParams p, cudaStream_t stream) {
   using namespace gemm;
   CUtensorMap tm_a, tm_b;
-  constexpr bool I8 = KIND == 0;
-  const int esize = I8 ? 1 : 2;
-  const CUtensorMapDataType dt = I8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8
-                                    : (KIND == 1 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16);
+  constexpr int esize = 2;
+  const CUtensorMapDataType dt = KIND == 1 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
   XQT_CUDA((cudaError_t)make_tile_map_ld(&tm_a, a, dt, esize, p.m, p.k, lda, kBM));
   XQT_CUDA((cudaError_t)make_tile_map_ld(&tm_b, b, dt, esize, p.n, p.k, ldb, BN));
   constexpr int stage_bytes = kBM * kRowBytes + BN * kRowBytes;
@@ -333,38 +300,13 @@ static int launch_tc(const void* a, long long lda, const void* b, long long ldb,
   p.kblocks = ceil_div(p.k * esize, kRowBytes);
   const size_t smem_bytes = (size_t)p.stages * stage_bytes + 1024;
   void (*kern)(const CUtensorMap, const CUtensorMap, const GemmTcParams) =
-      I8 ? gemm_i8_kernel<BN, OutT> : (KIND == 1 ? gemm_f16_kernel<BN, OutT> : gemm_bf16_kernel<BN, OutT>);
+      KIND == 1 ? gemm_f16_kernel<BN, OutT> : gemm_bf16_kernel<BN, OutT>;
   XQT_SMEM_OPT_IN(kern, kSmemBudget);
   int grid = sm_count();
   if (grid > p.mtiles * p.ntiles) grid = p.mtiles * p.ntiles;
   kern<<<grid, kThreads, smem_bytes, stream>>>(tm_a, tm_b, p);
   return launch_status();
 }
-
-// int8 A [M,K] x int8 B [N,K]^T, out = acc * row_scale[m] * col_scale[n] (+ bias[n]) (+ addend[m,n], fp32)
-int gemm_i8_addend_launch(const void* a, const void* b, const float* row_scale, const float* col_scale, const float* bias,
-                          const float* addend, void* out, int m, int n, int k, int out_dtype, unsigned int* status,
-                          cudaStream_t stream);
-int gemm_i8_launch(const void* a, const void* b, const float* row_scale, const float* col_scale, const float* bias,
-                   void* out, int m, int n, int k, int out_dtype, unsigned int* status, cudaStream_t stream) {
-  return gemm_i8_addend_launch(a, b, row_scale, col_scale, bias, nullptr, out, m, n, k, out_dtype, status, stream);
-}
-int gemm_i8_addend_launch(const void* a, const void* b, const float* row_scale, const float* col_scale, const float* bias,
-                          const float* addend, void* out, int m, int n, int k, int out_dtype, unsigned int* status,
-                          cudaStream_t stream) {
-  XQT_REQUIRE(m > 0 && n > 0 && k > 0 && k % 16 == 0 && n % 8 == 0 && ((uintptr_t)addend & 15) == 0);
-  XQT_REQUIRE(out_dtype == XQT_B200_BF16 || out_dtype == XQT_B200_FP16);
-  XQT_REQUIRE(a != nullptr && b != nullptr && row_scale != nullptr && col_scale != nullptr && out != nullptr && status != nullptr);
-  XQT_REQUIRE(((uintptr_t)out & 15) == 0);
-  GemmTcParams p{};
-  p.m = m; p.n = n; p.k = k;
-  p.row_scale = row_scale; p.col_scale = col_scale; p.bias = bias; p.addend = addend; p.out = out; p.status = status;
-  const bool wide = (n % 256 == 0);
-  if (out_dtype == XQT_B200_BF16)
-    return wide ? launch_tc<256, __nv_bfloat16, 0>(a, k, b, k, p, stream) : launch_tc<128, __nv_bfloat16, 0>(a, k, b, k, p, stream);
-  return wide ? launch_tc<256, __half, 0>(a, k, b, k, p, stream) : launch_tc<128, __half, 0>(a, k, b, k, p, stream);
-}
-
 
 // 16-bit A [M,K] x 16-bit B [N,K]^T (both fp16, or both bf16 with operand_bf16) with fp32
 // accumulation; out = acc (+ bias[n]) (+ residual[m,n]) in bf16 / fp16 (out_dtype) or fp32 (out_f32).

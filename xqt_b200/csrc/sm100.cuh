@@ -71,6 +71,14 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
   return false;
 }
 
+// The same by polling: a role that sets a pipeline's pace (MMA issuer, producer) must not be suspended, the wake-up of
+// try_wait lags the barrier.  False when the attempt limit (seconds) ran out.
+__device__ __forceinline__ bool mbar_spin(uint32_t bar, uint32_t parity) {
+  for (uint32_t i = 0; i < (kSpinLimit << 3); ++i)
+    if (mbar_test_wait(bar, parity)) return true;
+  return false;
+}
+
 // Two barriers at once.  A try_wait takes about 150 cycles to return its predicate even when the
 // phase has already completed, but independent ones pipeline: polling both in one go costs one
 // round trip instead of two.
@@ -381,6 +389,74 @@ __device__ __forceinline__ void umma_ts_f16(uint32_t d_tmem, uint32_t a_tmem, ui
 // arrive on `bar` once every tcgen05.mma issued so far by this thread has completed
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar) : "memory");
+}
+
+
+// ---------------------------------------------------------------- CTA pairs (cta_group::2)
+// The two CTAs of a cluster of two run one MMA: each holds its half of both operands in shared memory at the same offsets
+// and its 128 rows of the accumulators in tensor memory; the even-ranked CTA (the leader) issues.  CG is the group size.
+template <int CG>
+__device__ __forceinline__ void tmem_alloc_cg(uint32_t slot_smem, uint32_t cols) {
+  if constexpr (CG == 1) tmem_alloc(slot_smem, cols);
+  else asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(slot_smem), "r"(cols) : "memory");
+}
+template <int CG>
+__device__ __forceinline__ void tmem_relinquish_cg() {
+  if constexpr (CG == 1) tmem_relinquish();
+  else asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;\n" ::: "memory");
+}
+template <int CG>
+__device__ __forceinline__ void tmem_dealloc_cg(uint32_t base, uint32_t cols) {
+  if constexpr (CG == 1) tmem_dealloc(base, cols);
+  else asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;\n" ::"r"(base), "r"(cols) : "memory");
+}
+// 2-D tiled load into this CTA's shared memory whose bytes are counted on `bar`, a shared::cluster address that may be the
+// pair leader's barrier
+template <int CG>
+__device__ __forceinline__ void tma_load_2d_cg(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
+  if constexpr (CG == 1) tma_load_2d(dst, map, c0, c1, bar);
+  else
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n" ::"r"(dst),
+        "l"(map), "r"(c0), "r"(c1), "r"(bar)
+        : "memory");
+}
+// arrive on `bar` (the same offset in both CTAs of a pair) once the MMAs this thread has issued are complete
+template <int CG>
+__device__ __forceinline__ void umma_commit_cg(uint32_t bar) {
+  if constexpr (CG == 1) umma_commit(bar);
+  else
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n" ::"r"(bar), "h"((uint16_t)3)
+                 : "memory");
+}
+enum : int { kMmaI8 = 0, kMmaF16 = 1, kMmaF8 = 2 };
+template <int CG, int KIND>
+__device__ __forceinline__ void umma_ss_cg(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+#define XQT_UMMA(GROUP, NAME)                                                                                   \
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"                                             \
+               "tcgen05.mma.cta_group::" GROUP ".kind::" NAME " [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),    \
+               "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)                                              \
+               : "memory")
+  if constexpr (CG == 1 && KIND == kMmaI8) XQT_UMMA("1", "i8");
+  if constexpr (CG == 1 && KIND == kMmaF16) XQT_UMMA("1", "f16");
+  if constexpr (CG == 1 && KIND == kMmaF8) XQT_UMMA("1", "f8f6f4");
+  if constexpr (CG == 2 && KIND == kMmaI8) XQT_UMMA("2", "i8");
+  if constexpr (CG == 2 && KIND == kMmaF16) XQT_UMMA("2", "f16");
+  if constexpr (CG == 2 && KIND == kMmaF8) XQT_UMMA("2", "f8f6f4");
+#undef XQT_UMMA
+}
+// arrive on a barrier of another CTA of the cluster (address from cluster_map)
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t caddr) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(caddr) : "memory");
+}
+__device__ __forceinline__ void st_cluster_b128(uint32_t caddr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};\n" ::"r"(caddr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+// 32 bytes to global memory (32-byte aligned): one full sector per thread
+__device__ __forceinline__ void stg256(void* p, const uint32_t (&v)[8]) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]),
+               "r"(v[5]), "r"(v[6]), "r"(v[7])
+               : "memory");
 }
 
 }  // namespace sm100

@@ -8,6 +8,7 @@ Pointer arguments are addresses of tensors that the callable keeps, or one of th
 from __future__ import annotations
 
 import ctypes
+import struct
 import weakref
 
 import torch
@@ -19,7 +20,8 @@ INPUT, OUTPUT, RESIDUAL, SCRATCH, WORKSPACE = 1, 2, 3, 4, 5      # csrc/host.cpp
 # entry -> the step's number in csrc/host.cpp (Op)
 _OPS = {name: i for i, name in enumerate((
     "xqt_b200_w4a16_decode_lanes", "xqt_b200_w4a16_run", "xqt_b200_swiglu", "xqt_b200_rotate_quantize",
-    "xqt_b200_w8a8_gemm_addend", "xqt_b200_lowrank_down", "xqt_b200_w4a4_gemm"))}
+    "xqt_b200_w8a8_gemm_addend", "xqt_b200_lowrank_down", "xqt_b200_w4a4_gemm", "xqt_b200_act_prologue",
+    "xqt_b200_w8a8_gemm_lowrank"))}
 
 
 def step(symbol: str, pointers: tuple, integers: tuple, workspace=0, workspace_bytes: int = 0) -> tuple:
@@ -30,6 +32,12 @@ def step(symbol: str, pointers: tuple, integers: tuple, workspace=0, workspace_b
     address = ctypes.cast(getattr(native.library(), symbol), ctypes.c_void_p).value
     workspace = workspace.data_ptr() if isinstance(workspace, torch.Tensor) else workspace
     return (_OPS[symbol], address, resolved, tuple(int(v) for v in integers), workspace, int(workspace_bytes))
+
+
+def float_bits(value: float) -> int:
+    """The integer a step passes for a float argument."""
+
+    return struct.unpack("i", struct.pack("f", float(value)))[0]
 
 
 class ScratchPlan:
@@ -72,4 +80,4 @@ def bound_call(steps: list, slow, *, dtype: torch.dtype, device: torch.device, r
         any_rank=any_rank, takes_residual=residual, scratch_bytes=int(scratch_bytes), workspace=workspace, keep=keep)
 
 
-__all__ = ["INPUT", "OUTPUT", "RESIDUAL", "SCRATCH", "WORKSPACE", "ScratchPlan", "bound_call", "step", "weak_method"]
+__all__ = ["INPUT", "OUTPUT", "RESIDUAL", "SCRATCH", "WORKSPACE", "ScratchPlan", "bound_call", "float_bits", "step", "weak_method"]

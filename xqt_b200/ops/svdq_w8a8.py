@@ -2,10 +2,9 @@
 (xqt/kernels/ops/_impl/cute/svdq_w8a8_sm89.py): ``pack_svdq_w8a8_linear``, ``allocate_svdq_w8a8_workspace``,
 ``svdq_w8a8_linear``, ``bind_svdq_w8a8_linear``, ``w8a8_linear`` and the ``native_svdq_w8a8_*`` probes.
 
-    s_a[m] = T(amax_m / 127),  q_a = clamp(rint(x / s_a))          rotate_quant kernel, mode 9 (no rotation)
-    la     = x down^T            (fp32 [M, 32])                      lowrank_down_kernel
-    low    = T(lora_scale la) up^T   (fp32 [M, N])                   dense tcgen05 GEMM, bf16/fp16 operands
-    y      = T(int32(q_a q_w^T) s_a s_w + bias + low)                gemm_i8_kernel, fp32 addend in the epilogue
+    s_a[m] = T(amax_m / 127),  q_a = clamp(rint(x / s_a)),  la = T(lora_scale x down^T)     act_prologue_i8_kernel, mode 9
+    y      = T(int32(q_a q_w^T) s_a s_w + bias + la up^T)                                   gemm_scaled_kernel: both products on
+                                                                                            the tensor cores, fp32 sums for la up^T
 
 The reference's kernels are svdq_w8a8_sm89_kernel.cu (quantize_act_lora / gemm_lora); it multiplies by approximate
 reciprocals of the scales where this path divides (IEEE), which can move a code that sits on a rounding boundary."""
@@ -18,7 +17,7 @@ import torch
 
 from .. import native
 from ..errors import XQTBackendError
-from .activation import rotate_quantize
+from ..hostcall import INPUT, OUTPUT, bound_call, float_bits, step
 
 RANK_PAD = 32          # the down projection's width
 UP_PAD = 64            # the up projection's K extent (one 64-element tensor-core K block)
@@ -45,9 +44,7 @@ class PackedSVDQW8A8Linear:
 class W8A8SVDQWorkspace:
     quantized_activation: torch.Tensor     # int8 [rows, K]
     activation_scales: torch.Tensor        # fp32 [rows]
-    lora_activation: torch.Tensor          # fp32 [rows, 32]
     lora_activation16: torch.Tensor        # dtype [rows, 64], columns past 32 stay zero
-    low_rank_output: torch.Tensor          # fp32 [rows, N]
 
     @property
     def padded_rows(self) -> int:
@@ -103,13 +100,11 @@ def pack_svdq_w8a8_linear(residual_weight: torch.Tensor, down_weight: torch.Tens
 
 
 def allocate_svdq_w8a8_workspace(rows: int, packed: PackedSVDQW8A8Linear) -> W8A8SVDQWorkspace:
-    rows, k, n, device = int(rows), packed.input_features, packed.output_features, packed.qweight.device
+    rows, k, device = int(rows), packed.input_features, packed.qweight.device
     return W8A8SVDQWorkspace(
         quantized_activation=torch.empty((rows, k), dtype=torch.int8, device=device),
         activation_scales=torch.empty((rows,), dtype=torch.float32, device=device),
-        lora_activation=torch.empty((rows, RANK_PAD), dtype=torch.float32, device=device),
-        lora_activation16=torch.zeros((rows, UP_PAD), dtype=packed.dtype, device=device),
-        low_rank_output=torch.empty((rows, n), dtype=torch.float32, device=device))
+        lora_activation16=torch.zeros((rows, UP_PAD), dtype=packed.dtype, device=device))
 
 
 def _forward(inputs: torch.Tensor, packed: PackedSVDQW8A8Linear, workspace: W8A8SVDQWorkspace | None, lora_scale: float,
@@ -126,26 +121,22 @@ def _forward(inputs: torch.Tensor, packed: PackedSVDQW8A8Linear, workspace: W8A8
     if m == 0:
         return out
     ws = workspace or allocate_svdq_w8a8_workspace(m, packed)
-    if ws.padded_rows < m or int(ws.quantized_activation.shape[1]) != k or int(ws.low_rank_output.shape[1]) != n:
+    if ws.padded_rows < m or int(ws.quantized_activation.shape[1]) != k:
         raise ValueError("workspace extent does not match inputs")
-    codes, scales = rotate_quantize(x, None, bits=8, out=(ws.quantized_activation, ws.activation_scales), scale_in_act_dtype=True)
+    codes, scales, la = ws.quantized_activation[:m], ws.activation_scales[:m], ws.lora_activation16[:m]
     lib, stream, dcode = native.library(), native.stream_handle(device), native.DTYPE_CODE[packed.dtype]
-    low_ptr = 0
+    low_rank = low_rank and bool(packed.rank)
     with torch.cuda.device(device):
         scratch = native.workspace(device, 256, "gemm")
-        if low_rank and packed.rank:
-            la, la16, low = ws.lora_activation[:m], ws.lora_activation16[:m], ws.low_rank_output[:m]
-            native.check(lib.xqt_b200_lowrank_down(x.data_ptr(), packed.down.data_ptr(), la.data_ptr(), 0, m, k, dcode, stream),
-                         "xqt_b200_lowrank_down")
-            if lora_scale != 1.0:
-                la.mul_(float(lora_scale))
-            la16[:, :RANK_PAD].copy_(la)                     # the rounding to the activation dtype
-            native.check(lib.xqt_b200_lowrank_up(la16.data_ptr(), packed.up.data_ptr(), low.data_ptr(), m, n, UP_PAD, dcode,
-                                                 scratch.data_ptr(), scratch.numel(), stream), "xqt_b200_lowrank_up")
-            low_ptr = low.data_ptr()
-        native.check(lib.xqt_b200_w8a8_gemm_addend(
-            codes.data_ptr(), packed.qweight.data_ptr(), scales.data_ptr(), packed.weight_scales.data_ptr(), native.ptr(packed.bias),
-            low_ptr, out.data_ptr(), m, n, k, dcode, scratch.data_ptr(), scratch.numel(), stream), "xqt_b200_w8a8_gemm_addend")
+        native.check(lib.xqt_b200_act_prologue(x.data_ptr(), 0, codes.data_ptr(), scales.data_ptr(), packed.down.data_ptr() if low_rank else 0,
+                                               la.data_ptr() if low_rank else 0, lora_scale, m, k, 0, 0, 9, 3 if low_rank else 0, dcode, stream),
+                     "xqt_b200_act_prologue")
+        head = (codes.data_ptr(), packed.qweight.data_ptr(), scales.data_ptr(), packed.weight_scales.data_ptr(), native.ptr(packed.bias))
+        tail = (out.data_ptr(), m, n, k, dcode, scratch.data_ptr(), scratch.numel(), stream)
+        if low_rank:
+            native.check(lib.xqt_b200_w8a8_gemm_lowrank(*head, la.data_ptr(), packed.up.data_ptr(), *tail), "xqt_b200_w8a8_gemm_lowrank")
+        else:
+            native.check(lib.xqt_b200_w8a8_gemm(*head, *tail), "xqt_b200_w8a8_gemm")
     if return_parts:
         return out, {"codes": codes, "scales": scales}
     return out
@@ -175,47 +166,31 @@ def bind_svdq_w8a8_linear(packed: PackedSVDQW8A8Linear, workspace: W8A8SVDQWorks
     if workspace.padded_rows < rows:
         raise ValueError("workspace row extent does not match rows")
     k, n, dtype, device, scale = packed.input_features, packed.output_features, packed.dtype, packed.qweight.device, float(lora_scale)
-    # every pointer and code of the library calls is resolved here; a call checks its input, allocates its output and
-    # makes the calls (the general entry's per-call validation costs more host time than the kernels run)
-    lib, dcode = native.library(), native.DTYPE_CODE[dtype]
-    index = device.index if device.index is not None else torch.cuda.current_device()
-    codes, scales = workspace.quantized_activation[:rows], workspace.activation_scales[:rows]
-    la, la16, low = workspace.lora_activation[:rows], workspace.lora_activation16[:rows], workspace.low_rank_output[:rows]
-    la16_head = la16[:, :RANK_PAD]
+    if int(workspace.quantized_activation.shape[1]) != k:
+        raise ValueError("workspace extent does not match the packed layer")
+    dcode = native.DTYPE_CODE[dtype]
+    codes, scales, la = workspace.quantized_activation, workspace.activation_scales, workspace.lora_activation16
     scratch = native.workspace(device, 256, "gemm")
-    quant_tail = (0, codes.data_ptr(), scales.data_ptr(), 0, rows, k, 0, 0, 9, 0, dcode)
-    down_args = (packed.down.data_ptr(), la.data_ptr(), 0, rows, k, dcode)
-    up_args = (la16.data_ptr(), packed.up.data_ptr(), low.data_ptr(), rows, n, UP_PAD, dcode, scratch.data_ptr(), scratch.numel())
-    gemm_head = (codes.data_ptr(), packed.qweight.data_ptr(), scales.data_ptr(), packed.weight_scales.data_ptr(), native.ptr(packed.bias),
-                 low.data_ptr() if packed.rank else 0)
-    gemm_tail = (rows, n, k, dcode, scratch.data_ptr(), scratch.numel())
-    has_rank = bool(packed.rank)
 
     def run(inputs: torch.Tensor) -> torch.Tensor:
         if inputs.dtype != dtype or inputs.device != device or inputs.ndim != 2 or tuple(inputs.shape) != (rows, k) \
                 or not inputs.is_contiguous():
             raise XQTBackendError("bound SVDQ W8A8 call: input shape, dtype, device or layout mismatch")
-        if torch.cuda.current_device() != index:
+        if torch.cuda.current_device() != (device.index if device.index is not None else torch.cuda.current_device()):
             raise XQTBackendError("bound SVDQ W8A8 call: make the weight's device current before calling")
-        out = torch.empty((rows, n), device=device, dtype=dtype)
-        stream = torch.cuda.current_stream(device).cuda_stream
-        x_ptr = inputs.data_ptr()
-        code = lib.xqt_b200_rotate_quantize(x_ptr, *quant_tail, stream)
-        if code == 0 and has_rank:
-            code = lib.xqt_b200_lowrank_down(x_ptr, *down_args, stream)
-            if code == 0:
-                if scale != 1.0:
-                    la.mul_(scale)
-                la16_head.copy_(la)                          # the rounding to the activation dtype
-                code = lib.xqt_b200_lowrank_up(*up_args, stream)
-        if code == 0:
-            code = lib.xqt_b200_w8a8_gemm_addend(*gemm_head, out.data_ptr(), *gemm_tail, stream)
-        if code != 0:
-            native.check(code, "bound SVDQ W8A8 (quantise / low-rank / GEMM)")
-        return out
+        return _forward(inputs, packed, workspace, scale, True)
 
-    run.keep = (packed, workspace, scratch)
-    return run
+    low_rank = bool(packed.rank)
+    quantise = step("xqt_b200_act_prologue", ((INPUT, 0), 0, codes, scales, packed.down if low_rank else 0, la if low_rank else 0),
+                    (float_bits(scale), rows, k, 0, 0, 9, 3 if low_rank else 0, dcode))
+    if low_rank:
+        gemm = step("xqt_b200_w8a8_gemm_lowrank", (codes, packed.qweight, scales, packed.weight_scales, packed.bias, la, packed.up, (OUTPUT, 0)),
+                    (rows, n, k, dcode), scratch, scratch.numel())
+    else:
+        gemm = step("xqt_b200_w8a8_gemm_addend", (codes, packed.qweight, scales, packed.weight_scales, packed.bias, 0, (OUTPUT, 0)),
+                    (rows, n, k, dcode), scratch, scratch.numel())
+    return bound_call([quantise, gemm], run, dtype=dtype, device=device, rows=rows, k=k, n=n, keep=(packed, workspace, scratch),
+                      symbols="bound SVDQ W8A8 (quantise / GEMM)")
 
 
 __all__ = ["PackedSVDQW8A8Linear", "W8A8SVDQWorkspace", "allocate_svdq_w8a8_workspace", "bind_svdq_w8a8_linear",

@@ -27,7 +27,7 @@ import torch
 
 from .. import native
 from ..errors import XQTBackendError
-from ..hostcall import INPUT, OUTPUT, WORKSPACE, bound_call, step
+from ..hostcall import INPUT, OUTPUT, WORKSPACE, bound_call, float_bits, step
 from ..quantize import Rotation, quantize_residual_int4
 from .activation import _KIND, _column_scale, rotate_quantize
 
@@ -236,8 +236,19 @@ def svdq_w4a4_linear(inputs: torch.Tensor, packed: PackedSVDQW4A4Linear, *, work
     # the GEMM call launches no preparation kernel; callers that want the parts back, or scale the low-rank
     # activations, take the row-major forms.
     direct = not dense and not return_parts and lora_scale == 1.0
-    codes, scales, rotated = rotate_quantize(x, packed.rotation, bits=4, group_size=GROUP if packed.act_granularity == "group" else 0,
-                                             return_rotated=True, out=buffers, sign_magnitude=not dense, tiled_scales=direct)
+    rot = packed.rotation
+    kind, block = _KIND[None if rot is None else rot.kind], 0 if rot is None else rot.block
+    # one kernel for rotation, quantisation and down projection where it serves the options
+    fused = direct and packed.act_granularity == "group" and x.dtype == packed.dtype and x.is_cuda and bool(packed.rank) \
+        and bool(lib.xqt_b200_act_prologue_supported(k, kind, block, 6))
+    if fused:
+        if buffers is None:
+            buffers = (torch.empty((m, k), device=device, dtype=torch.int8),
+                       torch.empty((-(-m // TILE) * TILE, k // GROUP), device=device, dtype=torch.float32))
+        codes, scales = buffers[0], buffers[1]
+    else:
+        codes, scales, rotated = rotate_quantize(x, packed.rotation, bits=4, group_size=GROUP if packed.act_granularity == "group" else 0,
+                                                 return_rotated=True, out=buffers, sign_magnitude=not dense, tiled_scales=direct)
     if workspace is not None and workspace.lora_activation is not None:
         la = workspace.lora_activation          # rows past M stay zero: the kernels only write rows < M
     elif direct and packed.rank:
@@ -253,7 +264,12 @@ def svdq_w4a4_linear(inputs: torch.Tensor, packed: PackedSVDQW4A4Linear, *, work
     with torch.cuda.device(device):
         scratch = native.workspace(device, lib.xqt_b200_w4a4_dense_workspace_bytes(m, n, k) if dense else
                                    lib.xqt_b200_w4a4_workspace_bytes(m, n, k), "gemm")
-        if packed.rank:
+        if fused:
+            column_scale = None if rot is None else _column_scale(rot, device)
+            native.check(lib.xqt_b200_act_prologue(x.data_ptr(), native.ptr(column_scale), codes.data_ptr(), scales.data_ptr(), packed.down.data_ptr(),
+                                                   la.data_ptr(), 1.0, m, k, kind, block, 6, 2, native.DTYPE_CODE[packed.dtype], stream),
+                         "xqt_b200_act_prologue")
+        elif packed.rank:
             if dense:
                 native.check(lib.xqt_b200_lowrank_down_tc(
                     rotated.data_ptr(), packed.down.data_ptr(), la.data_ptr(), m, k, native.DTYPE_CODE[packed.dtype],
@@ -341,11 +357,16 @@ def bind_svdq_w4a4_linear(packed: PackedSVDQW4A4Linear, workspace: W4A4Workspace
         la = torch.zeros((-(-rows // TILE) * TILE, RANK_PAD), device=device, dtype=torch.float32)
     column_scale = None if rot is None else _column_scale(rot, device)
     codes, scales, rotated = workspace.quantized_activation, workspace.activation_scales, workspace.rotated_activation
-    steps = [step("xqt_b200_rotate_quantize", ((INPUT, 0), column_scale, codes, scales, rotated),
-                  (rows, k, _KIND[None if rot is None else rot.kind], 0 if rot is None else rot.block, 6,
-                   GROUP if packed.act_granularity == "group" else 0, dcode))]
-    if packed.rank:
-        steps.append(step("xqt_b200_lowrank_down", (rotated, packed.down, 0, la), (rows, k, dcode)))
+    kind, block = _KIND[None if rot is None else rot.kind], 0 if rot is None else rot.block
+    if packed.act_granularity == "group" and lib.xqt_b200_act_prologue_supported(k, kind, block, 6):
+        steps = [step("xqt_b200_act_prologue", ((INPUT, 0), column_scale, codes, scales, packed.down if packed.rank else 0,
+                                                la if packed.rank else 0),
+                      (float_bits(1.0), rows, k, kind, block, 6, 2 if packed.rank else 0, dcode))]
+    else:
+        steps = [step("xqt_b200_rotate_quantize", ((INPUT, 0), column_scale, codes, scales, rotated),
+                      (rows, k, kind, block, 6, GROUP if packed.act_granularity == "group" else 0, dcode))]
+        if packed.rank:
+            steps.append(step("xqt_b200_lowrank_down", (rotated, packed.down, 0, la), (rows, k, dcode)))
     nbytes = lib.xqt_b200_w4a4_workspace_bytes(rows, n, k)
     steps.append(step("xqt_b200_w4a4_gemm", (codes, scales, packed.qweight, packed.weight_bytes, packed.aux, la, packed.bias, (OUTPUT, 0)),
                       (rows, n, k, dcode, 3), (WORKSPACE, 0), nbytes))
