@@ -1,11 +1,10 @@
-// Fused W4A16 GEMM for 17 <= M <= 512 tokens on tcgen05:
+// Fused W4A16 GEMM for 17 <= M <= 128 tokens on tcgen05 (more tokens: gemm_w4a16_pair.cu):
 //   Y[M,N] = X[M,K] * dequant(W)[N,K]^T, weights read straight from the canonical xqt_int4_nk_v1 bytes and
 // dequantised in registers on their way to the tensor core -- no N*K*2 scratch, no second pass.
 //
-// A CTA tile is 128 output channels x up to 256 tokens (MT = 1 or 2 blocks of 128 rows that share ONE
-// dequantised weight tile): for M <= 256 every packed weight is read and converted exactly once per call; a
-// larger M is cut into 256-token chunks.  Per 64-K stage
-//   * TMA brings the activation blocks [MT x 128 x 64] fp16 (128-byte swizzle) and, through a deeper ring
+// A CTA tile is 128 output channels x all (up to 128) tokens: every packed weight is read and converted exactly once per
+// call.  Per 64-K stage
+//   * TMA brings the activations [128 x 64] fp16 (128-byte swizzle) and, through a deeper ring
 //     of its own, the packed weights of the stage (128 rows x 32 bytes, plain layout);
 //   * eight dequantisation warps turn the nibbles into fp16 values (code - zero) * scale -- the zero point
 //     folded into the exact magic-number subtraction, one rounding in the multiply -- and store them in the
@@ -13,8 +12,8 @@
 //     stages it = g (mod 4), a thread on two weight rows: converting a stage is a chain of waits (two barrier
 //     tests of ~200 cycles, the scale loads, the proxy fence) that one warp cannot overlap with itself, so four
 //     stages are in conversion at any time;
-//   * one thread issues 4 x MT MMAs (K = 16, kind::f16, fp32 accumulators in tensor memory, 128 columns per
-//     token block, the tile's accumulators double-buffered so the epilogue overlaps the next tile).
+//   * one thread issues 4 MMAs (K = 16, kind::f16, fp32 accumulators in tensor memory, the tile's accumulators
+//     double-buffered so the epilogue overlaps the next tile).
 // Warps (480 threads): 0 activation producer, 1 MMA issuer, 2-5 epilogue, 6-13 dequantisation, 14 packed-weight
 // producer.  What the pipeline's rate depended on, measured with cycle stamps (down projection 4096 x 14336 at M = 64:
 // 76 -> 43 us; gate/up 28672 x 4096: 133 -> 63 us): the packed-weight ring needs a producer of its own (one thread
@@ -33,6 +32,7 @@
 // (csrc/quantization/w4a16_fused_kernel.cu) on this range of M.
 #include "common.cuh"
 #include "sm100.cuh"
+#include "w4a16_dequant.cuh"
 
 namespace xqt_b200 {
 
@@ -60,92 +60,33 @@ constexpr int kBarTileFull = kBarRawEmpty + kMaxRaw, kBarTileEmpty = kBarTileFul
 
 struct W4FusedParams {
   int m, n, k, group_size, groups;
-  int mchunks, ntiles, splits, kb_per_split, kblocks, stages, raw_bufs;
+  int ntiles, splits, kb_per_split, kblocks, stages, raw_bufs;
   int param_dtype, nibble_signed, out_f32;
   const void* scales;
   const void* zeros;
   const float* bias;
   const void* residual;
   void* out;
-  float* partials;          // [tiles][splits][MT*128][128] fp32 (splits > 1)
+  float* partials;          // [tiles][splits][128][128] fp32 (splits > 1)
   unsigned int* tickets;    // [tiles], zero between calls
   unsigned int* status;
 };
 
-template <typename OutT>
-__device__ __forceinline__ void w4f_store8(OutT* dst, const float (&v)[8]);
-template <>
-__device__ __forceinline__ void w4f_store8<__nv_bfloat16>(__nv_bfloat16* dst, const float (&v)[8]) {
-  uint4 o;
-  __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), b = __floats2bfloat162_rn(v[2], v[3]);
-  __nv_bfloat162 c = __floats2bfloat162_rn(v[4], v[5]), d = __floats2bfloat162_rn(v[6], v[7]);
-  o.x = *reinterpret_cast<uint32_t*>(&a); o.y = *reinterpret_cast<uint32_t*>(&b);
-  o.z = *reinterpret_cast<uint32_t*>(&c); o.w = *reinterpret_cast<uint32_t*>(&d);
-  *reinterpret_cast<uint4*>(dst) = o;
-}
-template <>
-__device__ __forceinline__ void w4f_store8<__half>(__half* dst, const float (&v)[8]) {
-  uint4 o;
-  __half2 a = __floats2half2_rn(v[0], v[1]), b = __floats2half2_rn(v[2], v[3]);
-  __half2 c = __floats2half2_rn(v[4], v[5]), d = __floats2half2_rn(v[6], v[7]);
-  o.x = *reinterpret_cast<uint32_t*>(&a); o.y = *reinterpret_cast<uint32_t*>(&b);
-  o.z = *reinterpret_cast<uint32_t*>(&c); o.w = *reinterpret_cast<uint32_t*>(&d);
-  *reinterpret_cast<uint4*>(dst) = o;
-}
-template <typename T>
-__device__ __forceinline__ void w4f_load8(const T* src, float (&v)[8]) {
-  const uint4 raw = *reinterpret_cast<const uint4*>(src);
-  const T* e = reinterpret_cast<const T*>(&raw);
-#pragma unroll
-  for (int i = 0; i < 8; ++i) v[i] = to_float<T>(e[i]);
-}
-
-// 8 nibbles of `word` (k0..k7, canonical order) -> fp16 (code - zero) * scale as 4 registers in K order
-__device__ __forceinline__ uint4 w4f_dequant_word(uint32_t word, __half2 off2, __half2 scale2) {
-  uint32_t d[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    uint32_t r;
-    asm("lop3.b32 %0, %1, %2, %3, 0xea;\n" : "=r"(r) : "r"(word >> (4 * i)), "n"(0x000f000f), "n"(0x64006400));
-    __half2 v = __hmul2(__hsub2(*reinterpret_cast<__half2*>(&r), off2), scale2);   // (k_i, k_{i+4})
-    d[i] = *reinterpret_cast<uint32_t*>(&v);
-  }
-  uint4 o;
-  o.x = __byte_perm(d[0], d[1], 0x5410);   // (k0, k1)
-  o.y = __byte_perm(d[2], d[3], 0x5410);   // (k2, k3)
-  o.z = __byte_perm(d[0], d[1], 0x7632);   // (k4, k5)
-  o.w = __byte_perm(d[2], d[3], 0x7632);   // (k6, k7)
-  return o;
-}
-
-// tile -> (token chunk, channel tile, K split); the splits of one output tile are adjacent CTAs
+// tile -> (channel tile, K split); the splits of one output tile are adjacent CTAs
 struct W4FTile {
-  int mc, nt, sp, kb0, kbn, out_tile;
+  int nt, sp, kb0, kbn;
 };
 __device__ __forceinline__ W4FTile w4f_tile(const W4FusedParams& p, int tile) {
   W4FTile t;
   t.sp = tile % p.splits;
-  t.out_tile = tile / p.splits;
-  t.mc = t.out_tile % p.mchunks;
-  t.nt = t.out_tile / p.mchunks;
+  t.nt = tile / p.splits;
   t.kb0 = t.sp * p.kb_per_split;
   const int left = p.kblocks - t.kb0;
   t.kbn = left < p.kb_per_split ? left : p.kb_per_split;
   return t;
 }
 
-// Position in a ring of `n` slots that is walked in fixed steps: slot index and phase parity kept incrementally (a
-// runtime `it % n` / `it / n` pair per stage is two integer divisions on every role's critical path).
-struct W4FRing {
-  uint32_t slot, phase, n;
-  __device__ __forceinline__ W4FRing(uint32_t start, uint32_t slots) : slot(start % slots), phase((start / slots) & 1u), n(slots) {}
-  __device__ __forceinline__ void advance(uint32_t step) {
-    slot += step;
-    while (slot >= n) { slot -= n; phase ^= 1u; }
-  }
-};
-
-template <int MT, typename T>
+template <typename T>
 __global__ void __launch_bounds__(w4f::kThreads, 1)
 gemm_w4a16_fused_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w,
                         const __grid_constant__ W4FusedParams p) {
@@ -156,9 +97,9 @@ gemm_w4a16_fused_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_c
   __shared__ volatile unsigned int s_abort;
   __shared__ unsigned int s_ticket;
 
-  constexpr int kABytes = MT * kABlockBytes, kStageBytes = kABytes + kBBytes;
-  constexpr uint32_t kTileCols = MT * kBN;              // accumulator columns of one tile
-  constexpr uint32_t kTmemCols = 2 * kTileCols;         // double-buffered: 256 or 512
+  constexpr int kABytes = kABlockBytes, kStageBytes = kABytes + kBBytes;
+  constexpr uint32_t kTileCols = kBN;                   // accumulator columns of one tile
+  constexpr uint32_t kTmemCols = 2 * kTileCols;         // double-buffered
   constexpr uint32_t kIdesc = umma_idesc(kAccF32, kFmtF16, kFmtF16, kBM, kBN);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -195,7 +136,7 @@ gemm_w4a16_fused_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_c
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = s_tmem_base;
-  const int total_tiles = p.mchunks * p.ntiles * p.splits;
+  const int total_tiles = p.ntiles * p.splits;
 
   // Every wait is bounded: when one runs out the CTA stops waiting anywhere, reports and drains out.
   auto guarded_wait = [&](uint32_t b, uint32_t parity) {
@@ -222,9 +163,7 @@ gemm_w4a16_fused_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_c
           guarded_wait(bar(kBarEmpty + s), st_ring.phase ^ 1);
           unsigned char* st = tiles + (size_t)s * kStageBytes;
           mbar_expect_tx(bar(kBarFull + s), kABytes);
-#pragma unroll
-          for (int mb = 0; mb < MT; ++mb)      // a block past the last token row is filled with zeros
-            tma_load_2d(smem_addr(st + mb * kABlockBytes), &tm_a, (t.kb0 + kb) * kBK, (t.mc * MT + mb) * kBM, bar(kBarFull + s));
+          tma_load_2d(smem_addr(st), &tm_a, (t.kb0 + kb) * kBK, 0, bar(kBarFull + s));     // rows past the last token are zeros
         }
       }
     }
@@ -263,14 +202,9 @@ gemm_w4a16_fused_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_c
           if (!ready) guarded_wait2(bar(kBarReady + s), cur.phase, bar(kBarFull + s), cur.phase);
           tc_fence_after();
           const uint32_t a_addr = smem_addr(tiles + (size_t)s * kStageBytes);
-          const uint64_t bdesc = umma_desc_sw128(a_addr + kABytes);
+          const uint64_t adesc = umma_desc_sw128(a_addr), bdesc = umma_desc_sw128(a_addr + kABytes);
 #pragma unroll
-          for (int mb = 0; mb < MT; ++mb) {
-            const uint64_t adesc = umma_desc_sw128(a_addr + mb * kABlockBytes);
-            const uint32_t d_tmem = tmem_base + buf * kTileCols + mb * kBN;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) umma_ss<false>(d_tmem, adesc + 2 * q, bdesc + 2 * q, kIdesc, (kb != 0 || q != 0) ? 1u : 0u);
-          }
+          for (int q = 0; q < 4; ++q) umma_ss<false>(tmem_base + buf * kTileCols, adesc + 2 * q, bdesc + 2 * q, kIdesc, (kb != 0 || q != 0) ? 1u : 0u);
           umma_commit(bar(kBarEmpty + s));
           // the next stage's barriers, tested without blocking after this stage's MMAs are on their way
           ready = mbar_test_wait(bar(kBarReady + nxt.slot), nxt.phase) && mbar_test_wait(bar(kBarFull + nxt.slot), nxt.phase);
@@ -291,7 +225,7 @@ gemm_w4a16_fused_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_c
       const int n0 = t.nt * kBN;
       guarded_wait(bar(kBarTileFull + buf), (local >> 1) & 1);
       tc_fence_after();
-      float* part = p.partials + ((size_t)t.out_tile * p.splits + t.sp) * (MT * kBM * kBN);
+      float* part = p.partials + ((size_t)t.nt * p.splits + t.sp) * (kBM * kBN);
       // finished values of one row segment: bias, residual, rounding, store
       auto finish8 = [&](int row, int col, float (&v)[8]) {
         if (p.bias != nullptr) {
@@ -312,31 +246,27 @@ gemm_w4a16_fused_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_c
           w4f_store8<T>(out + (size_t)row * p.n + col, v);
         }
       };
+      const int row = quarter * 32 + lane;
+      const uint32_t taddr = tmem_base + buf * kTileCols + ((uint32_t)(quarter * 32) << 16);
 #pragma unroll 1
-      for (int mb = 0; mb < MT; ++mb) {
-        const int row_in_tile = mb * kBM + quarter * 32 + lane;
-        const int row = t.mc * (MT * kBM) + row_in_tile;
-        const uint32_t taddr = tmem_base + buf * kTileCols + mb * kBN + ((uint32_t)(quarter * 32) << 16);
-#pragma unroll 1
-        for (int c = 0; c < kBN / 32; ++c) {
-          uint32_t r[32];
-          tmem_ld_32x32(taddr + c * 32, r);
-          tmem_wait_ld();
-          if (p.splits > 1) {
-            float4* dst = reinterpret_cast<float4*>(part + (size_t)row_in_tile * kBN + c * 32);
+      for (int c = 0; c < kBN / 32; ++c) {
+        uint32_t r[32];
+        tmem_ld_32x32(taddr + c * 32, r);
+        tmem_wait_ld();
+        if (p.splits > 1) {
+          float4* dst = reinterpret_cast<float4*>(part + (size_t)row * kBN + c * 32);
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
-              dst[j] = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]), __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
-          } else if (row < p.m) {
+          for (int j = 0; j < 8; ++j)
+            dst[j] = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]), __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
+        } else if (row < p.m) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const int col = n0 + c * 32 + j * 8;
-              if (col < p.n) {   // N is a multiple of 8
-                float v[8];
+          for (int j = 0; j < 4; ++j) {
+            const int col = n0 + c * 32 + j * 8;
+            if (col < p.n) {   // N is a multiple of 8
+              float v[8];
 #pragma unroll
-                for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(r[j * 8 + e]);
-                finish8(row, col, v);
-              }
+              for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(r[j * 8 + e]);
+              finish8(row, col, v);
             }
           }
         }
@@ -348,23 +278,22 @@ gemm_w4a16_fused_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_c
         // ticket: the CTA whose partial tile is stored last adds all of them, in split order
         __threadfence();
         asm volatile("bar.sync 1, %0;\n" ::"n"(kEpiWarps * 32) : "memory");
-        if (et == 0) s_ticket = atomicAdd(p.tickets + t.out_tile, 1u);
+        if (et == 0) s_ticket = atomicAdd(p.tickets + t.nt, 1u);
         asm volatile("bar.sync 1, %0;\n" ::"n"(kEpiWarps * 32) : "memory");
         if (s_ticket == (unsigned int)(p.splits - 1)) {
           __threadfence();
-          if (et == 0) p.tickets[t.out_tile] = 0u;               // ready for the next call
-          const float* base = p.partials + (size_t)t.out_tile * p.splits * (MT * kBM * kBN);
-          // thread et adds 8-column segments: 16 segments per row, MT*128 rows
+          if (et == 0) p.tickets[t.nt] = 0u;               // ready for the next call
+          const float* base = p.partials + (size_t)t.nt * p.splits * (kBM * kBN);
+          // thread et adds 8-column segments: 16 segments per row
 #pragma unroll 1
-          for (int seg = et; seg < MT * kBM * (kBN / 8); seg += kEpiWarps * 32) {
-            const int row_in_tile = seg / (kBN / 8), c8 = seg % (kBN / 8);
-            const int row = t.mc * (MT * kBM) + row_in_tile, col = n0 + c8 * 8;
+          for (int seg = et; seg < kBM * (kBN / 8); seg += kEpiWarps * 32) {
+            const int row = seg / (kBN / 8), c8 = seg % (kBN / 8), col = n0 + c8 * 8;
             if (row < p.m && col < p.n) {
               float v[8];
 #pragma unroll
               for (int e = 0; e < 8; ++e) v[e] = 0.f;
               for (int sp = 0; sp < p.splits; ++sp) {
-                const float4* src = reinterpret_cast<const float4*>(base + (size_t)sp * (MT * kBM * kBN) + (size_t)row_in_tile * kBN + c8 * 8);
+                const float4* src = reinterpret_cast<const float4*>(base + (size_t)sp * (kBM * kBN) + (size_t)row * kBN + c8 * 8);
                 const float4 a = __ldcg(src), b = __ldcg(src + 1);
                 v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w;
                 v[4] += b.x; v[5] += b.y; v[6] += b.z; v[7] += b.w;
@@ -478,31 +407,32 @@ bool w4a16_gemm_fused_supported(int m, int n, int k, int padded_k, int group_siz
   return m >= 1 && n % 8 == 0 && k == padded_k && k % 64 == 0 && (group_size == 64 || group_size == 128);
 }
 
-// Measured on B200 (bf16, group 128), fused against two-pass: N = 4096, K = 14336 (32 channel tiles, split over K):
-// 45 / 47 / 52 / 70 / 109 us against 122 / 122 / 122 / 125 / 128 us at M = 32 / 64 / 128 / 256 / 512; N = 28672, K = 4096
-// (224 tiles): 71 / 72 / 74 / 89 / 159 us against 110 / 110 / 111 / 129 / 172 us.  So up to 512 tokens (two 256-token
-// chunks, the weights converted once per chunk); beyond that the two-pass form, whose conversion cost does not grow
-// with M, is ahead.
-// Small layers (the shards of a tensor-parallel block) change the balance for two chunks: at M = 512 a 3584 x 4096 layer
-// takes 61 us fused against 45 us two-pass, a 7168 x 4096 layer 47 against 53; below 24 M weights two chunks stay two-pass.
+// Measured on B200 (fp16, group 128, cold weights), fused against two-pass.  Up to 128 tokens, one CTA per tile: N = 4096,
+// K = 14336: 45 / 47 / 52 us against 122 at M = 32 / 64 / 128; N = 28672, K = 4096: 71 / 72 / 74 us against 110.  Above, the
+// CTA-pair form: N = 28672, K = 4096: 87 / 112 / 211 / 759 us against 132 / 177 / 249 / 771 at M = 256 / 512 / 1024 / 4096;
+// N = 4096, K = 14336: 58 / 75 / 368 against 124 / 124 / 400 at M = 256 / 512 / 4096; 8192 x 8192: 62 / 79 against 97 / 99 at
+// M = 256 / 512; 4096 x 4096: 38 against 44 at M = 300 but 56 against 46 at M = 1024: its tiles are too few waves of too short
+// a K loop.  So every size up to 512 tokens, and layers of 24 M weights or more beyond.
 bool w4a16_gemm_fused_preferred(int m, int n, int k, int padded_k, int group_size) {
-  if (!w4a16_gemm_fused_supported(m, n, k, padded_k, group_size) || m <= 16 || m > 4 * w4f::kBM) return false;
-  return m <= 2 * w4f::kBM || (long long)n * k >= 24ll * 1024 * 1024;
+  if (!w4a16_gemm_fused_supported(m, n, k, padded_k, group_size) || m <= 16) return false;
+  return m <= 4 * w4f::kBM || (long long)n * k >= 24ll * 1024 * 1024;
 }
 
+size_t w4a16_gemm_pair_scratch_bytes(int m, int n, int k);
+int w4a16_gemm_pair_launch(const void* x, const void* qw, const void* scales, const void* zeros, const float* bias, const void* residual,
+                           void* out, int m, int n, int k, int group_size, int nibble_signed, int act_dtype, int param_dtype, int out_f32,
+                           float* partials, unsigned int* status, cudaStream_t stream);
+
 struct W4FusedPlan {
-  int mt, mchunks, ntiles, splits, kb_per_split;
+  int ntiles, splits, kb_per_split;
 };
-static W4FusedPlan w4f_plan(int m, int n, int k, int sms) {
+static W4FusedPlan w4f_plan(int n, int k, int sms) {
   W4FusedPlan pl;
-  pl.mt = m > w4f::kBM ? 2 : 1;
-  pl.mchunks = ceil_div(m, pl.mt * w4f::kBM);
   pl.ntiles = ceil_div(n, w4f::kBN);
-  const int tiles = pl.mchunks * pl.ntiles, kblocks = k / w4f::kBK;
+  const int kblocks = k / w4f::kBK;
   // split K while the tiles leave more than half of the SMs idle; a split keeps at least 16 K blocks
   int splits = 1;
-  while (tiles * splits * 2 <= sms && kblocks / (splits * 2) >= 16 && splits < 8) splits *= 2;
-  pl.splits = splits;
+  while (pl.ntiles * splits * 2 <= sms && kblocks / (splits * 2) >= 16 && splits < 8) splits *= 2;
   pl.kb_per_split = ceil_div(kblocks, splits);
   pl.splits = ceil_div(kblocks, pl.kb_per_split);
   return pl;
@@ -512,30 +442,29 @@ static W4FusedPlan w4f_plan(int m, int n, int k, int sms) {
 static size_t w4f_align(size_t v) { return (v + 255) & ~(size_t)255; }
 constexpr size_t kW4FTicketBytes = 16384;
 size_t w4a16_gemm_fused_workspace_bytes(int m, int n, int k) {
-  const int sms = sm_count();
-  const W4FusedPlan pl = w4f_plan(m, n, k, sms);
-  size_t bytes = 256 + kW4FTicketBytes + w4f_align((size_t)m * k * 2);
-  if (pl.splits > 1) bytes += (size_t)pl.mchunks * pl.ntiles * pl.splits * pl.mt * w4f::kBM * w4f::kBN * sizeof(float);
-  return bytes;
+  const size_t bytes = 256 + kW4FTicketBytes + w4f_align((size_t)m * k * 2);
+  if (m > w4f::kBM) return bytes + w4a16_gemm_pair_scratch_bytes(m, n, k);
+  const W4FusedPlan pl = w4f_plan(n, k, sm_count());
+  return bytes + (pl.splits > 1 ? (size_t)pl.ntiles * pl.splits * w4f::kBM * w4f::kBN * sizeof(float) : 0);
 }
 
 int bf16_to_f16_launch(const void* src, void* dst, size_t elements, unsigned int* status, cudaStream_t stream);
 
-template <int MT, typename T>
+template <typename T>
 static int launch_w4f(const void* x, const void* qw, W4FusedParams p, cudaStream_t stream, int sms) {
   using namespace w4f;
   CUtensorMap tm_a, tm_w;
   XQT_CUDA((cudaError_t)make_tile_map(&tm_a, x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, p.m, p.k, kBM));
   XQT_CUDA((cudaError_t)make_byte_map(&tm_w, qw, p.n, p.k / 2, kBK / 2, kBN));
-  constexpr int stage_bytes = MT * kABlockBytes + kBBytes;
+  constexpr int stage_bytes = kABlockBytes + kBBytes;
   p.raw_bufs = kMaxRaw;
   int stages = (kSmemBudget - 1024 - p.raw_bufs * kRawBytes) / stage_bytes;
   p.stages = stages > kMaxStages ? kMaxStages : stages;
   const size_t smem_bytes = (size_t)p.stages * stage_bytes + (size_t)p.raw_bufs * kRawBytes + 1024;
-  auto kern = gemm_w4a16_fused_kernel<MT, T>;
+  auto kern = gemm_w4a16_fused_kernel<T>;
   XQT_SMEM_OPT_IN(kern, kSmemBudget);
   int grid = sms;
-  const int tiles = p.mchunks * p.ntiles * p.splits;
+  const int tiles = p.ntiles * p.splits;
   if (grid > tiles) grid = tiles;
   kern<<<grid, kThreads, smem_bytes, stream>>>(tm_a, tm_w, p);
   return launch_status();
@@ -549,27 +478,29 @@ int w4a16_gemm_fused_launch(const void* x, const void* qw, const void* scales, c
   XQT_REQUIRE(workspace != nullptr && workspace_bytes >= w4a16_gemm_fused_workspace_bytes(m, n, k) && ((uintptr_t)workspace & 255) == 0);
   XQT_REQUIRE(((uintptr_t)out & 15) == 0 && ((uintptr_t)qw & 15) == 0 && ((uintptr_t)x & 15) == 0);
   XQT_REQUIRE(!out_f32 || residual == nullptr);
-  const int sms = sm_count();
-  const W4FusedPlan pl = w4f_plan(m, n, k, sms);
   unsigned char* base = reinterpret_cast<unsigned char*>(workspace);
   unsigned int* status = reinterpret_cast<unsigned int*>(base);
   unsigned int* tickets = reinterpret_cast<unsigned int*>(base + 256);
   unsigned char* x16 = base + 256 + kW4FTicketBytes;
   float* partials = reinterpret_cast<float*>(x16 + w4f_align((size_t)m * k * 2));
-  XQT_REQUIRE((size_t)pl.mchunks * pl.ntiles * sizeof(unsigned int) <= kW4FTicketBytes);
   if (act_dtype == XQT_B200_BF16) {
     XQT_CUDA((cudaError_t)bf16_to_f16_launch(x, x16, (size_t)m * k, status, stream));
     x = x16;
   }
+  if (m > w4f::kBM)
+    return w4a16_gemm_pair_launch(x, qw, scales, zeros, bias, residual, out, m, n, k, group_size, nibble_signed, act_dtype, param_dtype, out_f32,
+                                  partials, status, stream);
+  const int sms = sm_count();
+  const W4FusedPlan pl = w4f_plan(n, k, sms);
+  XQT_REQUIRE((size_t)pl.ntiles * sizeof(unsigned int) <= kW4FTicketBytes);
   W4FusedParams p{};
   p.m = m; p.n = n; p.k = k; p.group_size = group_size; p.groups = k / group_size;
-  p.mchunks = pl.mchunks; p.ntiles = pl.ntiles; p.splits = pl.splits; p.kb_per_split = pl.kb_per_split; p.kblocks = k / w4f::kBK;
+  p.ntiles = pl.ntiles; p.splits = pl.splits; p.kb_per_split = pl.kb_per_split; p.kblocks = k / w4f::kBK;
   p.param_dtype = param_dtype; p.nibble_signed = nibble_signed; p.out_f32 = out_f32;
   p.scales = scales; p.zeros = zeros; p.bias = bias; p.residual = residual; p.out = out;
   p.partials = partials; p.tickets = tickets; p.status = status;
-  if (act_dtype == XQT_B200_BF16)
-    return pl.mt == 2 ? launch_w4f<2, __nv_bfloat16>(x, qw, p, stream, sms) : launch_w4f<1, __nv_bfloat16>(x, qw, p, stream, sms);
-  return pl.mt == 2 ? launch_w4f<2, __half>(x, qw, p, stream, sms) : launch_w4f<1, __half>(x, qw, p, stream, sms);
+  if (act_dtype == XQT_B200_BF16) return launch_w4f<__nv_bfloat16>(x, qw, p, stream, sms);
+  return launch_w4f<__half>(x, qw, p, stream, sms);
 }
 
 }  // namespace xqt_b200

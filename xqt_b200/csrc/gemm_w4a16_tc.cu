@@ -1,8 +1,8 @@
 // W4A16 GEMM for M > 16 on tcgen05, host side and the two-pass form: Y[M,N] = X[M,K] * dequant(W)[N,K]^T.
 //
 // Two forms share this entry.  The fused kernel (gemm_w4a16_fused.cu) dequantises the packed weights in
-// registers on their way to the tensor core and is the choice while M is a few hundred tokens.  At large M the
-// weights are dequantised once per call into an fp16 scratch (any real zero point, fp32 arithmetic, one
+// registers on their way to the tensor core (gemm_w4a16_pair.cu above 128 tokens) and is the choice up to 512 tokens and
+// for large layers.  Otherwise (and for zero points that are no integers) the weights are dequantised once per call into an fp16 scratch (any real zero point, fp32 arithmetic, one
 // rounding) and multiplied by the dense tcgen05 GEMM: the N*K*2-byte round trip is then small against the
 // 2*M*N*K flops, and the dense kernel's 256-wide tiles run nearer the tensor peak.
 //

@@ -351,8 +351,8 @@ class W4A16SwiGLUMLP:
             "inter_local": self.inter_local,
             "kernels": {"m<=16": {"lanes": "w4a16_decode_cl_kernel", "rows128": "w4a16_decode_tc_kernel"}.get(
                             None if self.gate_up.tiled is None else self.gate_up.tiled.layout, "w4a16_decode_kernel"),
-                        "17<=m<=128": "gemm_w4a16_fused_kernel (where it fills the SMs) else dequant_w4_f16_kernel + gemm_f16_kernel",
-                        "m>128": "dequant_w4_f16_kernel + gemm_f16_kernel",
+                        "17<=m<=128": "gemm_w4a16_fused_kernel",
+                        "m>128": "gemm_w4a16_pair_kernel (m > 512: layers of 24 M weights or more) else dequant_w4_f16_kernel + gemm_f16_kernel",
                         "gating": "w4a16_decode_cl_kernel epilogue (m <= 32) / swiglu_kernel" if getattr(self.gate_up, "glu", False) else "swiglu_kernel"},
         }
 

@@ -58,7 +58,7 @@ def resolve_w4a16_variant(m: int, n: int, k: int, padded_k: int, group_size: int
     variant = select_variant(m, n, k, padded_k, int(group_size), activation, has_residual)
     if variant == "tcgen05" and not lib.xqt_b200_w4a16_two_pass(m) and not _integer_zero_points(zero_points):
         variant = "simt"
-    # the fused single-pass form where it measures faster (17 <= M <= 512); integer zero points only
+    # the fused single-pass form where it measures faster (up to 512 tokens, and large layers beyond); integer zero points only
     if variant == "tcgen05" and lib.xqt_b200_w4a16_fused_preferred(m, n, k, padded_k, int(group_size)) and _integer_zero_points(zero_points):
         variant = "tcgen05_fused"
     return variant
