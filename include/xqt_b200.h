@@ -227,6 +227,18 @@ int xqt_b200_w4a16_decode_tiled_static(const void* activation, const void* tiled
                                        int act_dtype, int param_dtype, xqt_b200_stream_t stream);
 size_t xqt_b200_w4a16_decode_static_scratch_bytes(void);
 int xqt_b200_w4a16_decode_static_max_n(void);
+/* The whole SwiGLU block y = down(silu(gate x) * up x) above 128 tokens: gate_up_qweight is [gate; up] ([2*inter, hidden/2],
+ * canonical nibbles), down_qweight [hidden, inter/2]; integer zero points (or null).  The bits of
+ * xqt_b200_w4a16_run (fused) -> xqt_b200_swiglu -> xqt_b200_w4a16_run up to the order of the fp32 sums, without the [M, 2*inter]
+ * intermediate.  `_supported`: 1 where both projections take the CTA-pair GEMM. */
+int xqt_b200_w4a16_swiglu_mlp_supported(int m, int hidden, int inter, int gate_up_group, int down_group);
+size_t xqt_b200_w4a16_swiglu_mlp_workspace_bytes(int m, int hidden, int inter);
+int xqt_b200_w4a16_swiglu_mlp(const void* activation, const void* gate_up_qweight, const void* gate_up_scales,
+                              const void* gate_up_zero_points, const void* down_qweight, const void* down_scales,
+                              const void* down_zero_points, void* output, int m, int hidden, int inter, int gate_up_group,
+                              int down_group, int gate_up_signed, int down_signed, int act_dtype, int gate_up_param_dtype,
+                              int down_param_dtype, void* workspace, size_t workspace_bytes, xqt_b200_stream_t stream);
+
 /* Copies the status word of the built-in scratch of the current device to *host_status (host pointer)
  * and synchronises `stream`; it describes the LAST call of xqt_b200_w4a16_decode_tiled_static on that
  * device (each call clears it first): 0 = every bounded wait completed.  Allocates nothing. */

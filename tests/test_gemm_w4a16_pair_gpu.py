@@ -8,6 +8,7 @@ import torch
 
 from conftest import seeded
 from xqt_b200 import native, quantize
+from xqt_b200.ops.mlp import W4A16SwiGLUMLP
 from xqt_b200.ops.w4a16 import w4a16_linear
 
 pytestmark = pytest.mark.gpu
@@ -40,4 +41,22 @@ def test_pair_form_equals_two_pass(m, n, k, group, dtype, params, symmetric, shr
     assert ((got - want).abs() <= eps * want.abs() + 2.0 ** -23 * (k / 16) * values + 2.0 ** -24).all()
     assert (got - want).norm() <= 0.25 * eps * want.norm() + 1e-6
     assert torch.equal(run("tcgen05_fused", bias=bias, residual=residual).double(), got)      # the same bits every time
+    assert native.workspace_status(DEV) == 0
+
+
+@pytest.mark.parametrize("m,hidden,inter,group", [(129, 128, 128, 64), (300, 1024, 2944, 64), (512, 4096, 14336, 128), (513, 4096, 6144, 128), (256, 2048, 8192, 128)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_mlp_with_the_gating_in_the_epilogue(m, hidden, inter, group, dtype):
+    gen = seeded(m + hidden + inter)
+
+    def layer(rows, columns):
+        return quantize.quantize_w4_asymmetric(torch.randn((rows, columns), generator=gen) * 0.02, group_size=group, param_dtype=dtype)
+
+    block = W4A16SwiGLUMLP(layer(inter, hidden), layer(inter, hidden), layer(hidden, inter), device=DEV, dtype=dtype)
+    assert block._one_entry(m)
+    x = torch.randn((m, hidden), generator=gen).to(DEV, dtype)
+    got, want = block(x).double(), block._forward(x).double()      # linear, SwiGLU kernel, linear
+    # the same roundings in the same places; sums in another order flip some of them by a unit in the last place
+    eps = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}[dtype]
+    assert (got - want).norm() <= 0.5 * eps * want.norm() + 1e-6
     assert native.workspace_status(DEV) == 0

@@ -32,6 +32,10 @@ size_t w4a16_gemm_tc_workspace_bytes(int m, int n, int k);
 bool w4a16_gemm_tc_any_zero_point(int m);
 bool w4a16_gemm_tc_supported(int m, int n, int k, int padded_k, int group_size);
 bool w4a16_gemm_fused_preferred(int m, int n, int k, int padded_k, int group_size);
+bool w4a16_swiglu_mlp_supported(int m, int hidden, int inter, int group_gate_up, int group_down);
+size_t w4a16_swiglu_mlp_workspace_bytes(int m, int hidden, int inter);
+int w4a16_swiglu_mlp_launch(const void*, const void*, const void*, const void*, const void*, const void*, const void*, void*, int, int, int, int, int,
+                            int, int, int, int, int, void*, size_t, cudaStream_t);
 int lowrank_down_launch(const void*, const void*, float*, void*, int, int, int, cudaStream_t);
 size_t w4a4_workspace_bytes(int m, int n, int k);
 int w4a4_gemm_launch(const void*, const float*, const void*, const void*, const void*, const float*, const float*, void*, int,
@@ -421,6 +425,28 @@ int xqt_b200_swiglu(const void* gate_up, void* output, int m, int inter, int dty
   XQT_REQUIRE(gate_up != nullptr && output != nullptr && inter > 0 && inter % 8 == 0);
   XQT_REQUIRE(dtype == XQT_B200_FP16 || dtype == XQT_B200_BF16);
   return swiglu_launch(gate_up, output, m, inter, dtype, (cudaStream_t)stream);
+}
+
+int xqt_b200_w4a16_swiglu_mlp_supported(int m, int hidden, int inter, int gate_up_group, int down_group) {
+  return m > 0 && hidden > 0 && inter > 0 && w4a16_swiglu_mlp_supported(m, hidden, inter, gate_up_group, down_group) ? 1 : 0;
+}
+
+size_t xqt_b200_w4a16_swiglu_mlp_workspace_bytes(int m, int hidden, int inter) {
+  return m > 0 && hidden > 0 && inter > 0 ? w4a16_swiglu_mlp_workspace_bytes(m, hidden, inter) : 0;
+}
+
+int xqt_b200_w4a16_swiglu_mlp(const void* activation, const void* gate_up_qweight, const void* gate_up_scales, const void* gate_up_zero_points,
+                              const void* down_qweight, const void* down_scales, const void* down_zero_points, void* output, int m, int hidden,
+                              int inter, int gate_up_group, int down_group, int gate_up_signed, int down_signed, int act_dtype,
+                              int gate_up_param_dtype, int down_param_dtype, void* workspace, size_t workspace_bytes, xqt_b200_stream_t stream) {
+  XQT_REQUIRE(m > 0 && hidden > 0 && inter > 0);
+  XQT_REQUIRE(activation != nullptr && gate_up_qweight != nullptr && gate_up_scales != nullptr && down_qweight != nullptr && down_scales != nullptr &&
+              output != nullptr);
+  XQT_REQUIRE(act_dtype == XQT_B200_FP16 || act_dtype == XQT_B200_BF16);
+  for (int t : {gate_up_param_dtype, down_param_dtype}) XQT_REQUIRE(t == XQT_B200_FP16 || t == XQT_B200_BF16 || t == XQT_B200_FP32);
+  return w4a16_swiglu_mlp_launch(activation, gate_up_qweight, gate_up_scales, gate_up_zero_points, down_qweight, down_scales, down_zero_points, output, m,
+                                 hidden, inter, gate_up_group, down_group, gate_up_signed, down_signed, act_dtype, gate_up_param_dtype, down_param_dtype,
+                                 workspace, workspace_bytes, (cudaStream_t)stream);
 }
 
 int xqt_b200_workspace_status(const void* workspace, unsigned int* host_status, xqt_b200_stream_t stream) {

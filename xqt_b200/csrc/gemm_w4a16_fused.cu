@@ -503,4 +503,39 @@ int w4a16_gemm_fused_launch(const void* x, const void* qw, const void* scales, c
   return launch_w4f<__half>(x, qw, p, stream, sms);
 }
 
+// SwiGLU MLP block above 128 tokens: activations -> fp16, gate/up with the gating in the epilogue, down.
+int w4a16_gemm_pair_glu_launch(const void* x, const void* qw, const void* scales, const void* zeros, void* h, int m, int inter, int k,
+                               int group_size, int nibble_signed, int act_dtype, int param_dtype, unsigned int* status, cudaStream_t stream);
+
+bool w4a16_swiglu_mlp_supported(int m, int hidden, int inter, int group_gate_up, int group_down) {
+  return m > w4f::kBM && inter % 64 == 0 && hidden % 64 == 0 && w4a16_gemm_fused_preferred(m, 2 * inter, hidden, hidden, group_gate_up) &&
+         w4a16_gemm_fused_preferred(m, hidden, inter, inter, group_down);
+}
+
+// [0,256) status | the ticket area of the kernels that share this workspace | fp16 activations | fp16 h | partial sums of down
+size_t w4a16_swiglu_mlp_workspace_bytes(int m, int hidden, int inter) {
+  return 256 + kW4FTicketBytes + w4f_align((size_t)m * hidden * 2) + w4f_align((size_t)m * inter * 2) + w4a16_gemm_pair_scratch_bytes(m, hidden, inter);
+}
+
+int w4a16_swiglu_mlp_launch(const void* x, const void* gu_qw, const void* gu_scales, const void* gu_zeros, const void* dn_qw, const void* dn_scales,
+                            const void* dn_zeros, void* out, int m, int hidden, int inter, int gu_group, int dn_group, int gu_signed, int dn_signed,
+                            int act_dtype, int gu_param_dtype, int dn_param_dtype, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
+  XQT_REQUIRE(w4a16_swiglu_mlp_supported(m, hidden, inter, gu_group, dn_group));
+  XQT_REQUIRE(workspace != nullptr && workspace_bytes >= w4a16_swiglu_mlp_workspace_bytes(m, hidden, inter) && ((uintptr_t)workspace & 255) == 0);
+  XQT_REQUIRE(((uintptr_t)out & 15) == 0 && ((uintptr_t)gu_qw & 15) == 0 && ((uintptr_t)dn_qw & 15) == 0 && ((uintptr_t)x & 15) == 0);
+  unsigned char* base = reinterpret_cast<unsigned char*>(workspace);
+  unsigned int* status = reinterpret_cast<unsigned int*>(base);
+  unsigned char* x16 = base + 256 + kW4FTicketBytes;
+  unsigned char* h = x16 + w4f_align((size_t)m * hidden * 2);
+  float* partials = reinterpret_cast<float*>(h + w4f_align((size_t)m * inter * 2));
+  if (act_dtype == XQT_B200_BF16) {
+    XQT_CUDA((cudaError_t)bf16_to_f16_launch(x, x16, (size_t)m * hidden, status, stream));
+    x = x16;
+  }
+  const int rc = w4a16_gemm_pair_glu_launch(x, gu_qw, gu_scales, gu_zeros, h, m, inter, hidden, gu_group, gu_signed, act_dtype, gu_param_dtype, status, stream);
+  if (rc != 0) return rc;
+  return w4a16_gemm_pair_launch(h, dn_qw, dn_scales, dn_zeros, nullptr, nullptr, out, m, hidden, inter, dn_group, dn_signed, act_dtype, dn_param_dtype, 0,
+                                partials, status, stream);
+}
+
 }  // namespace xqt_b200

@@ -16,6 +16,11 @@
 // which a second kernel, on all SMs, adds in split order (bit-reproducible); letting the last CTA of a tile add them
 // took 128 threads of one SM 14 us for 512 KiB.
 //
+// GLU form (the gate/up projections of a SwiGLU block, rows [gate; up] of one weight): the first CTA converts gate rows, the
+// second the up rows of the same channels, so a token's gate and up sums meet in one tile and the epilogue writes
+// h = silu(gate) * up in fp16, the operand of the down projection.  The separate form moved [M, 2 inter] through memory
+// twice and h once more (SwiGLU kernel, conversion to fp16): about 30 of 219 us at 512 tokens of a 4096 x 14336 block.
+//
 // Warps (864 threads): 0 activation producer, 1 MMA issuer (the leader's), 2 packed-weight producer, 3-10 epilogue,
 // 11-26 conversion, four groups of four warps on the stages it = g (mod 4), one weight row per thread: converting a stage
 // is a chain of waits (two barrier tests, shared loads, the proxy fence), so four stages are in conversion at a time.
@@ -58,9 +63,31 @@ struct W4PairParams {
   void* out;
   float* partials;                    // [splits][M][N] fp32 (splits > 1)
   unsigned int* status;
+  int inter;                          // GLU: gate rows (= up rows); out is then h, fp16 [M, inter]
 };
 
-// 16 columns of one row: bias, residual, rounding, store (N is a multiple of 8: each half is inside or outside together)
+constexpr unsigned int kHiddenRange = 256;   // status bit: a value beyond fp16's range was clamped (as the activations' conversion sets it)
+
+// silu(gate) * up of eight channels as the separate kernels compute it (the sums rounded to T, the product in fp32 rounded
+// to T), then as an fp16 operand
+template <typename T>
+__device__ __forceinline__ void w4p_gate8(const float (&g)[8], const float (&u)[8], __half* dst, unsigned int* status) {
+  float v[8];
+  bool clipped = false;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    const float x = to_float<T>(from_float<T>(g[e]));
+    v[e] = to_float<T>(from_float<T>(x / (1.0f + expf(-x)) * to_float<T>(from_float<T>(u[e]))));
+    if constexpr (!__is_same(T, __half)) {
+      clipped |= fabsf(v[e]) > 65504.f;                        // false for NaN
+      v[e] = v[e] != v[e] ? v[e] : fminf(fmaxf(v[e], -65504.f), 65504.f);
+    }
+  }
+  w4f_store8<__half>(dst, v);
+  if (clipped) atomicOr(status, kHiddenRange);
+}
+
+// 8 columns of one row: bias, residual, rounding, store
 template <typename T>
 __device__ __forceinline__ void w4p_finish8(const float* bias, const void* residual, void* out, int out_f32, int n, int row, int col, float (&v)[8]) {
   if (bias != nullptr) {
@@ -97,7 +124,13 @@ __device__ __forceinline__ W4PTile w4p_tile(const W4PairParams& p, int tile) {
   return t;
 }
 
-template <int MB, typename T>
+// first weight row a CTA of the pair converts
+template <bool GLU>
+__device__ __forceinline__ int w4p_row0(const W4PairParams& p, int n0, int rank) {
+  return GLU ? n0 / 2 + rank * p.inter : n0 + rank * (p.tile_n / 2);
+}
+
+template <int MB, typename T, bool GLU>
 __global__ void __launch_bounds__(w4p::kThreads, 1)
 gemm_w4a16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ W4PairParams p) {
   using namespace w4p;
@@ -191,7 +224,7 @@ gemm_w4a16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_co
           const int r = ring.slot;
           guarded_spin(bar(kBarRawEmpty + r), ring.phase ^ 1);
           mbar_expect_tx(bar(kBarRawFull + r), raw_bytes);
-          tma_load_2d(raw_s + (uint32_t)(r * raw_bytes), &tm_w, (t.kb0 + kb) * (kBK / 2), t.n0 + (int)rank * half_rows, bar(kBarRawFull + r));
+          tma_load_2d(raw_s + (uint32_t)(r * raw_bytes), &tm_w, (t.kb0 + kb) * (kBK / 2), w4p_row0<GLU>(p, t.n0, (int)rank), bar(kBarRawFull + r));
         }
       }
     }
@@ -242,6 +275,34 @@ gemm_w4a16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_co
       const int block = MB == 2 ? part : 0, cbase = MB == 2 ? 0 : part * cols;
       const int row = ((t.mc * MB + block) * 2 + (int)rank) * kBM + quarter * 32 + lane;
       const uint32_t taddr = tmem_base + buf * (uint32_t)(MB * p.tile_n) + (uint32_t)(part * cols) + ((uint32_t)(quarter * 32) << 16);
+      if constexpr (GLU) {
+        // chunks of 16 channels: all of them for the warp's token block (MB = 2), every other one of the only block
+        const uint32_t gaddr = tmem_base + buf * (uint32_t)(MB * p.tile_n) + (uint32_t)(block * p.tile_n) + ((uint32_t)(quarter * 32) << 16);
+        const int j0 = t.n0 / 2;
+        __half* h = reinterpret_cast<__half*>(p.out) + (size_t)row * p.inter + j0;
+#pragma unroll 1
+        for (int c = MB == 2 ? 0 : part * 16; c < half_rows; c += MB == 2 ? 16 : 32) {
+          uint32_t rg[16], ru[16];
+          tmem_ld_32x16(gaddr + (uint32_t)c, rg);
+          tmem_ld_32x16(gaddr + (uint32_t)(half_rows + c), ru);
+          tmem_wait_ld_dep(rg);
+          tmem_wait_ld_dep(ru);
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            if (row < p.m && j0 + c + 8 * j < p.inter) {           // inter is a multiple of 8
+              float g[8], u[8];
+#pragma unroll
+              for (int e = 0; e < 8; ++e) { g[e] = __uint_as_float(rg[8 * j + e]); u[e] = __uint_as_float(ru[8 * j + e]); }
+              w4p_gate8<T>(g, u, h + c + 8 * j, p.status);
+            }
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(empty0 + 8u * buf);
+        if (++buf == (uint32_t)p.bufs) { buf = 0; buf_phase ^= 1u; }
+        continue;
+      }
       float* part_row = p.partials + ((size_t)t.sp * p.m + row) * p.n;
 #pragma unroll 1
       for (int c = 0; c < cols; c += 16) {
@@ -285,7 +346,7 @@ gemm_w4a16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_co
     bool ahead_raw = false, ahead_free = false;          // this group's next stage was already seen ready
     for (int tile = unit; tile < total_tiles; tile += units) {
       const W4PTile t = w4p_tile(p, tile);
-      const int wrow = t.n0 + (int)rank * half_rows + row;
+      const int wrow = w4p_row0<GLU>(p, t.n0, (int)rank) + row;
       const size_t prow = (size_t)(wrow < p.n ? wrow : p.n - 1) * p.groups;
       uint32_t nsc = 0u, nzp = 0u;                       // this group's next parameters, as raw bits (see the header of the single form)
       bool have_next = false;
@@ -372,14 +433,14 @@ struct PairPlan {
 };
 
 // Estimated SM clocks of the forms; the constants were fitted to sweeps on a B200.
-PairPlan pair_plan(int m, int n, int k) {
+PairPlan pair_plan(int m, int n, int k, int max_splits = 8) {
   const int units = sm_count() / 2, kblocks = k / w4p::kBK;
   PairPlan best{1, 64, 1, 1e30};
   for (int mb = 1; mb <= 2; ++mb) {
     const int mchunks = ceil_div(m, 256 * mb);
     for (int tile_n = 64; tile_n <= 256; tile_n += 32) {
       const int tiles = mchunks * ceil_div(n, tile_n);
-      for (int splits = 1; splits <= 8; ++splits) {
+      for (int splits = 1; splits <= max_splits; ++splits) {
         if (splits > 1 && kblocks < splits * 8) break;
         // clocks per 64-K block: the conversion's chain of barriers and the MMAs behind it
         const double per_kb = 900 + 1.25 * mb * tile_n;
@@ -417,7 +478,7 @@ int resident_pairs(Kern kern, size_t smem) {
   return cached[dev];
 }
 
-template <int MB, typename T>
+template <int MB, typename T, bool GLU>
 int launch_pair(const void* x, const void* qw, W4PairParams p, int k, cudaStream_t stream) {
   using namespace w4p;
   CUtensorMap tm_a, tm_w;
@@ -430,7 +491,7 @@ int launch_pair(const void* x, const void* qw, W4PairParams p, int k, cudaStream
   const int raws = (budget - p.stages * stage_bytes) / raw_bytes;
   p.raw_bufs = raws > kMaxRaw ? kMaxRaw : raws;
   const size_t smem_bytes = (size_t)p.stages * stage_bytes + (size_t)p.raw_bufs * raw_bytes + 1024;
-  auto kern = gemm_w4a16_pair_kernel<MB, T>;
+  auto kern = gemm_w4a16_pair_kernel<MB, T, GLU>;
   XQT_SMEM_OPT_IN(kern, kSmemBudget);
   const int tiles = p.mchunks * p.ntiles * p.splits, pairs = resident_pairs(kern, kSmemBudget);
   const int rc = launch_pdl_cluster(kern, dim3((unsigned)(2 * (tiles < pairs ? tiles : pairs))), dim3(kThreads), 2, smem_bytes, stream, tm_a, tm_w, p);
@@ -459,7 +520,23 @@ int w4a16_gemm_pair_launch(const void* x, const void* qw, const void* scales, co
   p.tile_n = plan.tile_n; p.bufs = 2 * plan.mb * plan.tile_n <= 512 ? 2 : 1;
   p.param_dtype = param_dtype; p.nibble_signed = nibble_signed; p.out_f32 = out_f32;
   p.scales = scales; p.zeros = zeros; p.bias = bias; p.residual = residual; p.out = out; p.partials = partials; p.status = status;
-#define XQT_PAIR(T) (plan.mb == 2 ? launch_pair<2, T>(x, qw, p, k, stream) : launch_pair<1, T>(x, qw, p, k, stream))
+#define XQT_PAIR(T) (plan.mb == 2 ? launch_pair<2, T, false>(x, qw, p, k, stream) : launch_pair<1, T, false>(x, qw, p, k, stream))
+  return act_dtype == XQT_B200_BF16 ? XQT_PAIR(__nv_bfloat16) : XQT_PAIR(__half);
+#undef XQT_PAIR
+}
+
+// h[M, inter] (fp16) = silu(x gate^T) * (x up^T), qw = [gate; up] with 2 * inter rows; x: fp16 [M, K].  act_dtype is the type the
+// sums and h are rounded to.
+int w4a16_gemm_pair_glu_launch(const void* x, const void* qw, const void* scales, const void* zeros, void* h, int m, int inter, int k,
+                               int group_size, int nibble_signed, int act_dtype, int param_dtype, unsigned int* status, cudaStream_t stream) {
+  const PairPlan plan = pair_plan(m, 2 * inter, k, 1);
+  W4PairParams p{};
+  p.m = m; p.n = 2 * inter; p.inter = inter; p.group_shift = group_size == 2 * w4p::kBK ? 1 : 0; p.groups = k / group_size;
+  p.mchunks = ceil_div(m, 256 * plan.mb); p.ntiles = ceil_div(2 * inter, plan.tile_n); p.splits = 1; p.kblocks = k / w4p::kBK;
+  p.tile_n = plan.tile_n; p.bufs = 2 * plan.mb * plan.tile_n <= 512 ? 2 : 1;
+  p.param_dtype = param_dtype; p.nibble_signed = nibble_signed;
+  p.scales = scales; p.zeros = zeros; p.out = h; p.status = status;
+#define XQT_PAIR(T) (plan.mb == 2 ? launch_pair<2, T, true>(x, qw, p, k, stream) : launch_pair<1, T, true>(x, qw, p, k, stream))
   return act_dtype == XQT_B200_BF16 ? XQT_PAIR(__nv_bfloat16) : XQT_PAIR(__half);
 #undef XQT_PAIR
 }

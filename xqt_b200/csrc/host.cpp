@@ -30,9 +30,9 @@ struct Pointer {
 
 // The library entry of a step.  Its arguments are its pointers, then its integers, in the order of the C prototype;
 // workspace address and size (where the entry takes them) and the stream come last.
-enum Op : int { kDecodeLanes, kW4A16Run, kSwiglu, kRotateQuantize, kW8A8Gemm, kLowrankDown, kW4A4Gemm, kActPrologue, kW8A8LowrankGemm, kOpCount };
-constexpr int kPointerCount[kOpCount] = {8, 7, 2, 5, 7, 4, 8, 6, 8};
-constexpr int kIntCount[kOpCount] = {9, 11, 3, 7, 4, 3, 5, 8, 4};
+enum Op : int { kDecodeLanes, kW4A16Run, kSwiglu, kRotateQuantize, kW8A8Gemm, kLowrankDown, kW4A4Gemm, kActPrologue, kW8A8LowrankGemm, kSwigluMlp, kOpCount };
+constexpr int kPointerCount[kOpCount] = {8, 7, 2, 5, 7, 4, 8, 6, 8, 8};
+constexpr int kIntCount[kOpCount] = {9, 11, 3, 7, 4, 3, 5, 8, 4, 10};
 constexpr int kMaxPointers = 8;
 struct Step {
   int op;
@@ -99,6 +99,9 @@ int run_step(const Step& s, void* const* p, void* ws, cudaStream_t stream) {
       return reinterpret_cast<decltype(&xqt_b200_w8a8_gemm_lowrank)>(s.fn)(p[0], p[1], (const float*)p[2], (const float*)p[3],
                                                                            (const float*)p[4], p[5], p[6], p[7], i[0], i[1], i[2], i[3],
                                                                            ws, s.ws_bytes, st);
+    case kSwigluMlp:
+      return reinterpret_cast<decltype(&xqt_b200_w4a16_swiglu_mlp)>(s.fn)(p[0], p[1], p[2], p[3], p[4], p[5], p[6], p[7], i[0], i[1], i[2], i[3],
+                                                                          i[4], i[5], i[6], i[7], i[8], i[9], ws, s.ws_bytes, st);
     case kActPrologue: {
       float scale;                     // the first integer is the bit pattern of lora_scale
       memcpy(&scale, &i[0], sizeof(scale));

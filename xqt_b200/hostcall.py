@@ -21,7 +21,7 @@ INPUT, OUTPUT, RESIDUAL, SCRATCH, WORKSPACE = 1, 2, 3, 4, 5      # csrc/host.cpp
 _OPS = {name: i for i, name in enumerate((
     "xqt_b200_w4a16_decode_lanes", "xqt_b200_w4a16_run", "xqt_b200_swiglu", "xqt_b200_rotate_quantize",
     "xqt_b200_w8a8_gemm_addend", "xqt_b200_lowrank_down", "xqt_b200_w4a4_gemm", "xqt_b200_act_prologue",
-    "xqt_b200_w8a8_gemm_lowrank"))}
+    "xqt_b200_w8a8_gemm_lowrank", "xqt_b200_w4a16_swiglu_mlp"))}
 
 
 def step(symbol: str, pointers: tuple, integers: tuple, workspace=0, workspace_bytes: int = 0) -> tuple:

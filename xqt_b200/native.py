@@ -75,6 +75,9 @@ SIGNATURES: dict[str, tuple] = {
     "xqt_b200_peer_allgather_counted": (_I, [_P, _P, _I, _I, _P, ctypes.c_longlong, ctypes.c_longlong, _P, ctypes.c_uint, _P, _P]),
     "xqt_b200_peer_allreduce_counted": (_I, [_P, _P, _I, _I, _P, ctypes.c_longlong, ctypes.c_longlong, _I, _P, _P, _I, ctypes.c_uint, _P, _P]),
     "xqt_b200_w4a16_decode_static_status": (_I, [ctypes.POINTER(ctypes.c_uint), _P]),
+    "xqt_b200_w4a16_swiglu_mlp_supported": (_I, [_I] * 5),
+    "xqt_b200_w4a16_swiglu_mlp_workspace_bytes": (_Z, [_I] * 3),
+    "xqt_b200_w4a16_swiglu_mlp": (_I, [_P] * 8 + [_I] * 10 + [_P, _Z, _P]),
     "xqt_b200_swiglu": (_I, [_P, _P, _I, _I, _I, _P]),
     "xqt_b200_workspace_status": (_I, [_P, ctypes.POINTER(ctypes.c_uint), _P]),
 }

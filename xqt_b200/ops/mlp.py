@@ -23,7 +23,7 @@ from ..contracts import PackedWeight, PackedWeightMetadata
 from ..errors import XQTBackendError
 from ..hostcall import INPUT, OUTPUT, WORKSPACE, ScratchPlan, bound_call, step, weak_method
 from ..parallel import shard_packed_weight
-from .w4a16 import bind_w4a16_decode, glu_row_order, prepare_decode, resolve_w4a16_variant, w4a16_linear
+from .w4a16 import _integer_zero_points, bind_w4a16_decode, glu_row_order, prepare_decode, resolve_w4a16_variant, w4a16_linear
 
 
 def swiglu(gate_up: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
@@ -249,10 +249,17 @@ class W4A16SwiGLUMLP:
         inter, lanes = self.inter_local, self.down.tiled.layout == "lanes"
         if m < 1 or device.type != "cuda" or (m <= CHUNKED_DECODE_MAX_ROWS and not (self.gate_up.glu and lanes)):
             return weak_method(self._forward)
-        h = scratch.take(2 * m * inter)
         if m <= CHUNKED_DECODE_MAX_ROWS:
+            h = scratch.take(2 * m * inter)
             steps = self.gate_up.decode_steps(m, (INPUT, 0), h, glu=True) + self.down.decode_steps(m, h, (OUTPUT, 0), glu=False)
+        elif self._one_entry(m):
+            nbytes = native.library().xqt_b200_w4a16_swiglu_mlp_workspace_bytes(m, self.hidden, inter)
+            gu, dn = self.gate_up, self.down
+            steps = [step("xqt_b200_w4a16_swiglu_mlp", ((INPUT, 0), gu.qweight, gu.scales, gu.zeros, dn.qweight, dn.scales, dn.zeros, (OUTPUT, 0)),
+                          (m, self.hidden, inter, gu.group, dn.group, gu.signed, dn.signed, native.DTYPE_CODE[self.dtype],
+                           native.DTYPE_CODE[gu.scales.dtype], native.DTYPE_CODE[dn.scales.dtype]), (WORKSPACE, 0), nbytes)]
         else:
+            h = scratch.take(2 * m * inter)
             both = scratch.take(4 * m * inter)
             first, need = self.gate_up.gemm_steps(m, (INPUT, 0), both)
             last, more = self.down.gemm_steps(m, h, (OUTPUT, 0))
@@ -261,6 +268,14 @@ class W4A16SwiGLUMLP:
         return bound_call(steps, weak_method(self._forward), dtype=self.dtype, device=device, rows=m, k=self.gate_up.k, n=self.hidden,
                           scratch_bytes=scratch.nbytes, workspace=(lambda: native.workspace(device, nbytes)) if nbytes else None,
                           keep=(self.gate_up, self.down, native.status_word(device)), symbols="bound W4A16 SwiGLU MLP")
+
+    def _one_entry(self, m: int) -> bool:
+        """Both projections take the CTA-pair GEMM: the block is then one library call with the gating in the gate/up epilogue."""
+
+        gu, dn = self.gate_up, self.down
+        exact = 2 * int(gu.qweight.shape[1]) == gu.k == self.hidden and 2 * int(dn.qweight.shape[1]) == dn.k and gu.n == 2 * self.inter_local
+        return exact and bool(native.library().xqt_b200_w4a16_swiglu_mlp_supported(m, self.hidden, self.inter_local, gu.group, dn.group)) \
+            and _integer_zero_points(gu.zeros) and _integer_zero_points(dn.zeros)
 
     def _forward(self, x: torch.Tensor) -> torch.Tensor:
         h = self.gate_up.gated(x) if isinstance(self.gate_up, _Linear) else None     # decode sizes: one launch
@@ -353,7 +368,7 @@ class W4A16SwiGLUMLP:
                             None if self.gate_up.tiled is None else self.gate_up.tiled.layout, "w4a16_decode_kernel"),
                         "17<=m<=128": "gemm_w4a16_fused_kernel",
                         "m>128": "gemm_w4a16_pair_kernel (m > 512: layers of 24 M weights or more) else dequant_w4_f16_kernel + gemm_f16_kernel",
-                        "gating": "w4a16_decode_cl_kernel epilogue (m <= 32) / swiglu_kernel" if getattr(self.gate_up, "glu", False) else "swiglu_kernel"},
+                        "gating": "w4a16_decode_cl_kernel epilogue (m <= 32) / gemm_w4a16_pair_kernel epilogue (m > 128, single GPU) / swiglu_kernel" if getattr(self.gate_up, "glu", False) else "swiglu_kernel"},
         }
 
 
