@@ -60,3 +60,24 @@ def test_mlp_with_the_gating_in_the_epilogue(m, hidden, inter, group, dtype):
     eps = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}[dtype]
     assert (got - want).norm() <= 0.5 * eps * want.norm() + 1e-6
     assert native.workspace_status(DEV) == 0
+
+
+# 160-column tiles of two token blocks (the narrowest that leave room for four stages only), in one wave, two waves and a
+# partial last tile; K short enough for the rings never to wrap, and long; token counts past 1000
+@pytest.mark.parametrize("m,n,k", [(300, 11008, 512), (512, 22016, 320), (512, 11000, 4096), (1024, 5120, 5120), (1024, 5112, 2304)])
+def test_tiles_of_160_columns(m, n, k):
+    gen = seeded(m + n + k)
+    pw = quantize.quantize_w4_asymmetric(torch.randn((n, k), generator=gen) * 0.02, group_size=64, param_dtype=torch.float16)
+    weight = (pw.qweight.to(DEV), pw.scales.to(DEV), pw.zero_points.to(DEV))
+    x = torch.randn((m, k), generator=gen).to(DEV, torch.float16)
+
+    def run(variant):
+        return w4a16_linear(x, *weight, group_size=64, nibble_signed=False, variant=variant, out_dtype=torch.float32)
+
+    got, want = run("tcgen05_fused"), run("tcgen05")
+    # the same exact products summed in fp32 in another order: 2^-24 of the partial sums for each of the K / 16 additions
+    bound = 2.0 ** -23 * (k / 16) * weight[1].float().abs().max() * 15 * x.float().abs().sum(1, keepdim=True)
+    assert ((got - want).abs() <= bound).all()
+    for _ in range(5):
+        assert torch.equal(run("tcgen05_fused"), got)
+    assert native.workspace_status(DEV) == 0

@@ -42,7 +42,7 @@ constexpr int kBM = 128, kBK = 64;
 constexpr int kRawWarp = 2, kFirstEpiWarp = 3, kEpiWarps = 8, kFirstDqWarp = kFirstEpiWarp + kEpiWarps;
 constexpr int kDqGroups = 4, kDqGroupWarps = 4;
 constexpr int kThreads = (kFirstDqWarp + kDqGroups * kDqGroupWarps) * 32;   // 864
-constexpr int kMaxRaw = 16;
+constexpr int kMinRaw = 2 * kDqGroups, kMaxRaw = 16;
 constexpr int kMaxStages = 5;
 constexpr int kABlockBytes = kBM * 128;
 constexpr int kSmemBudget = 226 * 1024;
@@ -50,6 +50,35 @@ enum Status : unsigned int { kTimeout = 48 };
 constexpr int kBarFull = 0, kBarEmpty = kBarFull + kMaxStages;
 constexpr int kBarRawFull = kBarEmpty + kMaxStages, kBarRawEmpty = kBarRawFull + kMaxRaw;
 constexpr int kBarTileFull = kBarRawEmpty + kMaxRaw, kBarTileEmpty = kBarTileFull + 2, kBarCount = kBarTileEmpty + 2;
+
+// Depths of the two rings: five stages, fewer where they do not fit beside kMinRaw packed-weight slots; the rest of the
+// memory deepens that ring.
+struct Rings {
+  int stages, raws;
+};
+constexpr Rings rings(int mb, int tile_n) {
+  const int stage_bytes = mb * kABlockBytes + tile_n / 2 * 128, raw_bytes = tile_n / 2 * (kBK / 2), budget = kSmemBudget - 1024;
+  const int stages = (budget - kMinRaw * raw_bytes) / stage_bytes < kMaxStages ? (budget - kMinRaw * raw_bytes) / stage_bytes : kMaxStages;
+  const int raws = (budget - stages * stage_bytes) / raw_bytes;
+  return {stages, raws < kMaxRaw ? raws : kMaxRaw};
+}
+// A parity test tells a barrier's phase from the one before it and no further.  The conversion groups look ahead by
+// kDqGroups steps, so at step `it` the phase before the one they test has to be known complete:
+//   Empty(it + 4): its slot's use at it + 4 - 2 * stages; Empty(it - stages) is known and MMAs complete in order, so
+//     stages >= 4 will do.
+//   RawFull(it + 4): its slot's use at it + 4 - raws.  Loads complete in any order.  Known are the group's own steps (it,
+//     it - 4, ..: raws == 8) and all steps up to it - stages (their conversions were waited for by MMAs that are complete:
+//     raws >= stages + 4).  Six slots beside five stages, as 160-column tiles had, are neither: a load overtaken by the
+//     next group's could have been taken for complete.
+constexpr bool look_ahead_is_sound() {
+  for (int mb = 1; mb <= 2; ++mb)
+    for (int tile_n = 64; tile_n <= 256; tile_n += 32) {
+      const Rings r = rings(mb, tile_n);
+      if (r.stages < kDqGroups || (r.raws != 2 * kDqGroups && r.raws < r.stages + kDqGroups)) return false;
+    }
+  return true;
+}
+static_assert(look_ahead_is_sound(), "a ring is too shallow for the conversion groups' look-ahead tests");
 }  // namespace w4p
 
 struct W4PairParams {
@@ -484,12 +513,10 @@ int launch_pair(const void* x, const void* qw, W4PairParams p, int k, cudaStream
   CUtensorMap tm_a, tm_w;
   XQT_CUDA((cudaError_t)make_tile_map(&tm_a, x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, p.m, k, kBM));
   XQT_CUDA((cudaError_t)make_byte_map(&tm_w, qw, p.n, k / 2, kBK / 2, p.tile_n / 2));
-  // five stages, fewer where they do not fit beside six packed-weight slots; the rest of the memory deepens that ring
-  const int stage_bytes = MB * kABlockBytes + p.tile_n / 2 * 128, raw_bytes = p.tile_n / 2 * (kBK / 2), budget = kSmemBudget - 1024;
-  const int stages = (budget - 6 * raw_bytes) / stage_bytes;
-  p.stages = stages > kMaxStages ? kMaxStages : stages;
-  const int raws = (budget - p.stages * stage_bytes) / raw_bytes;
-  p.raw_bufs = raws > kMaxRaw ? kMaxRaw : raws;
+  const Rings ring = rings(MB, p.tile_n);
+  p.stages = ring.stages;
+  p.raw_bufs = ring.raws;
+  const int stage_bytes = MB * kABlockBytes + p.tile_n / 2 * 128, raw_bytes = p.tile_n / 2 * (kBK / 2);
   const size_t smem_bytes = (size_t)p.stages * stage_bytes + (size_t)p.raw_bufs * raw_bytes + 1024;
   auto kern = gemm_w4a16_pair_kernel<MB, T, GLU>;
   XQT_SMEM_OPT_IN(kern, kSmemBudget);
