@@ -15,6 +15,7 @@ from oracle import w8a8 as o88
 from xqt_b200 import engine, native, quantize
 from xqt_b200.errors import XQTBackendError
 from xqt_b200.modules import AWQW4A16Linear, B200PackedDequantLinear, Int8MmaLinear
+from xqt_b200.ops.w4a16 import w4a16_linear
 
 pytestmark = pytest.mark.gpu
 DEV = torch.device("cuda", 0)
@@ -55,6 +56,32 @@ def test_awq_module_forward_bind_and_residual(dtype):
     with pytest.raises(XQTBackendError):
         plain.bind(rows=2, dtype=dtype)(torch.zeros((3, k), device=DEV, dtype=dtype))
     assert native.workspace_status(DEV) == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_awq_module_after_a_dtype_cast(dtype):
+    """A cast of the module casts its floating buffers, the bias among them; the kernels read the bias as fp32."""
+    n, k = 640, 1024
+    pw = _on_device(quantize.quantize_w4_asymmetric(torch.randn((n, k), generator=seeded(51)) * 0.02, group_size=128))
+    module = AWQW4A16Linear(pw, bias=torch.randn((n,), generator=seeded(52)).to(DEV)).eval()
+    xs = {m: torch.randn((m, k), generator=seeded(53 + m)).to(DEV, dtype) for m in (17, 300)}
+
+    def check():
+        for m, x in xs.items():
+            want = w4a16_linear(x, module.canonical_qweight, module.weight_scale, module.weight_zero_point, module.bias, group_size=128, nibble_signed=False)
+            for _ in range(2):
+                assert torch.equal(module(x), want)
+
+    check()
+    for cast in (torch.float16, torch.bfloat16, torch.float32):
+        module.to(cast)
+        assert module.bias.dtype == cast
+        check()
+        module.bias.mul_(-2)                               # changed in place
+        check()
+    module.bias = torch.ones((n - 8,), device=DEV)         # refused as w4a16_linear refuses it
+    with pytest.raises(XQTBackendError):
+        module(xs[17])
 
 
 def test_awq_module_freeze_and_signed_storage_import():

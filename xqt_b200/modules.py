@@ -228,10 +228,12 @@ class AWQW4A16Linear(nn.Module):
         buffers = self._buffers
         zeros = buffers["weight_zero_point"]
         made_from = (buffers["canonical_qweight"], buffers["weight_scale"], zeros, buffers["bias"])
-        hit = self._hot.get((rows, dtype))
-        if hit is not None and all(a is b for a, b in zip(hit[0], made_from)) and hit[3] == (None if zeros is None else zeros._version):
-            return hit
         canonical, scales, _, bias = made_from
+        # what the entry holds in a form of its own: the answer to "are the zero points integers", a bias of another dtype
+        versions = (None if zeros is None else zeros._version, None if bias is None or bias.dtype == torch.float32 else bias._version)
+        hit = self._hot.get((rows, dtype))
+        if hit is not None and all(a is b for a, b in zip(hit[0], made_from)) and hit[3] == versions:
+            return hit
         if self._native_only or canonical is None or not canonical.is_cuda or dtype not in _DTYPE_NAME or rows < 1 \
                 or any(t is not None and t.device != canonical.device for t in made_from):
             return None
@@ -239,20 +241,24 @@ class AWQW4A16Linear(nn.Module):
             run, kernel = self.bind(rows=rows, dtype=dtype), "w4a16_decode_cl_kernel"
         else:
             n, k, padded_k, group, device = self.output_features, self.input_features, int(canonical.shape[1]) * 2, self.group_size, canonical.device
-            if any(t is not None and not t.is_contiguous() for t in made_from) or scales.dtype not in native.DTYPE_CODE \
-                    or (zeros is not None and zeros.dtype != scales.dtype):
+            # whatever w4a16_linear converts or refuses is left to it
+            if any(t is not None and not t.is_contiguous() for t in made_from) or canonical.dtype != torch.uint8 or canonical.ndim != 2 \
+                    or canonical.shape[0] != n or scales.dtype not in native.DTYPE_CODE or tuple(scales.shape) != (n, padded_k // group) \
+                    or (zeros is not None and (zeros.dtype != scales.dtype or zeros.shape != scales.shape)) \
+                    or (bias is not None and bias.numel() != n):
                 return None
             variant = resolve_w4a16_variant(rows, n, k, padded_k, group, zero_points=zeros)
             nbytes = native.library().xqt_b200_w4a16_workspace_bytes(rows, n, k)
-            gemm = step("xqt_b200_w4a16_run", ((INPUT, 0), canonical, scales, zeros, bias, 0, (OUTPUT, 0)),
+            bias32 = None if bias is None else bias.reshape(-1).to(torch.float32).contiguous()     # a cast of the module casts the buffer
+            gemm = step("xqt_b200_w4a16_run", ((INPUT, 0), canonical, scales, zeros, bias32, 0, (OUTPUT, 0)),
                         (rows, n, k, padded_k, group, 0, native.DTYPE_CODE[dtype], native.DTYPE_CODE[scales.dtype], native.DTYPE_CODE[dtype],
                          0, native.VARIANT[variant]), (WORKSPACE, 0), nbytes)
             run = bound_call([gemm], weak_method(self._forward_flat), dtype=dtype, device=device, rows=rows, k=k, n=n,
-                             workspace=lambda: native.workspace(device, nbytes), keep=made_from, symbols="xqt_b200_w4a16_run")
+                             workspace=lambda: native.workspace(device, nbytes), keep=(made_from, bias32), symbols="xqt_b200_w4a16_run")
             kernel = "w4a16 tcgen05 GEMM"
         if len(self._hot) >= 512:
             self._hot.clear()
-        hit = (made_from, run, self._report(kernel, rows, dtype), None if zeros is None else zeros._version)
+        hit = (made_from, run, self._report(kernel, rows, dtype), versions)
         self._hot[(rows, dtype)] = hit
         return hit
 
