@@ -336,3 +336,23 @@ def test_counted_peer_kernels_on_one_gpu():
         assert int(gcounter[0].item()) == call and int(status[0]) == 0
         assert torch.equal(gathered[0], torch.full((count,), 2.0 if call & 1 else 1.0, device=dev))
         assert torch.equal(gathered[1], torch.full((count,), 20.0 if call & 1 else 10.0, device=dev))
+
+
+def test_block_refuses_zero_points_of_another_dtype_where_the_gemm_does():
+    """fp32 zero points beside bf16 scales: the decode layout converts them, ``w4a16_linear`` refuses them, and so does the block
+    at the sizes it sends there."""
+
+    from xqt_b200.errors import XQTBackendError
+    from xqt_b200.ops.mlp import W4A16SwiGLUMLP
+    dev = torch.device("cuda", 0)
+    weights = [type(w)(qweight=w.qweight, scales=w.scales.to(torch.bfloat16), zero_points=w.zero_points.to(torch.float32), metadata=w.metadata)
+               for w in _weights(512, 1024, 40)]
+    same = [type(w)(qweight=w.qweight, scales=w.scales, zero_points=w.zero_points.to(torch.bfloat16), metadata=w.metadata) for w in weights]
+    block, want = W4A16SwiGLUMLP(*weights, device=dev), W4A16SwiGLUMLP(*same, device=dev)
+    x = torch.randn((300, 512), generator=seeded(41)).to(torch.bfloat16).to(dev)
+    for m in (1, 16, 32):
+        assert torch.equal(block(x[:m]), want(x[:m]))
+    for m in (33, 128, 129, 300):
+        for _ in range(2):
+            with pytest.raises(XQTBackendError, match="zero_points must match scales"):
+                block(x[:m])

@@ -131,6 +131,16 @@ class _Linear:
         return w4a16_linear(x, self.qweight, self.scales, self.zeros, group_size=self.group,
                             nibble_signed=self.signed, k=self.k, out_dtype=odt, out=out)
 
+    @property
+    def canonical_served(self) -> bool:
+        """Whether the canonical tensors are what ``w4a16_linear`` takes (it refuses zero points that differ from the scales in
+        dtype or shape; the decode layout, which converts them, serves such a weight up to 16 or 32 rows)."""
+
+        shape = (self.n, int(self.qweight.shape[1]) * 2 // self.group)
+        return self.qweight.dtype == torch.uint8 and tuple(self.qweight.shape) == (self.n, shape[1] * self.group // 2) \
+            and self.scales.dtype in native.DTYPE_CODE and tuple(self.scales.shape) == shape \
+            and (self.zeros is None or (self.zeros.dtype == self.scales.dtype and self.zeros.shape == self.scales.shape))
+
     def decode_steps(self, m: int, source: tuple, target: tuple, *, glu: bool) -> list:
         """The decode launches of ``m`` rows (one per 16) as steps of a bound call."""
 
@@ -247,7 +257,8 @@ class W4A16SwiGLUMLP:
 
         device, scratch, nbytes = self.gate_up.qweight.device, ScratchPlan(), 0
         inter, lanes = self.inter_local, self.down.tiled.layout == "lanes"
-        if m < 1 or device.type != "cuda" or (m <= CHUNKED_DECODE_MAX_ROWS and not (self.gate_up.glu and lanes)):
+        served = self.gate_up.glu and lanes if m <= CHUNKED_DECODE_MAX_ROWS else self.gate_up.canonical_served and self.down.canonical_served
+        if m < 1 or device.type != "cuda" or not served:
             return weak_method(self._forward)
         if m <= CHUNKED_DECODE_MAX_ROWS:
             h = scratch.take(2 * m * inter)
