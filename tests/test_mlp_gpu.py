@@ -356,3 +356,18 @@ def test_block_refuses_zero_points_of_another_dtype_where_the_gemm_does():
         for _ in range(2):
             with pytest.raises(XQTBackendError, match="zero_points must match scales"):
                 block(x[:m])
+
+
+@pytest.mark.parametrize("m", [129, 300])
+def test_the_fusion_switch_holds_at_every_size(m, monkeypatch):
+    """``XQT_B200_FUSED_SWIGLU=0``: linear, SwiGLU kernel and linear as calls of their own above the decode sizes too."""
+
+    from xqt_b200.ops.mlp import W4A16SwiGLUMLP
+    dev = torch.device("cuda", 0)
+    weights = _weights(512, 1024, 50)
+    x = torch.randn((m, 512), generator=seeded(m)).to(torch.bfloat16).to(dev)
+    assert W4A16SwiGLUMLP(*weights, device=dev)._one_entry(m)
+    monkeypatch.setenv("XQT_B200_FUSED_SWIGLU", "0")
+    plain = W4A16SwiGLUMLP(*weights, device=dev)
+    assert not plain._one_entry(m)
+    assert torch.equal(plain(x), plain.down(plain._swiglu(plain.gate_up(x))))

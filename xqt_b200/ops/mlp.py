@@ -217,12 +217,13 @@ class W4A16SwiGLUMLP:
         self._native: dict[int, tuple] = {}       # row count -> (zero-point versions, bound call), single-GPU blocks
         self._can_bind = world == 1 and local_linear is None and swiglu_fn is None
         self._swiglu = swiglu_fn or swiglu
+        self._fuse_gating = swiglu_fn is None and os.environ.get("XQT_B200_FUSED_SWIGLU", "1") not in {"0", ""}
         if local_linear is not None:
             self.gate_up = _InjectedLinear(_concat_rows(gate, up), local_linear)
             self.down = _InjectedLinear(down, local_linear)
             peer_reduce = False
         else:
-            self.gate_up = _Linear(_concat_rows(gate, up), device, dtype, glu=swiglu_fn is None and os.environ.get("XQT_B200_FUSED_SWIGLU", "1") not in {"0", ""})
+            self.gate_up = _Linear(_concat_rows(gate, up), device, dtype, glu=self._fuse_gating)
             self.down = _Linear(down, device, dtype)
         self.hidden, self.inter_local = self.down.n, self.down.k
         # decode sizes (M <= 16): the partial sums of down are added by our own kernel over NVLink peer
@@ -281,11 +282,12 @@ class W4A16SwiGLUMLP:
                           keep=(self.gate_up, self.down, native.status_word(device)), symbols="bound W4A16 SwiGLU MLP")
 
     def _one_entry(self, m: int) -> bool:
-        """Both projections take the CTA-pair GEMM: the block is then one library call with the gating in the gate/up epilogue."""
+        """Both projections take the CTA-pair GEMM: the block is then one library call with the gating in the gate/up epilogue
+        (unless ``XQT_B200_FUSED_SWIGLU=0`` turned the fused gating off when the block was built)."""
 
         gu, dn = self.gate_up, self.down
         exact = 2 * int(gu.qweight.shape[1]) == gu.k == self.hidden and 2 * int(dn.qweight.shape[1]) == dn.k and gu.n == 2 * self.inter_local
-        return exact and bool(native.library().xqt_b200_w4a16_swiglu_mlp_supported(m, self.hidden, self.inter_local, gu.group, dn.group)) \
+        return self._fuse_gating and exact and bool(native.library().xqt_b200_w4a16_swiglu_mlp_supported(m, self.hidden, self.inter_local, gu.group, dn.group)) \
             and _integer_zero_points(gu.zeros) and _integer_zero_points(dn.zeros)
 
     def _forward(self, x: torch.Tensor) -> torch.Tensor:
