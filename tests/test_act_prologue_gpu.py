@@ -62,3 +62,40 @@ def test_matches_the_separate_kernels(m, k, rotation, mode, dtype):
             assert torch.equal(straight[:, :32], hi) and torch.equal(straight[:, 32:], (plain - hi).to(torch.bfloat16).float())
         elif form == 3:
             assert torch.equal(la[:, :32], plain.to(dtype)) and not la[:, 32:].any()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("m,k,rotation,mode", [
+    (21, 768, "s128", 6), (21, 320, "r64", 6), (21, 3072, "none", 6), (1300, 512, "r256", 6), (2400, 512, "none", 6),
+    (21, 2304, "r256", 8), (21, 544, "none", 8), (21, 20480, "s32", 8), (1300, 512, "s128", 8), (21, 1056, "none", 9), (2400, 640, "none", 9)])
+def test_values_that_are_not_finite(m, k, rotation, mode, dtype):
+    """Infinities, NaN and sums that overflow: the separate kernels' codes and scales, which leave a NaN out of a maximum, give
+    it the lowest code and let an infinite maximum make an infinite scale."""
+
+    rot, gen = ROTATIONS[rotation], seeded(m * k)
+    x = torch.randn((m, k), generator=gen) * 3
+    inf, nan, top = float("inf"), float("nan"), torch.finfo(dtype).max
+    x[1, 5], x[2, k - 1], x[3, 7] = inf, -inf, nan
+    x[4, :64], x[5, 64:] = nan, nan
+    x[6], x[7] = nan, inf
+    x[8, 3], x[8, 40], x[8, k - 2] = nan, inf, -inf
+    x[9], x[10, ::5], x[11] = 0.0, -top, top
+    x[12, k // 2:] = -nan
+    x[13, 11], x[13, 12] = inf, -inf
+    x[14, 0] = -nan
+    x[m - 1, k - 1] = nan
+    x = x.to(DEV, dtype)
+    down = (torch.randn((32, k), generator=gen) * 0.05).to(DEV, dtype)
+    want_codes, want_scales, _ = rotate_quantize(x, rot, bits=4 if mode == 6 else 8, sign_magnitude=mode == 6, tiled_scales=mode == 6,
+                                                 scale_in_act_dtype=mode == 9, return_rotated=True)
+    kind, block = _KIND[None if rot is None else rot.kind], 0 if rot is None else rot.block
+    column_scale = None if rot is None else _column_scale(rot, DEV)
+    for form in (0, 1):
+        codes, scales = torch.full((m, k), 99, device=DEV, dtype=torch.int8), torch.full_like(want_scales, -1.0)
+        la = torch.zeros((m, 32), device=DEV)
+        native.check(native.library().xqt_b200_act_prologue(
+            x.data_ptr(), native.ptr(column_scale), codes.data_ptr(), scales.data_ptr(), down.data_ptr() if form else 0, la.data_ptr() if form else 0,
+            1.0, m, k, kind, block, mode, form, native.DTYPE_CODE[dtype], native.stream_handle(DEV)), "xqt_b200_act_prologue")
+        assert torch.equal(codes, want_codes)
+        order = (lambda s: s.reshape(-1, k // 64, 128).permute(0, 2, 1).reshape(-1, k // 64)[:m]) if mode == 6 else (lambda s: s)
+        assert torch.equal(order(scales), order(want_scales))        # no scale is NaN

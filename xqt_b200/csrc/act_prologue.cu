@@ -54,22 +54,28 @@ struct ProloguePar {
 // 0..3 of a unit in different 32-byte quarters (the unit's stores)
 __device__ __forceinline__ int chunk_at(int r, int c) { return c ^ (((r & 1) << 2) | (r & 2)); }
 
+// Maxima of packed absolute values propagate NaN, so a maximum also says whether a value was not finite, at no cost to the
+// values that are; a NaN does not count towards a scale (see where it is found).
+__device__ __forceinline__ uint32_t apro_top(uint32_t v) { return max(v & 0xffffu, v >> 16); }
+
 template <typename T> struct Pack16;
 template <> struct Pack16<__nv_bfloat16> {
+  static __device__ __forceinline__ uint32_t max2(uint32_t a, uint32_t b) {
+    const __nv_bfloat162 v = __hmax2_nan(*reinterpret_cast<const __nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&b));
+    return *reinterpret_cast<const uint32_t*>(&v);
+  }
+  static constexpr uint32_t kInf = 0x7f80;
   static __device__ __forceinline__ uint32_t round2(float a, float b) { const __nv_bfloat162 v = __floats2bfloat162_rn(a, b); return *reinterpret_cast<const uint32_t*>(&v); }
   static __device__ __forceinline__ float2 wide2(uint32_t w) { return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
-  static __device__ __forceinline__ uint32_t max2(uint32_t a, uint32_t b) {
-    const __nv_bfloat162 v = __hmax2(*reinterpret_cast<const __nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&b));
-    return *reinterpret_cast<const uint32_t*>(&v);
-  }
 };
 template <> struct Pack16<__half> {
-  static __device__ __forceinline__ uint32_t round2(float a, float b) { const __half2 v = __floats2half2_rn(a, b); return *reinterpret_cast<const uint32_t*>(&v); }
-  static __device__ __forceinline__ float2 wide2(uint32_t w) { return __half22float2(*reinterpret_cast<const __half2*>(&w)); }
   static __device__ __forceinline__ uint32_t max2(uint32_t a, uint32_t b) {
-    const __half2 v = __hmax2(*reinterpret_cast<const __half2*>(&a), *reinterpret_cast<const __half2*>(&b));
+    const __half2 v = __hmax2_nan(*reinterpret_cast<const __half2*>(&a), *reinterpret_cast<const __half2*>(&b));
     return *reinterpret_cast<const uint32_t*>(&v);
   }
+  static constexpr uint32_t kInf = 0x7c00;
+  static __device__ __forceinline__ uint32_t round2(float a, float b) { const __half2 v = __floats2half2_rn(a, b); return *reinterpret_cast<const uint32_t*>(&v); }
+  static __device__ __forceinline__ float2 wide2(uint32_t w) { return __half22float2(*reinterpret_cast<const __half2*>(&w)); }
 };
 
 __device__ __forceinline__ unsigned long long apro_sub2(unsigned long long a, unsigned long long b) {
@@ -128,8 +134,8 @@ __device__ __forceinline__ uint32_t apro_unit(const ProloguePar& p, int row0, in
       const uint32_t w[8] = {raw[i][0].x, raw[i][0].y, raw[i][0].z, raw[i][0].w, raw[i][1].x, raw[i][1].y, raw[i][1].z, raw[i][1].w};
       mx[i] = 0u;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) mx[i] = P::max2(mx[i], w[j] & 0x7fff7fffu);
-      mx[i] = P::max2(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 8));      // lanes l and l ^ 8
+      for (int j = 0; j < 8; ++j) mx[i] = Pack16<T>::max2(mx[i], w[j] & 0x7fff7fffu);
+      mx[i] = Pack16<T>::max2(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 8));      // lanes l and l ^ 8
     }
     // lane 16 h + l now holds rows h and 2 + h; lane / 8 wants rows 0..3: half 0 keeps rows 0 (l < 8) and 1, half 1 rows 2 and 3
     const uint32_t give = hh ? mx[0] : mx[1];
@@ -220,7 +226,7 @@ __device__ __forceinline__ uint32_t apro_unit(const ProloguePar& p, int row0, in
       float a, b;
       f32x2_unpack(s, a, b);
       const uint32_t o = P::round2(a, b);
-      top = P::max2(top, o & 0x7fff7fffu);
+      top = Pack16<T>::max2(top, o & 0x7fff7fffu);
       *reinterpret_cast<uint32_t*>(out[i & 3] + (i >> 2) * 128) = o;
     }
     return top;
@@ -243,8 +249,34 @@ __device__ __forceinline__ unsigned long long apro_div2(unsigned long long a, un
   return f32x2_fma(f32x2_fma(neg_b, q0, a), y, q0);
 }
 
+// largest absolute value in N words of packed pairs that is not NaN, and no less than mx
+template <typename T, int N>
+__device__ __forceinline__ float apro_number_max(const uint32_t (&w)[N], float mx) {
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    const float2 f = Pack16<T>::wide2(w[j]);
+    mx = fmaxf(mx, fmaxf(fabsf(f.x), fabsf(f.y)));
+  }
+  return mx;
+}
+
+// The same over tile row r, whose 16-byte chunks 0 .. chunks - 1 a warp shares
+template <typename T>
+__device__ __noinline__ float apro_row_number_max(const unsigned char* row, int r, int chunks) {
+  float mx = 0.f;
+  for (int c = threadIdx.x & 31; c < chunks; c += 32) {
+    const uint4 v = *reinterpret_cast<const uint4*>(row + chunk_at(r, c) * 16);
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    mx = apro_number_max<T>(w, mx);
+  }
+#pragma unroll
+  for (int off = 1; off <= 16; off <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+  return mx;
+}
+
 // Codes of 16 consecutive values (8 packed words): rint of the IEEE quotient value / sc.  `divide`: the quotient may leave
-// the code range or the scale is subnormal (a token's own rule, rare).  FORM 0: int8; 1: int4 as sign << 7 | magnitude.
+// the code range, the scale is subnormal or a value is not finite (a token's or group's own rule, rare; a NaN quotient takes
+// the lowest code).  FORM 0: int8; 1: int4 as sign << 7 | magnitude.
 template <typename T, int FORM>
 __device__ __forceinline__ uint4 quantise16(const uint32_t (&w)[8], float sc, float rcp, bool divide) {
   using namespace apro;
@@ -260,19 +292,24 @@ __device__ __forceinline__ uint4 quantise16(const uint32_t (&w)[8], float sc, fl
     code[2 * j] = __float_as_uint(rx);
     code[2 * j + 1] = __float_as_uint(ry);
   }
-  if (FORM == 0 && divide) {
+  if (divide) {
+    constexpr float low = FORM == 0 ? -128.f : -8.f, high = FORM == 0 ? 127.f : 7.f;
+    auto exact = [&](float v) {
+      const int c = (int)fminf(fmaxf(rintf(__fdiv_rn(v, sc)), low), high);
+      return (uint32_t)(FORM == 0 || c >= 0 ? c : 0x80 - c);
+    };
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const float2 f = Pack16<T>::wide2(w[j]);
-      code[2 * j] = (uint32_t)(int)fminf(fmaxf(rintf(__fdiv_rn(f.x, sc)), -128.f), 127.f);
-      code[2 * j + 1] = (uint32_t)(int)fminf(fmaxf(rintf(__fdiv_rn(f.y, sc)), -128.f), 127.f);
+      code[2 * j] = exact(f.x);
+      code[2 * j + 1] = exact(f.y);
     }
   }
   uint32_t o[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     o[j] = __byte_perm(__byte_perm(code[4 * j], code[4 * j + 1], 0x0040), __byte_perm(code[4 * j + 2], code[4 * j + 3], 0x0040), 0x5410);
-    if (FORM == 1) {
+    if (FORM == 1 && !divide) {
       // magnitudes are 0..7: the sign bit only where the magnitude is not zero
       const uint32_t sign = __byte_perm(w[2 * j], w[2 * j + 1], 0x7531) & 0x80808080u;
       o[j] |= sign & (o[j] + 0x7f7f7f7fu);
@@ -381,7 +418,7 @@ act_prologue_i8_kernel(const ProloguePar p) {
   using namespace apro;
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ float cs[kChunk];
-  __shared__ int s_top[16], s_peer[kMaxSplit][16];
+  __shared__ int s_top[16], s_peer[kMaxSplit][16], s_nan[17];         // s_nan: per token, then of any
   __shared__ float4 s_scale[16];                       // per token: scale, reciprocal, "divide" (see quantise16)
   const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int rank, first, last;
@@ -392,7 +429,7 @@ act_prologue_i8_kernel(const ProloguePar p) {
   float* xpose = reinterpret_cast<float*>(smem + p.rows * stride + warp * kXposeBytes);
   const int row0 = (int)(blockIdx.x / p.split) * p.rows;
   if (p.split > 1) cluster_arrive_relaxed();           // "this CTA runs"; waited for before the first remote store
-  if (threadIdx.x < 16) s_top[threadIdx.x] = 0;
+  if (threadIdx.x < 17) s_top[threadIdx.x & 15] = s_nan[threadIdx.x] = 0;
   apro_column_scale<ROT>(p, cs);
   __syncthreads();
   grid_dependency_wait();
@@ -405,10 +442,21 @@ act_prologue_i8_kernel(const ProloguePar p) {
       uint32_t top = apro_unit<T, ROT>(p, row0 + ur, first + chunk, tile, stride, ur, chunk * (kChunk / 8), xpose, cs);
 #pragma unroll
       for (int off = 1; off <= 4; off <<= 1) top = Pack16<T>::max2(top, __shfl_xor_sync(0xffffffffu, top, off));
-      if ((lane & 7) == 0) atomicMax(&s_top[ur + (lane >> 3)], __float_as_int(apro_wide_max<T>(top)));   // values are not negative
+      if ((lane & 7) == 0) {
+        atomicMax(&s_top[ur + (lane >> 3)], __float_as_int(apro_wide_max<T>(top)));   // values are not negative
+        if (apro_top(top) > Pack16<T>::kInf) s_nan[ur + (lane >> 3)] = s_nan[16] = 1;
+      }
     }
   }
   __syncthreads();
+  if (s_nan[16] != 0) {                                // a NaN in a token: its maximum is that of its other values
+    for (int r = warp; r < p.rows; r += warps) {
+      if (s_nan[r] == 0) continue;
+      const float mx = apro_row_number_max<T>(tile + r * stride, r, own * (kChunk / 8));
+      if (lane == 0) s_top[r] = __float_as_int(mx);
+    }
+    __syncthreads();
+  }
   if (p.split > 1) {
     cluster_wait_acquire();
     for (int i = threadIdx.x; i < 16 * p.split; i += blockDim.x)
@@ -423,7 +471,7 @@ act_prologue_i8_kernel(const ProloguePar p) {
     const float s0 = SCALE16 ? to_float<T>(from_float<T>(__fdiv_rn(mx, 127.0f))) : __fdiv_rn(fmaxf(mx, 1e-8f), 127.0f);
     const float sc = SCALE16 ? (s0 > 0.f ? s0 : 1.f) : fmaxf(s0, 1e-8f);
     const float rcp = __frcp_rn(sc);
-    s_scale[threadIdx.x] = make_float4(sc, rcp, sc < 1e-30f || !(mx * rcp < 127.4f) ? 1.f : 0.f, 0.f);
+    s_scale[threadIdx.x] = make_float4(sc, rcp, sc < 1e-30f || !(mx * rcp < 127.4f) || s_nan[threadIdx.x] != 0 ? 1.f : 0.f, 0.f);
     if (rank == 0 && row0 + (int)threadIdx.x < p.m) p.scales[row0 + threadIdx.x] = s0;
   }
   __syncthreads();
@@ -495,10 +543,17 @@ act_prologue_i4_kernel(const ProloguePar p) {
       top = Pack16<T>::max2(top, __shfl_xor_sync(0xffffffffu, top, 1));
       top = Pack16<T>::max2(top, __shfl_xor_sync(0xffffffffu, top, 2));
       const float mx = apro_wide_max<T>(top), by7 = mx * kSeventh;
-      const float sc = fmaxf(fmaf(fmaf(-7.0f, by7, mx), kSeventh, by7), 1e-6f);      // mx / 7, see apro_div2
+      float sc = fmaxf(fmaf(fmaf(-7.0f, by7, mx), kSeventh, by7), 1e-6f);            // mx / 7, see apro_div2
+      const bool odd = apro_top(top) >= Pack16<T>::kInf;                             // infinity or NaN in the group
+      if (__any_sync(0xffffffffu, odd)) {
+        float number = apro_number_max<T>(w, 0.f);
+        number = fmaxf(number, __shfl_xor_sync(0xffffffffu, number, 1));
+        number = fmaxf(number, __shfl_xor_sync(0xffffffffu, number, 2));
+        if (odd) sc = fmaxf(__fdiv_rn(number, 7.0f), 1e-6f);
+      }
       if (inside && row < p.m) {
         if ((l & 3) == 0) p.scales[((size_t)(row >> 7) * groups + f0 / 64) * 128 + (row & 127)] = sc;
-        *reinterpret_cast<uint4*>(p.codes + (size_t)row * p.k + f0) = quantise16<T, 1>(w, sc, __frcp_rn(sc), false);
+        *reinterpret_cast<uint4*>(p.codes + (size_t)row * p.k + f0) = quantise16<T, 1>(w, sc, __frcp_rn(sc), odd);
       }
     }
     if (p.down != nullptr) apro_down<T>(p, tile, stride, chunk * kChunk, 0, 1, min(kChunk, p.k - chunk * kChunk) / 32, acc);
