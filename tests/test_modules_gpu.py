@@ -15,6 +15,7 @@ from oracle import w8a8 as o88
 from xqt_b200 import engine, native, quantize
 from xqt_b200.errors import XQTBackendError
 from xqt_b200.modules import AWQW4A16Linear, B200PackedDequantLinear, Int8MmaLinear
+from xqt_b200.ops.mlp import W4A16SwiGLUMLP
 from xqt_b200.ops.w4a16 import w4a16_linear
 
 pytestmark = pytest.mark.gpu
@@ -229,3 +230,33 @@ def test_decode_lanes_symmetric_weights_without_a_zero_plane():
         x = torch.randn((m, k), generator=seeded(96 + m)).to(torch.float16)
         want = o16.gemm(x, pw.qweight, pw.scales, None, group_size=128, signed=True)
         assert o16.rel_l2(bind_w4a16_decode(tiled, rows=m, dtype=torch.float16)(x.to(DEV)).cpu(), want) <= 1e-3
+
+
+def test_layers_built_under_inference_mode():
+    """Tensors made under ``torch.inference_mode`` have no version counter."""
+    n, k = 256, 512
+    w = torch.randn((n, k), generator=seeded(61)) * 0.02
+    make = lambda: _on_device(quantize.quantize_w4_asymmetric(w, group_size=128))
+    square = lambda: _on_device(quantize.quantize_w4_asymmetric(w[:, :n].contiguous(), group_size=128))
+    want, want_block = AWQW4A16Linear(make()).eval(), W4A16SwiGLUMLP(square(), square(), square(), device=DEV)
+    with torch.inference_mode():
+        module, block = AWQW4A16Linear(make()).eval(), W4A16SwiGLUMLP(square(), square(), square(), device=DEV)
+    moved = AWQW4A16Linear(make()).eval()
+    with torch.inference_mode():
+        moved = moved.to(torch.float16).to(torch.bfloat16)
+    assert moved.weight_zero_point.is_inference()
+    for m in (1, 16, 40, 300, 600):
+        x = torch.randn((m, k), generator=seeded(62 + m)).to(DEV, torch.bfloat16)
+        for mode in (True, False):
+            with torch.inference_mode(mode):
+                assert torch.equal(module(x), want(x)) and torch.equal(block(x[:, :n].contiguous()), want_block(x[:, :n].contiguous()))
+                assert m <= 16 or torch.equal(moved(x), w4a16_linear(x, want.canonical_qweight, moved.weight_scale, moved.weight_zero_point.clone(),
+                                                                     group_size=128, nibble_signed=False))
+    # a change nobody can see the version of: the zero points stop being integers
+    x = torch.randn((40, k), generator=seeded(63)).to(DEV, torch.bfloat16)
+    before = moved(x)
+    with torch.inference_mode():
+        moved.weight_zero_point.add_(0.5)
+    after = moved(x)
+    assert not torch.equal(before, after)
+    assert torch.equal(after, w4a16_linear(x, moved.canonical_qweight, moved.weight_scale, moved.weight_zero_point.clone(), group_size=128, nibble_signed=False))

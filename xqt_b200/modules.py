@@ -26,7 +26,7 @@ from .errors import XQTBackendError
 from .hostcall import INPUT, OUTPUT, WORKSPACE, bound_call, step, weak_method
 from .layout import signed_storage_to_unsigned
 from .ops import awq as awq_ops
-from .ops.w4a16 import resolve_w4a16_variant, w4a16_linear
+from .ops.w4a16 import resolve_w4a16_variant, version_of, w4a16_linear, with_version
 
 _DTYPE_NAME = {torch.float16: "fp16", torch.bfloat16: "bf16"}
 MAX_DECODE_ROWS = 16
@@ -55,7 +55,7 @@ class AWQW4A16Linear(nn.Module):
         self.register_buffer("qweight", prepacked.qweight)
         self.register_buffer("canonical_qweight", prepacked.canonical_qweight)
         self.register_buffer("weight_scale", prepacked.scales)
-        self.register_buffer("weight_zero_point", prepacked.zero_points)
+        self.register_buffer("weight_zero_point", with_version(prepacked.zero_points))
         self.register_buffer("bias", None if bias is None else bias.detach().reshape(-1).to(torch.float32))
         self._has_bias = bias is not None
         self._prepared: dict[torch.dtype, tuple] = {}
@@ -230,7 +230,8 @@ class AWQW4A16Linear(nn.Module):
         made_from = (buffers["canonical_qweight"], buffers["weight_scale"], zeros, buffers["bias"])
         canonical, scales, _, bias = made_from
         # what the entry holds in a form of its own: the answer to "are the zero points integers", a bias of another dtype
-        versions = (None if zeros is None else zeros._version, None if bias is None or bias.dtype == torch.float32 else bias._version)
+        own = (zeros, None if bias is None or bias.dtype == torch.float32 else bias)
+        versions = tuple(version_of(t) for t in own)
         hit = self._hot.get((rows, dtype))
         if hit is not None and all(a is b for a, b in zip(hit[0], made_from)) and hit[3] == versions:
             return hit
@@ -241,8 +242,8 @@ class AWQW4A16Linear(nn.Module):
             run, kernel = self.bind(rows=rows, dtype=dtype), "w4a16_decode_cl_kernel"
         else:
             n, k, padded_k, group, device = self.output_features, self.input_features, int(canonical.shape[1]) * 2, self.group_size, canonical.device
-            # whatever w4a16_linear converts or refuses is left to it
-            if any(t is not None and not t.is_contiguous() for t in made_from) or canonical.dtype != torch.uint8 or canonical.ndim != 2 \
+            # whatever w4a16_linear converts or refuses is left to it, and what changes unseen
+            if any(t is not None and t.is_inference() for t in own) or any(t is not None and not t.is_contiguous() for t in made_from) or canonical.dtype != torch.uint8 or canonical.ndim != 2 \
                     or canonical.shape[0] != n or scales.dtype not in native.DTYPE_CODE or tuple(scales.shape) != (n, padded_k // group) \
                     or (zeros is not None and (zeros.dtype != scales.dtype or zeros.shape != scales.shape)) \
                     or (bias is not None and bias.numel() != n):

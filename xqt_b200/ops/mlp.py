@@ -23,7 +23,7 @@ from ..contracts import PackedWeight, PackedWeightMetadata
 from ..errors import XQTBackendError
 from ..hostcall import INPUT, OUTPUT, WORKSPACE, ScratchPlan, bound_call, step, weak_method
 from ..parallel import shard_packed_weight
-from .w4a16 import _integer_zero_points, bind_w4a16_decode, glu_row_order, prepare_decode, resolve_w4a16_variant, w4a16_linear
+from .w4a16 import _integer_zero_points, bind_w4a16_decode, glu_row_order, prepare_decode, resolve_w4a16_variant, version_of, w4a16_linear, with_version
 
 
 def swiglu(gate_up: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
@@ -71,7 +71,7 @@ class _Linear:
         self.group, self.signed, self.dtype = int(meta.group_size), bool(meta.nibble_signed), dtype
         self.qweight = weight.qweight.to(device).contiguous()
         self.scales = weight.scales.to(device).contiguous()
-        self.zeros = None if weight.zero_points is None else weight.zero_points.to(device).contiguous()
+        self.zeros = with_version(None if weight.zero_points is None else weight.zero_points.to(device).contiguous())
         self._bound: dict[tuple[int, torch.dtype], object] = {}
         self._gated: dict[int, object] = {}
         # glu: this is a fused [gate; up] layer.  Where the decode layout is the lanes one its tiles are built from the
@@ -250,8 +250,7 @@ class W4A16SwiGLUMLP:
         return self._forward(x)
 
     def _zero_versions(self) -> tuple:
-        gate_up, down = self.gate_up.zeros, self.down.zeros
-        return (-1 if gate_up is None else gate_up._version, -1 if down is None else down._version)
+        return (version_of(self.gate_up.zeros), version_of(self.down.zeros))
 
     def _bind(self, m: int):
         """The block for ``m`` rows as one bound call: the launches of :meth:`_forward` with their arguments resolved."""

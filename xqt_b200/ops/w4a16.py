@@ -28,18 +28,36 @@ def _check_cuda(name: str, tensor: torch.Tensor | None, device: torch.device) ->
 _integral_cache = WeakIdDict()      # zero-point tensor -> (version, answer); dies with the tensor
 
 
+def version_of(tensor: torch.Tensor | None) -> int | None:
+    """The tensor's version counter; None where changes cannot be seen (a tensor made under ``torch.inference_mode`` has no
+    counter: nothing that was learnt from its values may be kept)."""
+
+    return None if tensor is None or tensor.is_inference() else tensor._version
+
+
+def with_version(tensor: torch.Tensor | None) -> torch.Tensor | None:
+    """``tensor``, as a copy that has a version counter where it has none."""
+
+    if tensor is None or not tensor.is_inference():
+        return tensor
+    with torch.inference_mode(False):
+        return tensor.clone()
+
+
 def _integer_zero_points(zero_points: torch.Tensor | None) -> bool:
-    """True when every zero point is an integer in [0, 1000] (cached per tensor: one device sync
+    """True when every zero point is an integer in [0, 1000] (cached per tensor and version: one device sync
     the first time a weight is seen).  The tensor-core GEMM folds the zero point into an exact
     integer subtraction and is only valid then."""
 
     if zero_points is None:
         return True
-    hit = _integral_cache.get(zero_points)
-    if hit is None or hit[0] != zero_points._version:
+    version = version_of(zero_points)
+    hit = None if version is None else _integral_cache.get(zero_points)
+    if hit is None or hit[0] != version:
         z = zero_points.to(torch.float32)
-        hit = (zero_points._version, bool(((z == z.round()) & (z >= 0) & (z <= 1000)).all().item()))
-        _integral_cache[zero_points] = hit
+        hit = (version, bool(((z == z.round()) & (z >= 0) & (z <= 1000)).all().item()))
+        if version is not None:
+            _integral_cache[zero_points] = hit
     return hit[1]
 
 
