@@ -9,8 +9,8 @@ import pytest
 import torch
 
 from conftest import seeded
-from xqt_b200 import quantize
-from xqt_b200.errors import XQTBackendError
+from xqt_b200 import native, quantize
+from xqt_b200.errors import CudaCallError, XQTBackendError
 from xqt_b200.ops import w8a8
 from xqt_b200.ops.mlp import W4A16SwiGLUMLP
 from xqt_b200.ops.w4a16 import bind_w4a16_decode, prepare_decode
@@ -69,3 +69,20 @@ def test_leading_dimensions_and_lifetime():
         assert gone() is None
     finally:
         gc.enable()
+
+
+def test_errors_keep_their_types():
+    n, k = 256, 512
+    w = _layer(n, k, 10)
+    run = bind_w4a16_decode(prepare_decode(w.qweight, w.scales, w.zero_points, group_size=128, nibble_signed=False), rows=2, dtype=torch.bfloat16)
+    x = torch.randn((2, k), generator=seeded(11)).to(DEV, torch.bfloat16)
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    with FakeTensorMode():
+        fake = torch.empty((2, k), device=DEV, dtype=torch.bfloat16)
+    with pytest.raises((RuntimeError, CudaCallError)):        # no data: torch or the library refuses the pointer
+        run(fake)
+    # an output of 8 TiB: the error is torch's own, as from torch.empty
+    big = native.host().Bound((), run.slow, None, torch.bfloat16, torch.bfloat16, 0, 2, k, 1 << 41)
+    with pytest.raises(torch.OutOfMemoryError):
+        big(x)
+    assert torch.equal(run(x), run.slow(x))

@@ -8,13 +8,16 @@
 // The object checks what it must in order to pass a raw pointer on (dtype, device, shape, contiguity, current device).
 // Whatever it does not take on itself -- keyword arguments, a failed check, an output or residual that does not fit --
 // goes to the Python callable it was built with, which raises the layer's own error or serves the call.
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/utils/object_ptr.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
 #include <structmember.h>
 
 #include <cstring>
+#include <memory>
 #include <vector>
 
 #include "../../include/xqt_b200.h"
@@ -112,28 +115,27 @@ int run_step(const Step& s, void* const* p, void* ws, cudaStream_t stream) {
   return (int)cudaErrorInvalidValue;
 }
 
-char* stream_space(Bound* b, cudaStream_t stream, PyObject** held) {
+char* stream_space(Bound* b, cudaStream_t stream, THPObjectPtr& held) {
   for (const StreamSpace& s : *b->spaces)
     if (s.stream == stream) {
       Py_INCREF(s.tensor);
-      *held = s.tensor;
+      held = s.tensor;
       return s.data;
     }
-  PyObject* t = PyObject_CallNoArgs(b->workspace);
-  if (t == nullptr) return nullptr;
-  if (!THPVariable_Check(t)) {
-    Py_DECREF(t);
+  held = PyObject_CallNoArgs(b->workspace);
+  if (!held) return nullptr;
+  if (!THPVariable_Check(held.get())) {
     PyErr_SetString(PyExc_TypeError, "Bound: workspace() must return a tensor");
     return nullptr;
   }
-  char* data = static_cast<char*>(THPVariable_Unpack(t).data_ptr());
+  char* data = static_cast<char*>(THPVariable_Unpack(held.get()).data_ptr());
   if (b->spaces->size() >= 16) {                 // a program that keeps making streams: forget the oldest
-    Py_DECREF(b->spaces->front().tensor);
+    PyObject* oldest = b->spaces->front().tensor;
     b->spaces->erase(b->spaces->begin());
+    Py_DECREF(oldest);
   }
-  Py_INCREF(t);
-  b->spaces->push_back({stream, t, data});
-  *held = t;
+  b->spaces->push_back({stream, held.get(), data});
+  Py_INCREF(held.get());
   return data;
 }
 
@@ -141,7 +143,14 @@ bool plain(const at::Tensor& t, at::ScalarType dtype, int device) {
   return t.scalar_type() == dtype && t.is_cuda() && t.device().index() == device && t.layout() == at::kStrided && t.is_contiguous();
 }
 
-PyObject* bound_call(PyObject* self, PyObject* const* args, size_t nargsf, PyObject* kwnames) {
+struct WithoutGil {
+  PyThreadState* state = PyEval_SaveThread();
+  ~WithoutGil() { PyEval_RestoreThread(state); }
+};
+
+// Any of the queries below may throw (a fake or functorch tensor has no data, symbolic sizes are no integers, an allocation
+// fails): `bound_call` turns that into the Python exception torch would raise.
+PyObject* call(PyObject* self, PyObject* const* args, size_t nargsf, PyObject* kwnames) {
   Bound* b = reinterpret_cast<Bound*>(self);
   const Py_ssize_t nargs = PyVectorcall_NARGS(nargsf);
   auto slow = [&]() { return PyObject_Vectorcall(b->slow, args, nargsf, kwnames); };
@@ -152,60 +161,43 @@ PyObject* bound_call(PyObject* self, PyObject* const* args, size_t nargsf, PyObj
   const int64_t dim = (int64_t)shape.size();
   if (dim < 1 || shape[dim - 1] != b->k || x.numel() != b->rows * b->k || (!b->any_rank && dim != 2)) return slow();
 
-  at::Tensor out;
-  PyObject* result = nullptr;
-  if (nargs >= 2 && args[1] != Py_None) {
+  const bool has_out = nargs >= 2 && args[1] != Py_None;
+  if (has_out) {
     if (!THPVariable_Check(args[1])) return slow();
     const at::Tensor& o = THPVariable_Unpack(args[1]);
     if (b->any_rank || !plain(o, b->out_dtype, b->device) || o.dim() != 2 || o.size(0) != b->rows || o.size(1) != b->n) return slow();
-    result = args[1];
-    Py_INCREF(result);
   }
-  const void* residual = nullptr;
+  void* residual = nullptr;
   if (nargs == 3 && args[2] != Py_None) {
-    bool fits = b->takes_residual && THPVariable_Check(args[2]);
-    if (fits) {
-      const at::Tensor& r = THPVariable_Unpack(args[2]);
-      fits = plain(r, b->dtype, b->device) && r.dim() == 2 && r.size(0) == b->rows && r.size(1) == b->n;
-      if (fits) residual = r.data_ptr();
-    }
-    if (!fits) {
-      Py_XDECREF(result);
-      return slow();
-    }
+    if (!b->takes_residual || !THPVariable_Check(args[2])) return slow();
+    const at::Tensor& r = THPVariable_Unpack(args[2]);
+    if (!plain(r, b->dtype, b->device) || r.dim() != 2 || r.size(0) != b->rows || r.size(1) != b->n) return slow();
+    residual = r.data_ptr();
   }
-  PyObject* held = nullptr;
+  const c10::Device device(c10::kCUDA, (c10::DeviceIndex)b->device);
+  at::Tensor out, scratch;
+  if (has_out) {
+    out = THPVariable_Unpack(args[1]);
+  } else if (dim == 2) {
+    out = at::detail::empty_cuda({b->rows, b->n}, b->out_dtype, device, c10::nullopt);
+  } else {
+    std::vector<int64_t> oshape(shape.begin(), shape.end());
+    oshape.back() = b->n;
+    out = at::detail::empty_cuda(oshape, b->out_dtype, device, c10::nullopt);
+  }
+  if (b->scratch_bytes > 0) scratch = at::detail::empty_cuda({b->scratch_bytes}, at::kByte, device, c10::nullopt);
+  const cudaStream_t stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)b->device).stream();
+  char* base[6] = {nullptr, static_cast<char*>(x.data_ptr()), static_cast<char*>(out.data_ptr()), static_cast<char*>(residual),
+                   scratch.defined() ? static_cast<char*>(scratch.data_ptr()) : nullptr, nullptr};
+  THPObjectPtr held;
+  if (b->workspace != Py_None) {
+    base[kWorkspace] = stream_space(b, stream, held);
+    if (base[kWorkspace] == nullptr) return nullptr;
+  }
   int code = 0;
   size_t at_step = 0;
-  try {
-    const c10::Device device(c10::kCUDA, (c10::DeviceIndex)b->device);
-    void* out_data;
-    if (result == nullptr) {
-      if (dim == 2) {
-        out = at::detail::empty_cuda({b->rows, b->n}, b->out_dtype, device, c10::nullopt);
-      } else {
-        std::vector<int64_t> oshape(shape.begin(), shape.end());
-        oshape.back() = b->n;
-        out = at::detail::empty_cuda(oshape, b->out_dtype, device, c10::nullopt);
-      }
-      out_data = out.data_ptr();
-    } else {
-      out_data = THPVariable_Unpack(result).data_ptr();
-    }
-    at::Tensor scratch;
-    if (b->scratch_bytes > 0) scratch = at::detail::empty_cuda({b->scratch_bytes}, at::kByte, device, c10::nullopt);
-    const cudaStream_t stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)b->device).stream();
-    char* base[6] = {nullptr, static_cast<char*>(x.data_ptr()), static_cast<char*>(out_data),
-                     static_cast<char*>(const_cast<void*>(residual)),
-                     scratch.defined() ? static_cast<char*>(scratch.data_ptr()) : nullptr, nullptr};
-    if (b->workspace != Py_None) {
-      base[kWorkspace] = stream_space(b, stream, &held);
-      if (base[kWorkspace] == nullptr) {
-        Py_XDECREF(result);
-        return nullptr;
-      }
-    }
-    Py_BEGIN_ALLOW_THREADS
+  {
+    const WithoutGil released;
     for (; at_step < b->steps->size(); ++at_step) {
       const Step& s = (*b->steps)[at_step];
       void* p[kMaxPointers];
@@ -216,24 +208,26 @@ PyObject* bound_call(PyObject* self, PyObject* const* args, size_t nargsf, PyObj
       code = run_step(s, p, base[s.ws.source] + s.ws.value, stream);
       if (code != 0) break;
     }
-    Py_END_ALLOW_THREADS
-  } catch (const std::exception& e) {
-    Py_XDECREF(held);
-    Py_XDECREF(result);
-    PyErr_SetString(PyExc_RuntimeError, e.what());
-    return nullptr;
   }
-  Py_XDECREF(held);
   if (code != 0) {
-    Py_XDECREF(result);
-    PyObject* r = PyObject_CallFunction(b->on_error, "in", code, (Py_ssize_t)at_step);
-    if (r != nullptr) {
-      Py_DECREF(r);
-      PyErr_SetString(PyExc_RuntimeError, "Bound: library call failed");
-    }
+    THPObjectPtr r(PyObject_CallFunction(b->on_error, "in", code, (Py_ssize_t)at_step));
+    if (r) PyErr_SetString(PyExc_RuntimeError, "Bound: library call failed");
     return nullptr;
   }
-  return result != nullptr ? result : THPVariable_Wrap(std::move(out));
+  if (has_out) {
+    Py_INCREF(args[1]);
+    return args[1];
+  }
+  return THPVariable_Wrap(std::move(out));
+}
+
+PyObject* bound_call(PyObject* self, PyObject* const* args, size_t nargsf, PyObject* kwnames) {
+  try {
+    return call(self, args, nargsf, kwnames);
+  } catch (...) {
+    torch::translate_exception_to_python(std::current_exception());
+    return nullptr;
+  }
 }
 
 bool parse_pointer(PyObject* o, Pointer* p) {
@@ -303,7 +297,7 @@ void bound_dealloc(PyObject* self) {
   Py_TYPE(self)->tp_free(self);
 }
 
-PyObject* bound_new(PyTypeObject* type, PyObject* args, PyObject* kwargs) {
+PyObject* make(PyTypeObject* type, PyObject* args, PyObject* kwargs) {
   static const char* names[] = {"steps", "slow", "on_error", "dtype", "out_dtype", "device", "rows", "k", "n", "any_rank",
                                 "takes_residual", "scratch_bytes", "workspace", "keep", nullptr};
   PyObject *steps, *slow, *on_error, *dtype, *out_dtype, *workspace = Py_None, *keep = Py_None;
@@ -317,20 +311,15 @@ PyObject* bound_new(PyTypeObject* type, PyObject* args, PyObject* kwargs) {
     PyErr_SetString(PyExc_TypeError, "Bound: dtype and out_dtype must be torch dtypes");
     return nullptr;
   }
-  auto parsed = new std::vector<Step>((size_t)PyTuple_GET_SIZE(steps));
+  auto parsed = std::make_unique<std::vector<Step>>((size_t)PyTuple_GET_SIZE(steps));
   for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(steps); ++i)
-    if (!parse_step(PyTuple_GET_ITEM(steps, i), &(*parsed)[(size_t)i])) {
-      delete parsed;
-      return nullptr;
-    }
+    if (!parse_step(PyTuple_GET_ITEM(steps, i), &(*parsed)[(size_t)i])) return nullptr;
+  auto spaces = std::make_unique<std::vector<StreamSpace>>();
   Bound* b = reinterpret_cast<Bound*>(type->tp_alloc(type, 0));
-  if (b == nullptr) {
-    delete parsed;
-    return nullptr;
-  }
+  if (b == nullptr) return nullptr;
   b->vectorcall = bound_call;
-  b->steps = parsed;
-  b->spaces = new std::vector<StreamSpace>();
+  b->steps = parsed.release();
+  b->spaces = spaces.release();
   Py_INCREF(slow); b->slow = slow;
   Py_INCREF(on_error); b->on_error = on_error;
   Py_INCREF(workspace); b->workspace = workspace;
@@ -343,6 +332,15 @@ PyObject* bound_new(PyTypeObject* type, PyObject* args, PyObject* kwargs) {
   b->takes_residual = takes_residual != 0;
   b->scratch_bytes = scratch_bytes;
   return reinterpret_cast<PyObject*>(b);
+}
+
+PyObject* bound_new(PyTypeObject* type, PyObject* args, PyObject* kwargs) {
+  try {
+    return make(type, args, kwargs);
+  } catch (...) {
+    torch::translate_exception_to_python(std::current_exception());
+    return nullptr;
+  }
 }
 
 PyMemberDef bound_members[] = {{"keep", T_OBJECT, offsetof(Bound, keep), 0, "the objects whose memory the calls use"},
