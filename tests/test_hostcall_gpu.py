@@ -13,7 +13,7 @@ from xqt_b200 import native, quantize
 from xqt_b200.errors import CudaCallError, XQTBackendError
 from xqt_b200.ops import w8a8
 from xqt_b200.ops.mlp import W4A16SwiGLUMLP
-from xqt_b200.ops.w4a16 import bind_w4a16_decode, prepare_decode
+from xqt_b200.ops.w4a16 import bind_w4a16_decode, bind_w4a16_linear, prepare_decode
 
 pytestmark = pytest.mark.gpu
 DEV = torch.device("cuda", 0)
@@ -86,3 +86,50 @@ def test_errors_keep_their_types():
     with pytest.raises(torch.OutOfMemoryError):
         big(x)
     assert torch.equal(run(x), run.slow(x))
+
+
+def _bound_gemm(rows, n, k, seed):
+    w = _layer(n, k, seed)
+    return bind_w4a16_linear(w.qweight, w.scales, w.zero_points, rows=rows, dtype=torch.bfloat16, group_size=128, nibble_signed=False, variant="tcgen05")
+
+
+def test_workspace_is_the_pools_current_one():
+    """Calls bound before the pool has grown report into the buffer that ``workspace_status`` reads, and the buffer before
+    it is released."""
+    k = 512
+    stream = torch.cuda.Stream(DEV)
+    with torch.cuda.stream(stream):
+        small, x = _bound_gemm(40, 256, k, 20), torch.randn((40, k), generator=seeded(21)).to(DEV, torch.bfloat16)
+        want = small(x)
+        key = (0, native.stream_handle(DEV), "run")
+        before = weakref.ref(native._workspaces[key])
+        size = before().numel()
+        large = _bound_gemm(64, 1024 + size // (2 * k), k, 22)
+        large(torch.randn((64, k), generator=seeded(23)).to(DEV, torch.bfloat16))
+        assert before() is None and native._workspaces[key].numel() > size
+        assert torch.equal(small(x), want) and native.workspace_status(DEV) == 0
+        small(x * 2.0 ** 20)                                   # beyond fp16's range: clamped and reported
+        assert native.workspace_status(DEV) == 256
+        native._workspaces[key][:4].zero_()
+        stream.synchronize()
+
+
+def test_workspace_of_a_captured_graph_outlives_its_replacement():
+    k = 512
+    stream = torch.cuda.Stream(DEV)
+    with torch.cuda.stream(stream):
+        run, x = _bound_gemm(40, 256, k, 24), torch.randn((40, k), generator=seeded(25)).to(DEV, torch.bfloat16)
+        want = run(x)
+        key = (0, native.stream_handle(DEV), "run")
+        used = weakref.ref(native._workspaces[key])
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            got = run(x)
+        size = used().numel()
+        assert native.workspace(DEV, size + 1).numel() >= 2 * size and used() is not None
+        filler = [torch.full((size // 4,), float("nan"), device=DEV) for _ in range(4)]      # would take its memory
+        got.zero_()
+        graph.replay()
+        assert torch.equal(got, want) and len(filler) == 4
+        assert native.workspace_status(DEV) == 0
+        stream.synchronize()

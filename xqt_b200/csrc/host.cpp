@@ -13,11 +13,14 @@
 #include <torch/csrc/utils/object_ptr.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAStream.h>
 #include <structmember.h>
 
 #include <cstring>
 #include <memory>
+#include <string>
+#include <unordered_map>
 #include <vector>
 
 #include "../../include/xqt_b200.h"
@@ -46,20 +49,42 @@ struct Step {
   size_t ws_bytes;
 };
 
-// The workspace of a stream.  The reference keeps the buffer alive even where the pool it came from has since replaced
-// it by a larger one.
-struct StreamSpace {
-  cudaStream_t stream;
+// The workspaces of native.py's pool, mirrored here so that a call finds the current one without running Python code: per
+// device, stream and tag the buffer in use (guarded by the GIL).  A call holds a reference while it launches; a bound layer
+// keeps none, so a buffer that the pool has replaced is released, and status words are read where the kernels write them.
+struct SpaceKey {
+  int device;
+  uintptr_t stream;
+  int tag;
+  bool operator==(const SpaceKey& o) const { return device == o.device && stream == o.stream && tag == o.tag; }
+};
+struct SpaceHash {
+  size_t operator()(const SpaceKey& k) const { return std::hash<uintptr_t>()(k.stream * 31 + (uintptr_t)k.tag * 7 + (uintptr_t)k.device); }
+};
+struct Space {
   PyObject* tensor;
   char* data;
+  size_t bytes;
+  bool captured;         // a graph capture has recorded its address
 };
+std::unordered_map<SpaceKey, Space, SpaceHash>& spaces() {
+  static auto* map = new std::unordered_map<SpaceKey, Space, SpaceHash>();
+  return *map;
+}
+int tag_id(const char* tag) {
+  static auto* tags = new std::vector<std::string>();
+  for (size_t i = 0; i < tags->size(); ++i)
+    if ((*tags)[i] == tag) return (int)i;
+  tags->push_back(tag);
+  return (int)tags->size() - 1;
+}
 
 struct Bound {
   PyObject_HEAD
   vectorcallfunc vectorcall;
   PyObject* slow;        // the Python callable with the same signature
   PyObject* on_error;    // called with (code, step) when a library call fails: raises
-  PyObject* workspace;   // None, or called without arguments: the current stream's workspace tensor
+  PyObject* workspace;   // None, or called with a size: the pool's workspace for the current stream, at least that large
   PyObject* keep;
   at::ScalarType dtype, out_dtype;
   int device;
@@ -67,8 +92,9 @@ struct Bound {
   bool any_rank;         // the input may have any leading dimensions that multiply to `rows`
   bool takes_residual;   // a third positional argument, [rows, n] in the input dtype
   int64_t scratch_bytes;
+  int tag;               // the workspace's
+  size_t ws_bytes;       // the largest workspace a step needs
   std::vector<Step>* steps;
-  std::vector<StreamSpace>* spaces;
 };
 
 int run_step(const Step& s, void* const* p, void* ws, cudaStream_t stream) {
@@ -115,27 +141,23 @@ int run_step(const Step& s, void* const* p, void* ws, cudaStream_t stream) {
   return (int)cudaErrorInvalidValue;
 }
 
-char* stream_space(Bound* b, cudaStream_t stream, THPObjectPtr& held) {
-  for (const StreamSpace& s : *b->spaces)
-    if (s.stream == stream) {
-      Py_INCREF(s.tensor);
-      held = s.tensor;
-      return s.data;
+char* stream_space(Bound* b, cudaStream_t stream, size_t bytes, THPObjectPtr& held) {
+  const SpaceKey key{b->device, (uintptr_t)stream, b->tag};
+  auto it = spaces().find(key);
+  if (it == spaces().end() || it->second.bytes < bytes) {
+    held = PyObject_CallFunction(b->workspace, "n", (Py_ssize_t)bytes);
+    if (!held) return nullptr;
+    it = spaces().find(key);
+    if (it == spaces().end() || it->second.bytes < bytes) {
+      PyErr_SetString(PyExc_RuntimeError, "Bound: the workspace pool has no buffer of the size asked for");
+      return nullptr;
     }
-  held = PyObject_CallNoArgs(b->workspace);
-  if (!held) return nullptr;
-  if (!THPVariable_Check(held.get())) {
-    PyErr_SetString(PyExc_TypeError, "Bound: workspace() must return a tensor");
-    return nullptr;
   }
-  char* data = static_cast<char*>(THPVariable_Unpack(held.get()).data_ptr());
-  if (b->spaces->size() >= 16) {                 // a program that keeps making streams: forget the oldest
-    PyObject* oldest = b->spaces->front().tensor;
-    b->spaces->erase(b->spaces->begin());
-    Py_DECREF(oldest);
-  }
-  b->spaces->push_back({stream, held.get(), data});
-  Py_INCREF(held.get());
+  Space& space = it->second;
+  if (!space.captured && c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) space.captured = true;
+  char* data = space.data;
+  Py_INCREF(space.tensor);
+  held = space.tensor;
   return data;
 }
 
@@ -191,7 +213,7 @@ PyObject* call(PyObject* self, PyObject* const* args, size_t nargsf, PyObject* k
                    scratch.defined() ? static_cast<char*>(scratch.data_ptr()) : nullptr, nullptr};
   THPObjectPtr held;
   if (b->workspace != Py_None) {
-    base[kWorkspace] = stream_space(b, stream, held);
+    base[kWorkspace] = stream_space(b, stream, b->ws_bytes, held);
     if (base[kWorkspace] == nullptr) return nullptr;
   }
   int code = 0;
@@ -290,22 +312,20 @@ void bound_dealloc(PyObject* self) {
   Bound* b = reinterpret_cast<Bound*>(self);
   PyObject_GC_UnTrack(self);
   bound_clear(self);
-  if (b->spaces != nullptr)
-    for (const StreamSpace& s : *b->spaces) Py_DECREF(s.tensor);
-  delete b->spaces;
   delete b->steps;
   Py_TYPE(self)->tp_free(self);
 }
 
 PyObject* make(PyTypeObject* type, PyObject* args, PyObject* kwargs) {
   static const char* names[] = {"steps", "slow", "on_error", "dtype", "out_dtype", "device", "rows", "k", "n", "any_rank",
-                                "takes_residual", "scratch_bytes", "workspace", "keep", nullptr};
+                                "takes_residual", "scratch_bytes", "workspace", "tag", "keep", nullptr};
   PyObject *steps, *slow, *on_error, *dtype, *out_dtype, *workspace = Py_None, *keep = Py_None;
+  const char* tag = "run";
   int device, any_rank = 0, takes_residual = 0;
   long long rows, k, n, scratch_bytes = 0;
-  if (!PyArg_ParseTupleAndKeywords(args, kwargs, "O!OOOOiLLL|ppLOO", const_cast<char**>(names), &PyTuple_Type, &steps, &slow, &on_error,
+  if (!PyArg_ParseTupleAndKeywords(args, kwargs, "O!OOOOiLLL|ppLOsO", const_cast<char**>(names), &PyTuple_Type, &steps, &slow, &on_error,
                                    &dtype, &out_dtype, &device, &rows, &k, &n, &any_rank, &takes_residual, &scratch_bytes, &workspace,
-                                   &keep))
+                                   &tag, &keep))
     return nullptr;
   if (!THPDtype_Check(dtype) || !THPDtype_Check(out_dtype)) {
     PyErr_SetString(PyExc_TypeError, "Bound: dtype and out_dtype must be torch dtypes");
@@ -314,12 +334,14 @@ PyObject* make(PyTypeObject* type, PyObject* args, PyObject* kwargs) {
   auto parsed = std::make_unique<std::vector<Step>>((size_t)PyTuple_GET_SIZE(steps));
   for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(steps); ++i)
     if (!parse_step(PyTuple_GET_ITEM(steps, i), &(*parsed)[(size_t)i])) return nullptr;
-  auto spaces = std::make_unique<std::vector<StreamSpace>>();
   Bound* b = reinterpret_cast<Bound*>(type->tp_alloc(type, 0));
   if (b == nullptr) return nullptr;
   b->vectorcall = bound_call;
   b->steps = parsed.release();
-  b->spaces = spaces.release();
+  b->tag = tag_id(tag);
+  b->ws_bytes = 0;
+  for (const Step& s : *b->steps)
+    if (s.ws.source == kWorkspace && s.ws_bytes > b->ws_bytes) b->ws_bytes = s.ws_bytes;
   Py_INCREF(slow); b->slow = slow;
   Py_INCREF(on_error); b->on_error = on_error;
   Py_INCREF(workspace); b->workspace = workspace;
@@ -347,7 +369,56 @@ PyMemberDef bound_members[] = {{"keep", T_OBJECT, offsetof(Bound, keep), 0, "the
                                {"slow", T_OBJECT, offsetof(Bound, slow), 0, "the callable that gets what the native path does not take"},
                                {nullptr, 0, 0, 0, nullptr}};
 PyTypeObject bound_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
-PyModuleDef host_module = {PyModuleDef_HEAD_INIT, "_host", "Native call path of the bound layers.", -1, nullptr, nullptr, nullptr, nullptr, nullptr};
+
+// set_workspace(device, stream, tag, tensor): the pool's buffer from now on; the one before it is released
+PyObject* set_workspace(PyObject*, PyObject* args) {
+  int device;
+  unsigned long long stream;
+  const char* tag;
+  PyObject* tensor;
+  if (!PyArg_ParseTuple(args, "iKsO", &device, &stream, &tag, &tensor)) return nullptr;
+  if (!THPVariable_Check(tensor)) {
+    PyErr_SetString(PyExc_TypeError, "set_workspace: a tensor is needed");
+    return nullptr;
+  }
+  try {
+    const at::Tensor& t = THPVariable_Unpack(tensor);
+    Space fresh{tensor, static_cast<char*>(t.data_ptr()), (size_t)t.nbytes(), false};
+    Space& space = spaces()[SpaceKey{device, (uintptr_t)stream, tag_id(tag)}];
+    THPObjectPtr before(space.tensor);       // value-initialised when new
+    Py_INCREF(tensor);
+    space = fresh;
+  } catch (...) {
+    torch::translate_exception_to_python(std::current_exception());
+    return nullptr;
+  }
+  Py_RETURN_NONE;
+}
+
+// workspace_captured(device, stream, tag[, mark]): whether a graph capture has recorded the buffer's address; `mark` says so
+PyObject* workspace_captured(PyObject*, PyObject* args) {
+  int device, mark = 0;
+  unsigned long long stream;
+  const char* tag;
+  if (!PyArg_ParseTuple(args, "iKs|p", &device, &stream, &tag, &mark)) return nullptr;
+  bool captured = false;
+  try {
+    auto it = spaces().find(SpaceKey{device, (uintptr_t)stream, tag_id(tag)});
+    if (it != spaces().end()) {
+      it->second.captured |= mark != 0;
+      captured = it->second.captured;
+    }
+  } catch (...) {
+    torch::translate_exception_to_python(std::current_exception());
+    return nullptr;
+  }
+  return PyBool_FromLong(captured);
+}
+
+PyMethodDef host_methods[] = {{"set_workspace", set_workspace, METH_VARARGS, "Mirror a buffer of the workspace pool."},
+                              {"workspace_captured", workspace_captured, METH_VARARGS, "Whether a graph capture uses a buffer of the pool."},
+                              {nullptr, nullptr, 0, nullptr}};
+PyModuleDef host_module = {PyModuleDef_HEAD_INIT, "_host", "Native call path of the bound layers.", -1, host_methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace
 

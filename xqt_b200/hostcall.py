@@ -65,19 +65,22 @@ def weak_method(method):
 
 
 def bound_call(steps: list, slow, *, dtype: torch.dtype, device: torch.device, rows: int, k: int, n: int, out_dtype: torch.dtype | None = None,
-               any_rank: bool = False, residual: bool = False, scratch_bytes: int = 0, workspace=None, keep=(), symbols: str = ""):
+               any_rank: bool = False, residual: bool = False, scratch_bytes: int = 0, workspace: str | None = None, keep=(), symbols: str = ""):
     """``run(x[, out[, residual]])``: checks ``x`` (``[rows, k]``, or with ``any_rank`` any shape of that many elements
     with trailing dimension ``k``), allocates ``[rows, n]`` and makes the calls.  ``slow`` has the same signature and
-    gets every call whose arguments the native path does not take: it raises, or serves it."""
+    gets every call whose arguments the native path does not take: it raises, or serves it.  ``workspace``: the tag of the
+    pool's buffer (:func:`native.workspace`) that steps with a ``WORKSPACE`` pointer use, looked up on every call."""
 
     index = device.index if device.index is not None else torch.cuda.current_device()
 
     def failed(code: int, at: int) -> None:
         native.check(code, symbols or f"bound call, step {at}")
 
+    pool = None if workspace is None else lambda nbytes: native.workspace(device, nbytes, workspace)
     return native.host().Bound(
         tuple(steps), slow, failed, dtype, dtype if out_dtype is None else out_dtype, index, int(rows), int(k), int(n),
-        any_rank=any_rank, takes_residual=residual, scratch_bytes=int(scratch_bytes), workspace=workspace, keep=keep)
+        any_rank=any_rank, takes_residual=residual, scratch_bytes=int(scratch_bytes), workspace=pool,
+        tag=workspace or "run", keep=keep)
 
 
 __all__ = ["INPUT", "OUTPUT", "RESIDUAL", "SCRATCH", "WORKSPACE", "ScratchPlan", "bound_call", "float_bits", "step", "weak_method"]

@@ -255,7 +255,7 @@ class AWQW4A16Linear(nn.Module):
                         (rows, n, k, padded_k, group, 0, native.DTYPE_CODE[dtype], native.DTYPE_CODE[scales.dtype], native.DTYPE_CODE[dtype],
                          0, native.VARIANT[variant]), (WORKSPACE, 0), nbytes)
             run = bound_call([gemm], weak_method(self._forward_flat), dtype=dtype, device=device, rows=rows, k=k, n=n,
-                             workspace=lambda: native.workspace(device, nbytes), keep=(made_from, bias32), symbols="xqt_b200_w4a16_run")
+                             workspace="run", keep=(made_from, bias32), symbols="xqt_b200_w4a16_run")
             kernel = "w4a16 tcgen05 GEMM"
         if len(self._hot) >= 512:
             self._hot.clear()

@@ -158,9 +158,19 @@ def stream_handle(device: torch.device) -> int:
     return torch.cuda.current_stream(device).cuda_stream
 
 
-# One scratch buffer per (device, stream): launches on one stream are ordered, so they may share
+# One scratch buffer per (device, stream, tag): launches on one stream are ordered, so they may share
 # it; launches on different streams may overlap and must not.
 _workspaces: dict[tuple[int, int, str], torch.Tensor] = {}
+# Buffers that a graph capture has recorded and the pool has replaced since: the graph may be replayed.
+_retired: dict[tuple[int, int, str], list[torch.Tensor]] = {}
+
+
+def _workspace_size(nbytes: int) -> int:
+    """``nbytes`` rounded up to an eighth of its power of two (1 MiB at least): callers whose needs creep up, a token at a time,
+    get a new buffer now and then and not on each call."""
+
+    unit = max(1 << 17, 1 << max(0, int(nbytes).bit_length() - 4))
+    return max(1 << 20, -(-int(nbytes) // unit) * unit)
 
 
 def workspace(device: torch.device, nbytes: int, tag: str = "run") -> torch.Tensor:
@@ -168,15 +178,25 @@ def workspace(device: torch.device, nbytes: int, tag: str = "run") -> torch.Tens
 
     ``tag`` separates kernel families whose scratch layouts differ: the decode kernels keep tickets
     that must stay zero between launches where the GEMM keeps a converted copy of the activations,
-    so they never share a buffer."""
+    so they never share a buffer.  A buffer that is too small is replaced and released, unless a graph capture has recorded
+    it: then it stays for the replays, and its successor is at least twice as large (all that is kept stays below the buffer
+    in use)."""
 
     index = device.index if device.index is not None else torch.cuda.current_device()
     key = (index, stream_handle(device), tag)
     buffer = _workspaces.get(key)
     if buffer is None or buffer.numel() < nbytes:
-        size = max(int(nbytes), 1 << 20)
-        buffer = torch.zeros(size, dtype=torch.uint8, device=torch.device("cuda", index))
-        _workspaces[key] = buffer
+        size = _workspace_size(nbytes)
+        captured = buffer is not None and host().workspace_captured(*key)
+        if captured:
+            size = max(size, 2 * buffer.numel())
+        fresh = torch.zeros(size, dtype=torch.uint8, device=torch.device("cuda", index))
+        if captured:
+            _retired.setdefault(key, []).append(buffer)
+        _workspaces[key] = buffer = fresh
+        host().set_workspace(*key, buffer)
+    if torch.cuda.is_current_stream_capturing():
+        host().workspace_captured(*key, True)
     return buffer
 
 
@@ -204,13 +224,14 @@ def workspace_status(device: torch.device) -> int:
     word = _status_words.get(index)
     if word is not None:
         worst = int(word[0].item()) & 0xFFFFFFFF
-    for (dev_index, stream, _tag), buffer in list(_workspaces.items()):
-        if dev_index != index or stream != stream_handle(device):
+    for key, current in list(_workspaces.items()):
+        if key[:2] != (index, stream_handle(device)):
             continue
-        value = ctypes.c_uint(0)
-        check(library().xqt_b200_workspace_status(buffer.data_ptr(), ctypes.byref(value), stream_handle(device)),
-              "xqt_b200_workspace_status")
-        worst = max(worst, int(value.value))
+        for buffer in (current, *_retired.get(key, ())):
+            value = ctypes.c_uint(0)
+            check(library().xqt_b200_workspace_status(buffer.data_ptr(), ctypes.byref(value), stream_handle(device)),
+                  "xqt_b200_workspace_status")
+            worst = max(worst, int(value.value))
     return worst
 
 

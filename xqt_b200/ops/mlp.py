@@ -277,7 +277,7 @@ class W4A16SwiGLUMLP:
             steps = first + [step("xqt_b200_swiglu", (both, h), (m, inter, native.DTYPE_CODE[self.dtype]))] + last
             nbytes = max(need, more)
         return bound_call(steps, weak_method(self._forward), dtype=self.dtype, device=device, rows=m, k=self.gate_up.k, n=self.hidden,
-                          scratch_bytes=scratch.nbytes, workspace=(lambda: native.workspace(device, nbytes)) if nbytes else None,
+                          scratch_bytes=scratch.nbytes, workspace="run" if nbytes else None,
                           keep=(self.gate_up, self.down, native.status_word(device)), symbols="bound W4A16 SwiGLU MLP")
 
     def _one_entry(self, m: int) -> bool:

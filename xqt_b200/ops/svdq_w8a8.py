@@ -17,7 +17,7 @@ import torch
 
 from .. import native
 from ..errors import XQTBackendError
-from ..hostcall import INPUT, OUTPUT, bound_call, float_bits, step
+from ..hostcall import INPUT, OUTPUT, WORKSPACE, bound_call, float_bits, step
 
 RANK_PAD = 32          # the down projection's width
 UP_PAD = 64            # the up projection's K extent (one 64-element tensor-core K block)
@@ -168,9 +168,9 @@ def bind_svdq_w8a8_linear(packed: PackedSVDQW8A8Linear, workspace: W8A8SVDQWorks
     k, n, dtype, device, scale = packed.input_features, packed.output_features, packed.dtype, packed.qweight.device, float(lora_scale)
     if int(workspace.quantized_activation.shape[1]) != k:
         raise ValueError("workspace extent does not match the packed layer")
+    native.workspace(device, 256, "gemm")            # the current stream's status word, made now
     dcode = native.DTYPE_CODE[dtype]
     codes, scales, la = workspace.quantized_activation, workspace.activation_scales, workspace.lora_activation16
-    scratch = native.workspace(device, 256, "gemm")
 
     def run(inputs: torch.Tensor) -> torch.Tensor:
         if inputs.dtype != dtype or inputs.device != device or inputs.ndim != 2 or tuple(inputs.shape) != (rows, k) \
@@ -185,11 +185,11 @@ def bind_svdq_w8a8_linear(packed: PackedSVDQW8A8Linear, workspace: W8A8SVDQWorks
                     (float_bits(scale), rows, k, 0, 0, 9, 3 if low_rank else 0, dcode))
     if low_rank:
         gemm = step("xqt_b200_w8a8_gemm_lowrank", (codes, packed.qweight, scales, packed.weight_scales, packed.bias, la, packed.up, (OUTPUT, 0)),
-                    (rows, n, k, dcode), scratch, scratch.numel())
+                    (rows, n, k, dcode), (WORKSPACE, 0), 256)
     else:
         gemm = step("xqt_b200_w8a8_gemm_addend", (codes, packed.qweight, scales, packed.weight_scales, packed.bias, 0, (OUTPUT, 0)),
-                    (rows, n, k, dcode), scratch, scratch.numel())
-    return bound_call([quantise, gemm], run, dtype=dtype, device=device, rows=rows, k=k, n=n, keep=(packed, workspace, scratch),
+                    (rows, n, k, dcode), (WORKSPACE, 0), 256)
+    return bound_call([quantise, gemm], run, dtype=dtype, device=device, rows=rows, k=k, n=n, workspace="gemm", keep=(packed, workspace),
                       symbols="bound SVDQ W8A8 (quantise / GEMM)")
 
 

@@ -222,7 +222,7 @@ def bind_w4a16_linear(
         return out
 
     run_step = step("xqt_b200_w4a16_run", ((INPUT, 0), *static, (OUTPUT, 0)), (*tail, variant_code), (WORKSPACE, 0), nbytes)
-    return bound_call([run_step], run, dtype=dtype, device=device, rows=rows, k=kk, n=n, workspace=lambda: native.workspace(device, nbytes),
+    return bound_call([run_step], run, dtype=dtype, device=device, rows=rows, k=kk, n=n, workspace="run",
                       keep=keep, symbols="xqt_b200_w4a16_run")          # the callable owns the tensors whose raw pointers it passes
 
 

@@ -371,7 +371,7 @@ def bind_svdq_w4a4_linear(packed: PackedSVDQW4A4Linear, workspace: W4A4Workspace
     steps.append(step("xqt_b200_w4a4_gemm", (codes, scales, packed.qweight, packed.weight_bytes, packed.aux, la, packed.bias, (OUTPUT, 0)),
                       (rows, n, k, dcode, 3), (WORKSPACE, 0), nbytes))
     return bound_call(steps, run, dtype=dtype, device=device, rows=rows, k=k, n=n, any_rank=True,
-                      workspace=lambda: native.workspace(device, nbytes, "gemm"), keep=(packed, workspace, la, column_scale),
+                      workspace="gemm", keep=(packed, workspace, la, column_scale),
                       symbols="bound SVDQ W4A4 (xqt_b200_rotate_quantize / xqt_b200_lowrank_down / xqt_b200_w4a4_gemm)")
 
 

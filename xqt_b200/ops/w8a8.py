@@ -19,7 +19,7 @@ import torch
 
 from .. import native
 from ..errors import XQTBackendError
-from ..hostcall import INPUT, OUTPUT, bound_call, step
+from ..hostcall import INPUT, OUTPUT, WORKSPACE, bound_call, step
 from ..quantize import Rotation, regular_rotation
 from .activation import rotate_quantize
 
@@ -303,12 +303,12 @@ def bind_convrot_w8a8_linear(packed: PackedConvRotW8A8Linear, workspace: ConvRot
     codes, scales = workspace.quantized_activation[:rows], workspace.activation_scales[:rows]
     column_scale = None if rot is None else _column_scale(rot, device)
     index = device.index if device.index is not None else torch.cuda.current_device()
-    scratch = native.workspace(device, 256, "gemm")
+    native.workspace(device, 256, "gemm")            # the current stream's status word, made now
     dcode = native.DTYPE_CODE[dtype]
     prologue = (native.ptr(column_scale), codes.data_ptr(), scales.data_ptr(), 0, rows, k, _KIND[None if rot is None else rot.kind],
                 0 if rot is None else rot.block, 8, 0, dcode)
     gemm_head = (codes.data_ptr(), packed.qweight.data_ptr(), scales.data_ptr(), packed.weight_scales.data_ptr(), native.ptr(packed.bias))
-    gemm_tail = (rows, n, k, dcode, scratch.data_ptr(), scratch.numel())
+    gemm_tail = (rows, n, k, dcode)
 
     def run(inputs: torch.Tensor) -> torch.Tensor:
         if inputs.dtype != dtype or inputs.device != device or inputs.shape[-1] != k or inputs.numel() != rows * k \
@@ -317,18 +317,18 @@ def bind_convrot_w8a8_linear(packed: PackedConvRotW8A8Linear, workspace: ConvRot
         if torch.cuda.current_device() != index:
             raise XQTBackendError("bound ConvRot W8A8 call: make the weight's device current before calling")
         out = torch.empty((*inputs.shape[:-1], n), device=device, dtype=dtype)
-        stream = torch.cuda.current_stream(device).cuda_stream
+        stream, scratch = torch.cuda.current_stream(device).cuda_stream, native.workspace(device, 256, "gemm")
         code = lib.xqt_b200_rotate_quantize(inputs.data_ptr(), *prologue, stream)
         if code == 0:
-            code = lib.xqt_b200_w8a8_gemm(*gemm_head, out.data_ptr(), *gemm_tail, stream)
+            code = lib.xqt_b200_w8a8_gemm(*gemm_head, out.data_ptr(), *gemm_tail, scratch.data_ptr(), scratch.numel(), stream)
         if code != 0:
             native.check(code, "bound ConvRot W8A8 (xqt_b200_rotate_quantize / xqt_b200_w8a8_gemm)")
         return out
 
     quantise = step("xqt_b200_rotate_quantize", ((INPUT, 0), *prologue[:4]), prologue[4:])
-    gemm = step("xqt_b200_w8a8_gemm_addend", (*gemm_head, 0, (OUTPUT, 0)), gemm_tail[:4], scratch, scratch.numel())
+    gemm = step("xqt_b200_w8a8_gemm_addend", (*gemm_head, 0, (OUTPUT, 0)), gemm_tail, (WORKSPACE, 0), 256)
     return bound_call([quantise, gemm], run, dtype=dtype, device=device, rows=rows, k=k, n=n, any_rank=True,
-                      keep=(packed, workspace, rot, column_scale, scratch),
+                      workspace="gemm", keep=(packed, workspace, rot, column_scale),
                       symbols="bound ConvRot W8A8 (xqt_b200_rotate_quantize / xqt_b200_w8a8_gemm)")
 
 
