@@ -13,7 +13,7 @@ from xqt_b200 import native, quantize
 from xqt_b200.errors import CudaCallError, XQTBackendError
 from xqt_b200.ops import w8a8
 from xqt_b200.ops.mlp import W4A16SwiGLUMLP
-from xqt_b200.ops.w4a16 import bind_w4a16_decode, bind_w4a16_linear, prepare_decode
+from xqt_b200.ops.w4a16 import bind_w4a16_decode, bind_w4a16_linear, prepare_decode, w4a16_linear
 
 pytestmark = pytest.mark.gpu
 DEV = torch.device("cuda", 0)
@@ -133,3 +133,19 @@ def test_workspace_of_a_captured_graph_outlives_its_replacement():
         assert torch.equal(got, want) and len(filler) == 4
         assert native.workspace_status(DEV) == 0
         stream.synchronize()
+
+
+def test_weights_first_seen_inside_a_graph_capture():
+    """Whether the zero points are integers takes a device-to-host copy, which a capture cannot hold: such a call takes the two
+    passes, which serve any zero point, and is captured."""
+    n, k, m = 24576, 1024, 600
+    w = _layer(n, k, 40)
+    x = torch.randn((m, k), generator=seeded(41)).to(DEV, torch.bfloat16)
+    want = w4a16_linear(x, w.qweight, w.scales, w.zero_points.clone(), group_size=128, nibble_signed=False, variant="tcgen05")
+    stream, graph = torch.cuda.Stream(DEV), torch.cuda.CUDAGraph()
+    stream.wait_stream(torch.cuda.current_stream(DEV))
+    with torch.cuda.graph(graph, stream=stream):
+        got = w4a16_linear(x, w.qweight, w.scales, w.zero_points, group_size=128, nibble_signed=False)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)

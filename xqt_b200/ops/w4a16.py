@@ -61,6 +61,17 @@ def _integer_zero_points(zero_points: torch.Tensor | None) -> bool:
     return hit[1]
 
 
+def integer_zero_points_now(zero_points: torch.Tensor | None) -> bool | None:
+    """:func:`_integer_zero_points`, or None where that would have to wait for the device inside a graph capture (which it may not)."""
+
+    if zero_points is not None and zero_points.is_cuda and torch.cuda.is_current_stream_capturing():
+        version = version_of(zero_points)
+        hit = None if version is None else _integral_cache.get(zero_points)
+        if hit is None or hit[0] != version:
+            return None
+    return _integer_zero_points(zero_points)
+
+
 def select_variant(m: int, n: int, k: int, padded_k: int, group_size: int, activation: str = "none",
                    has_residual: bool = False) -> str:
     code = native.library().xqt_b200_w4a16_select_variant(
@@ -74,10 +85,13 @@ def resolve_w4a16_variant(m: int, n: int, k: int, padded_k: int, group_size: int
 
     lib = native.library()
     variant = select_variant(m, n, k, padded_k, int(group_size), activation, has_residual)
-    if variant == "tcgen05" and not lib.xqt_b200_w4a16_two_pass(m) and not _integer_zero_points(zero_points):
+    two_pass = bool(lib.xqt_b200_w4a16_two_pass(m))
+    if variant == "tcgen05" and not two_pass and not _integer_zero_points(zero_points):
         variant = "simt"
-    # the fused single-pass form where it measures faster (up to 512 tokens, and large layers beyond); integer zero points only
-    if variant == "tcgen05" and lib.xqt_b200_w4a16_fused_preferred(m, n, k, padded_k, int(group_size)) and _integer_zero_points(zero_points):
+    # the fused single-pass form where it measures faster (up to 512 tokens, and large layers beyond); integer zero points only.
+    # Two passes take any zero point: a weight that is first seen inside a graph capture goes there
+    if variant == "tcgen05" and lib.xqt_b200_w4a16_fused_preferred(m, n, k, padded_k, int(group_size)) and \
+            (integer_zero_points_now if two_pass else _integer_zero_points)(zero_points):
         variant = "tcgen05_fused"
     return variant
 
