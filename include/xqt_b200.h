@@ -45,6 +45,7 @@ typedef struct CUstream_st* xqt_b200_stream_t; /* == cudaStream_t */
                                     /* xqt_b200_w4a16_two_pass(m) is 1 (every M > 16 by default) the  */
                                     /* weights are first dequantised to an fp16 scratch, any zero     */
                                     /* point; otherwise the single-pass kernel below                  */
+#define XQT_B200_VARIANT_AUTO_INTEGER 5  /* AUTO for a caller who knows that its zero points are integers in [0, 1000] */
 #define XQT_B200_VARIANT_TCGEN05_FUSED 4  /* single-pass form of 3: dequantisation inside the GEMM, no */
                                     /* N*K*2 scratch, INTEGER zero points only                        */
 

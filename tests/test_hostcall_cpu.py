@@ -16,7 +16,7 @@ from torch._subclasses.fake_tensor import FakeTensorMode
 from torch.fx.experimental.symbolic_shapes import ShapeEnv
 from xqt_b200 import native
 
-bound = native.host().Bound((), lambda *args: "slow", None, torch.bfloat16, torch.bfloat16, 0, 2, 16, 8, takes_residual=True)
+bound = native.host().Bound(((2, 2, (), (), 0, 0),), lambda *args: "slow", None, torch.bfloat16, torch.bfloat16, 0, 2, 16, 8, takes_residual=True)
 assert bound(torch.zeros(2, 16)) == "slow" and bound(torch.zeros(2, 16), None) == "slow"
 with FakeTensorMode() as mode:
     fixed = torch.empty(2, 16, dtype=torch.bfloat16, device="cuda:0")

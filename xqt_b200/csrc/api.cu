@@ -117,6 +117,8 @@ int xqt_b200_w4a16_run(const void* activation, const void* qweight, const void* 
   const int out_f32 = out_dtype == XQT_B200_FP32 && act_dtype != XQT_B200_FP32 ? 1 : 0;
   if (m == 0) return 0;
   XQT_REQUIRE(activation != nullptr && qweight != nullptr && scales != nullptr && output != nullptr);
+  const bool integer = zero_points == nullptr || variant == XQT_B200_VARIANT_AUTO_INTEGER;
+  if (variant == XQT_B200_VARIANT_AUTO_INTEGER) variant = XQT_B200_VARIANT_AUTO;
   if (out_f32) {
     // fp32 partial sums (K-sharded layers) are produced by the tensor-core GEMM only
     XQT_REQUIRE(variant == XQT_B200_VARIANT_AUTO || variant == XQT_B200_VARIANT_TCGEN05 ||
@@ -128,10 +130,10 @@ int xqt_b200_w4a16_run(const void* activation, const void* qweight, const void* 
     // the tensor-core GEMM folds the zero point into an exact integer subtraction: only a caller who
     // knows its zero points are integers may ask for it; AUTO takes it for symmetric weights only
     // (at large M the weights are dequantised in fp32 first, which serves any zero point)
-    if (variant == XQT_B200_VARIANT_TCGEN05 && zero_points != nullptr && !w4a16_gemm_tc_any_zero_point(m))
+    if (variant == XQT_B200_VARIANT_TCGEN05 && !integer && !w4a16_gemm_tc_any_zero_point(m))
       variant = XQT_B200_VARIANT_SIMT;
     // the fused form where it measures faster; with zero points only a caller who knows they are integers asks for it
-    if (variant == XQT_B200_VARIANT_TCGEN05 && zero_points == nullptr && !out_f32 &&
+    if (variant == XQT_B200_VARIANT_TCGEN05 && integer && !out_f32 &&
         w4a16_gemm_fused_preferred(m, n, k, padded_k, group_size))
       variant = XQT_B200_VARIANT_TCGEN05_FUSED;
   }

@@ -1,6 +1,8 @@
 // Native call path of the bound layers: a `Bound` object holds everything one layer call needs -- the checks of its
 // input, the shape of its output, its scratch, and the library calls to make with their resolved arguments -- and a
-// call goes from the Python argument to the kernel launches without running Python code.
+// call goes from the Python argument to the kernel launches without running Python code.  A layer that takes any number of
+// rows is one object too: row counts enter the resolved arguments as factors, so a prompt length that was never seen costs
+// what a repeated one does.
 //
 // What bounds it: a decode projection's kernel runs 4 us, and the same call made by a Python closure (attribute checks,
 // torch.empty, a 19-argument ctypes call) cost 12-17 us of host time, so every small call ran at the host's pace.
@@ -27,11 +29,17 @@
 
 namespace {
 
-// Where a pointer argument comes from; `value` is an address or a byte offset.
+// An integer argument that may depend on the number of rows.
+struct Number {
+  int value, per_row;
+  int at(int m) const { return value + per_row * m; }
+};
+
+// Where a pointer argument comes from; `value` is an address or a byte offset, to which `per_row` bytes are added per row.
 enum Source : int { kConst = 0, kInput = 1, kOutput = 2, kResidual = 3, kScratch = 4, kWorkspace = 5 };
 struct Pointer {
   int source;
-  intptr_t value;
+  intptr_t value, per_row;
 };
 
 // The library entry of a step.  Its arguments are its pointers, then its integers, in the order of the C prototype;
@@ -44,9 +52,36 @@ struct Step {
   int op;
   void* fn;
   std::vector<Pointer> ptrs;
-  std::vector<int> ints;
+  std::vector<Number> ints;
   Pointer ws;
-  size_t ws_bytes;
+  size_t ws_bytes;                       // or, for the rows m of a call:
+  size_t (*ws_need)(int m, int, int);
+  int ws_args[2];
+};
+
+// The calls of one range of row counts.  A layer that takes any number of rows has several; the first one whose range and
+// guards (library functions that say whether an entry serves a size) hold is taken.
+constexpr int kMaxInts = 11, kMaxSteps = 4;
+struct Guard {
+  void* fn;
+  Number rows;
+  std::vector<int> args;
+  bool holds(int m) const {
+    if (args.size() == 3) return reinterpret_cast<int (*)(int, int, int, int)>(fn)(rows.at(m), args[0], args[1], args[2]) != 0;
+    return reinterpret_cast<int (*)(int, int, int, int, int)>(fn)(rows.at(m), args[0], args[1], args[2], args[3]) != 0;
+  }
+};
+struct Plan {
+  int lo, hi;
+  std::vector<Guard> guards;
+  std::vector<Step> steps;
+  int64_t scratch_bytes, scratch_per_row;
+};
+// What a row count resolves to; the last one is kept, so a repeated count asks the library nothing.
+struct Resolved {
+  int m;
+  const Plan* plan;
+  size_t ws_bytes[kMaxSteps], ws_most;
 };
 
 // The workspaces of native.py's pool, mirrored here so that a call finds the current one without running Python code: per
@@ -88,17 +123,36 @@ struct Bound {
   PyObject* keep;
   at::ScalarType dtype, out_dtype;
   int device;
-  int64_t rows, k, n;
+  int64_t rows, k, n;    // rows < 0: any number that one of the plans takes
   bool any_rank;         // the input may have any leading dimensions that multiply to `rows`
   bool takes_residual;   // a third positional argument, [rows, n] in the input dtype
-  int64_t scratch_bytes;
   int tag;               // the workspace's
-  size_t ws_bytes;       // the largest workspace a step needs
-  std::vector<Step>* steps;
+  std::vector<Plan>* plans;
+  Resolved last;
 };
 
-int run_step(const Step& s, void* const* p, void* ws, cudaStream_t stream) {
-  const int* i = s.ints.data();
+const Resolved* resolve(Bound* b, int m) {
+  Resolved& r = b->last;
+  if (r.m == m) return &r;
+  for (const Plan& plan : *b->plans) {
+    if (m < plan.lo || m > plan.hi) continue;
+    bool holds = true;
+    for (const Guard& g : plan.guards) holds = holds && g.holds(m);
+    if (!holds) continue;
+    r.plan = &plan;
+    r.ws_most = 0;
+    for (size_t i = 0; i < plan.steps.size(); ++i) {
+      const Step& s = plan.steps[i];
+      r.ws_bytes[i] = s.ws_need != nullptr ? s.ws_need(m, s.ws_args[0], s.ws_args[1]) : s.ws_bytes;
+      if (s.ws.source == kWorkspace && r.ws_bytes[i] > r.ws_most) r.ws_most = r.ws_bytes[i];
+    }
+    r.m = m;
+    return &r;
+  }
+  return nullptr;
+}
+
+int run_step(const Step& s, void* const* p, const int* i, void* ws, size_t ws_bytes, cudaStream_t stream) {
   xqt_b200_stream_t st = (xqt_b200_stream_t)stream;
   switch (s.op) {
     case kDecodeLanes:
@@ -108,7 +162,7 @@ int run_step(const Step& s, void* const* p, void* ws, cudaStream_t stream) {
     case kW4A16Run:
       return reinterpret_cast<decltype(&xqt_b200_w4a16_run)>(s.fn)(
           p[0], p[1], p[2], p[3], (const float*)p[4], p[5], p[6], i[0], i[1], i[2], i[3], i[4], i[5], i[6], i[7], i[8], i[9], ws,
-          s.ws_bytes, i[10], st);
+          ws_bytes, i[10], st);
     case kSwiglu:
       return reinterpret_cast<decltype(&xqt_b200_swiglu)>(s.fn)(p[0], p[1], i[0], i[1], i[2], st);
     case kRotateQuantize:
@@ -117,20 +171,20 @@ int run_step(const Step& s, void* const* p, void* ws, cudaStream_t stream) {
     case kW8A8Gemm:
       return reinterpret_cast<decltype(&xqt_b200_w8a8_gemm_addend)>(s.fn)(p[0], p[1], (const float*)p[2], (const float*)p[3],
                                                                           (const float*)p[4], (const float*)p[5], p[6], i[0], i[1],
-                                                                          i[2], i[3], ws, s.ws_bytes, st);
+                                                                          i[2], i[3], ws, ws_bytes, st);
     case kLowrankDown:
       return reinterpret_cast<decltype(&xqt_b200_lowrank_down)>(s.fn)(p[0], p[1], (float*)p[2], p[3], i[0], i[1], i[2], st);
     case kW4A4Gemm:
       return reinterpret_cast<decltype(&xqt_b200_w4a4_gemm)>(s.fn)(p[0], (const float*)p[1], p[2], p[3], p[4], (const float*)p[5],
                                                                    (const float*)p[6], p[7], i[0], i[1], i[2], i[3], i[4], ws,
-                                                                   s.ws_bytes, st);
+                                                                   ws_bytes, st);
     case kW8A8LowrankGemm:
       return reinterpret_cast<decltype(&xqt_b200_w8a8_gemm_lowrank)>(s.fn)(p[0], p[1], (const float*)p[2], (const float*)p[3],
                                                                            (const float*)p[4], p[5], p[6], p[7], i[0], i[1], i[2], i[3],
-                                                                           ws, s.ws_bytes, st);
+                                                                           ws, ws_bytes, st);
     case kSwigluMlp:
       return reinterpret_cast<decltype(&xqt_b200_w4a16_swiglu_mlp)>(s.fn)(p[0], p[1], p[2], p[3], p[4], p[5], p[6], p[7], i[0], i[1], i[2], i[3],
-                                                                          i[4], i[5], i[6], i[7], i[8], i[9], ws, s.ws_bytes, st);
+                                                                          i[4], i[5], i[6], i[7], i[8], i[9], ws, ws_bytes, st);
     case kActPrologue: {
       float scale;                     // the first integer is the bit pattern of lora_scale
       memcpy(&scale, &i[0], sizeof(scale));
@@ -181,19 +235,25 @@ PyObject* call(PyObject* self, PyObject* const* args, size_t nargsf, PyObject* k
   if (!plain(x, b->dtype, b->device) || c10::cuda::current_device() != b->device) return slow();
   const auto shape = x.sizes();
   const int64_t dim = (int64_t)shape.size();
-  if (dim < 1 || shape[dim - 1] != b->k || x.numel() != b->rows * b->k || (!b->any_rank && dim != 2)) return slow();
+  if (dim < 1 || shape[dim - 1] != b->k || b->k < 1 || (!b->any_rank && dim != 2)) return slow();
+  const int64_t rows = x.numel() / b->k;
+  if (b->rows >= 0 ? rows != b->rows : rows < 1 || rows > INT32_MAX) return slow();
+  const Resolved* found = resolve(b, (int)rows);
+  if (found == nullptr) return slow();
+  const Resolved how = *found;                   // another thread may resolve another count while this one launches
+  const int m = how.m;
 
   const bool has_out = nargs >= 2 && args[1] != Py_None;
   if (has_out) {
     if (!THPVariable_Check(args[1])) return slow();
     const at::Tensor& o = THPVariable_Unpack(args[1]);
-    if (b->any_rank || !plain(o, b->out_dtype, b->device) || o.dim() != 2 || o.size(0) != b->rows || o.size(1) != b->n) return slow();
+    if (b->any_rank || !plain(o, b->out_dtype, b->device) || o.dim() != 2 || o.size(0) != rows || o.size(1) != b->n) return slow();
   }
   void* residual = nullptr;
   if (nargs == 3 && args[2] != Py_None) {
     if (!b->takes_residual || !THPVariable_Check(args[2])) return slow();
     const at::Tensor& r = THPVariable_Unpack(args[2]);
-    if (!plain(r, b->dtype, b->device) || r.dim() != 2 || r.size(0) != b->rows || r.size(1) != b->n) return slow();
+    if (!plain(r, b->dtype, b->device) || r.dim() != 2 || r.size(0) != rows || r.size(1) != b->n) return slow();
     residual = r.data_ptr();
   }
   const c10::Device device(c10::kCUDA, (c10::DeviceIndex)b->device);
@@ -201,33 +261,37 @@ PyObject* call(PyObject* self, PyObject* const* args, size_t nargsf, PyObject* k
   if (has_out) {
     out = THPVariable_Unpack(args[1]);
   } else if (dim == 2) {
-    out = at::detail::empty_cuda({b->rows, b->n}, b->out_dtype, device, c10::nullopt);
+    out = at::detail::empty_cuda({rows, b->n}, b->out_dtype, device, c10::nullopt);
   } else {
     std::vector<int64_t> oshape(shape.begin(), shape.end());
     oshape.back() = b->n;
     out = at::detail::empty_cuda(oshape, b->out_dtype, device, c10::nullopt);
   }
-  if (b->scratch_bytes > 0) scratch = at::detail::empty_cuda({b->scratch_bytes}, at::kByte, device, c10::nullopt);
+  const int64_t scratch_bytes = how.plan->scratch_bytes + how.plan->scratch_per_row * rows;
+  if (scratch_bytes > 0) scratch = at::detail::empty_cuda({scratch_bytes}, at::kByte, device, c10::nullopt);
   const cudaStream_t stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)b->device).stream();
   char* base[6] = {nullptr, static_cast<char*>(x.data_ptr()), static_cast<char*>(out.data_ptr()), static_cast<char*>(residual),
                    scratch.defined() ? static_cast<char*>(scratch.data_ptr()) : nullptr, nullptr};
   THPObjectPtr held;
-  if (b->workspace != Py_None) {
-    base[kWorkspace] = stream_space(b, stream, b->ws_bytes, held);
+  if (how.ws_most > 0) {
+    base[kWorkspace] = stream_space(b, stream, how.ws_most, held);
     if (base[kWorkspace] == nullptr) return nullptr;
   }
   int code = 0;
   size_t at_step = 0;
   {
     const WithoutGil released;
-    for (; at_step < b->steps->size(); ++at_step) {
-      const Step& s = (*b->steps)[at_step];
+    const std::vector<Step>& steps = how.plan->steps;
+    for (; at_step < steps.size(); ++at_step) {
+      const Step& s = steps[at_step];
       void* p[kMaxPointers];
+      int ints[kMaxInts];
       for (size_t i = 0; i < s.ptrs.size(); ++i) {
         char* from = base[s.ptrs[i].source];
-        p[i] = s.ptrs[i].source == kResidual && from == nullptr ? nullptr : from + s.ptrs[i].value;
+        p[i] = s.ptrs[i].source == kResidual && from == nullptr ? nullptr : from + (s.ptrs[i].value + s.ptrs[i].per_row * m);
       }
-      code = run_step(s, p, base[s.ws.source] + s.ws.value, stream);
+      for (size_t i = 0; i < s.ints.size(); ++i) ints[i] = s.ints[i].at(m);
+      code = run_step(s, p, ints, base[s.ws.source] + s.ws.value, how.ws_bytes[at_step], stream);
       if (code != 0) break;
     }
   }
@@ -253,10 +317,10 @@ PyObject* bound_call(PyObject* self, PyObject* const* args, size_t nargsf, PyObj
 }
 
 bool parse_pointer(PyObject* o, Pointer* p) {
-  long long value = 0;
+  long long value = 0, per_row = 0;
   int source = 0;
   if (PyTuple_Check(o)) {
-    if (!PyArg_ParseTuple(o, "iL", &source, &value)) return false;
+    if (!PyArg_ParseTuple(o, "iL|L", &source, &value, &per_row)) return false;
   } else {
     value = PyLong_AsLongLong(o);
     if (value == -1 && PyErr_Occurred()) return false;
@@ -265,31 +329,83 @@ bool parse_pointer(PyObject* o, Pointer* p) {
     PyErr_SetString(PyExc_ValueError, "Bound: unknown pointer source");
     return false;
   }
-  p->source = source;
-  p->value = (intptr_t)value;
+  *p = Pointer{source, (intptr_t)value, (intptr_t)per_row};
+  return true;
+}
+
+bool parse_number(PyObject* o, Number* n) {
+  n->per_row = 0;
+  if (PyTuple_Check(o)) return PyArg_ParseTuple(o, "ii", &n->value, &n->per_row) != 0;
+  const long v = PyLong_AsLong(o);
+  if (v == -1 && PyErr_Occurred()) return false;
+  n->value = (int)v;
   return true;
 }
 
 bool parse_step(PyObject* o, Step* s) {
-  PyObject *ptrs, *ints, *ws;
+  PyObject *ptrs, *ints, *ws, *ws_bytes;
   unsigned long long fn;
-  Py_ssize_t ws_bytes;
-  if (!PyArg_ParseTuple(o, "iKO!O!On", &s->op, &fn, &PyTuple_Type, &ptrs, &PyTuple_Type, &ints, &ws, &ws_bytes)) return false;
+  if (!PyArg_ParseTuple(o, "iKO!O!OO", &s->op, &fn, &PyTuple_Type, &ptrs, &PyTuple_Type, &ints, &ws, &ws_bytes)) return false;
   if (s->op < 0 || s->op >= kOpCount || fn == 0 || PyTuple_GET_SIZE(ptrs) != kPointerCount[s->op] || PyTuple_GET_SIZE(ints) != kIntCount[s->op]) {
     PyErr_SetString(PyExc_ValueError, "Bound: a step does not have the arguments of its library entry");
     return false;
   }
   s->fn = reinterpret_cast<void*>(fn);
-  s->ws_bytes = (size_t)ws_bytes;
+  s->ws_bytes = 0;
+  s->ws_need = nullptr;
+  if (PyTuple_Check(ws_bytes)) {
+    unsigned long long need;
+    if (!PyArg_ParseTuple(ws_bytes, "Kii", &need, &s->ws_args[0], &s->ws_args[1])) return false;
+    s->ws_need = reinterpret_cast<size_t (*)(int, int, int)>(need);
+  } else {
+    s->ws_bytes = PyLong_AsSize_t(ws_bytes);
+    if (PyErr_Occurred()) return false;
+  }
   s->ptrs.resize((size_t)PyTuple_GET_SIZE(ptrs));
   for (size_t i = 0; i < s->ptrs.size(); ++i)
     if (!parse_pointer(PyTuple_GET_ITEM(ptrs, (Py_ssize_t)i), &s->ptrs[i])) return false;
-  for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(ints); ++i) {
-    const long v = PyLong_AsLong(PyTuple_GET_ITEM(ints, i));
-    if (v == -1 && PyErr_Occurred()) return false;
-    s->ints.push_back((int)v);
-  }
+  s->ints.resize((size_t)PyTuple_GET_SIZE(ints));
+  for (size_t i = 0; i < s->ints.size(); ++i)
+    if (!parse_number(PyTuple_GET_ITEM(ints, (Py_ssize_t)i), &s->ints[i])) return false;
   return parse_pointer(ws, &s->ws);
+}
+
+// (function, rows, (3 or 4 integers))
+bool parse_guard(PyObject* o, Guard* g) {
+  unsigned long long fn;
+  PyObject *rows, *args;
+  if (!PyArg_ParseTuple(o, "KOO!", &fn, &rows, &PyTuple_Type, &args) || !parse_number(rows, &g->rows)) return false;
+  if (fn == 0 || PyTuple_GET_SIZE(args) < 3 || PyTuple_GET_SIZE(args) > 4) {
+    PyErr_SetString(PyExc_ValueError, "Bound: a guard takes a function of the row count and three or four integers");
+    return false;
+  }
+  g->fn = reinterpret_cast<void*>(fn);
+  for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(args); ++i) {
+    Number n;
+    if (!parse_number(PyTuple_GET_ITEM(args, i), &n)) return false;
+    g->args.push_back(n.value);
+  }
+  return true;
+}
+
+// (first row count, last row count, guards, steps, scratch bytes, scratch bytes per row)
+bool parse_plan(PyObject* o, Plan* p) {
+  PyObject *guards, *steps;
+  long long bytes, per_row;
+  if (!PyArg_ParseTuple(o, "iiO!O!LL", &p->lo, &p->hi, &PyTuple_Type, &guards, &PyTuple_Type, &steps, &bytes, &per_row)) return false;
+  if (PyTuple_GET_SIZE(steps) > kMaxSteps) {
+    PyErr_SetString(PyExc_ValueError, "Bound: too many steps");
+    return false;
+  }
+  p->scratch_bytes = bytes;
+  p->scratch_per_row = per_row;
+  p->guards.resize((size_t)PyTuple_GET_SIZE(guards));
+  for (size_t i = 0; i < p->guards.size(); ++i)
+    if (!parse_guard(PyTuple_GET_ITEM(guards, (Py_ssize_t)i), &p->guards[i])) return false;
+  p->steps.resize((size_t)PyTuple_GET_SIZE(steps));
+  for (size_t i = 0; i < p->steps.size(); ++i)
+    if (!parse_step(PyTuple_GET_ITEM(steps, (Py_ssize_t)i), &p->steps[i])) return false;
+  return true;
 }
 
 int bound_traverse(PyObject* self, visitproc visit, void* arg) {
@@ -312,36 +428,42 @@ void bound_dealloc(PyObject* self) {
   Bound* b = reinterpret_cast<Bound*>(self);
   PyObject_GC_UnTrack(self);
   bound_clear(self);
-  delete b->steps;
+  delete b->plans;
   Py_TYPE(self)->tp_free(self);
 }
 
 PyObject* make(PyTypeObject* type, PyObject* args, PyObject* kwargs) {
-  static const char* names[] = {"steps", "slow", "on_error", "dtype", "out_dtype", "device", "rows", "k", "n", "any_rank",
-                                "takes_residual", "scratch_bytes", "workspace", "tag", "keep", nullptr};
-  PyObject *steps, *slow, *on_error, *dtype, *out_dtype, *workspace = Py_None, *keep = Py_None;
+  static const char* names[] = {"plans", "slow", "on_error", "dtype", "out_dtype", "device", "rows", "k", "n", "any_rank",
+                                "takes_residual", "workspace", "tag", "keep", nullptr};
+  PyObject *plans, *slow, *on_error, *dtype, *out_dtype, *workspace = Py_None, *keep = Py_None;
   const char* tag = "run";
   int device, any_rank = 0, takes_residual = 0;
-  long long rows, k, n, scratch_bytes = 0;
-  if (!PyArg_ParseTupleAndKeywords(args, kwargs, "O!OOOOiLLL|ppLOsO", const_cast<char**>(names), &PyTuple_Type, &steps, &slow, &on_error,
-                                   &dtype, &out_dtype, &device, &rows, &k, &n, &any_rank, &takes_residual, &scratch_bytes, &workspace,
+  long long rows, k, n;
+  if (!PyArg_ParseTupleAndKeywords(args, kwargs, "O!OOOOiLLL|ppOsO", const_cast<char**>(names), &PyTuple_Type, &plans, &slow, &on_error,
+                                   &dtype, &out_dtype, &device, &rows, &k, &n, &any_rank, &takes_residual, &workspace,
                                    &tag, &keep))
     return nullptr;
   if (!THPDtype_Check(dtype) || !THPDtype_Check(out_dtype)) {
     PyErr_SetString(PyExc_TypeError, "Bound: dtype and out_dtype must be torch dtypes");
     return nullptr;
   }
-  auto parsed = std::make_unique<std::vector<Step>>((size_t)PyTuple_GET_SIZE(steps));
-  for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(steps); ++i)
-    if (!parse_step(PyTuple_GET_ITEM(steps, i), &(*parsed)[(size_t)i])) return nullptr;
+  auto parsed = std::make_unique<std::vector<Plan>>((size_t)PyTuple_GET_SIZE(plans));
+  for (size_t i = 0; i < parsed->size(); ++i) {
+    Plan& plan = (*parsed)[i];
+    if (!parse_plan(PyTuple_GET_ITEM(plans, (Py_ssize_t)i), &plan)) return nullptr;
+    for (const Step& s : plan.steps)
+      if (s.ws.source == kWorkspace && workspace == Py_None) {
+        PyErr_SetString(PyExc_ValueError, "Bound: a step needs a workspace");
+        return nullptr;
+      }
+  }
   Bound* b = reinterpret_cast<Bound*>(type->tp_alloc(type, 0));
   if (b == nullptr) return nullptr;
   b->vectorcall = bound_call;
-  b->steps = parsed.release();
+  b->plans = parsed.release();
+  b->last = Resolved{};
+  b->last.m = -1;
   b->tag = tag_id(tag);
-  b->ws_bytes = 0;
-  for (const Step& s : *b->steps)
-    if (s.ws.source == kWorkspace && s.ws_bytes > b->ws_bytes) b->ws_bytes = s.ws_bytes;
   Py_INCREF(slow); b->slow = slow;
   Py_INCREF(on_error); b->on_error = on_error;
   Py_INCREF(workspace); b->workspace = workspace;
@@ -352,7 +474,6 @@ PyObject* make(PyTypeObject* type, PyObject* args, PyObject* kwargs) {
   b->rows = rows; b->k = k; b->n = n;
   b->any_rank = any_rank != 0;
   b->takes_residual = takes_residual != 0;
-  b->scratch_bytes = scratch_bytes;
   return reinterpret_cast<PyObject*>(b);
 }
 

@@ -23,10 +23,10 @@ from torch import nn
 from . import native
 from .contracts import PackedWeight
 from .errors import XQTBackendError
-from .hostcall import INPUT, OUTPUT, WORKSPACE, bound_call, step, weak_method
+from .hostcall import INPUT, MANY_ROWS, OUTPUT, bound_layer, plan, weak_method
 from .layout import signed_storage_to_unsigned
 from .ops import awq as awq_ops
-from .ops.w4a16 import resolve_w4a16_variant, version_of, w4a16_linear, with_version
+from .ops.w4a16 import integer_zero_points_now, version_of, w4a16_linear, w4a16_step, with_version
 
 _DTYPE_NAME = {torch.float16: "fp16", torch.bfloat16: "bf16"}
 MAX_DECODE_ROWS = 16
@@ -61,14 +61,13 @@ class AWQW4A16Linear(nn.Module):
         self._prepared: dict[torch.dtype, tuple] = {}
         self._bound: dict[tuple[int, torch.dtype], Callable] = {}
         self._residual_bound: dict[tuple[int, torch.dtype], Callable] = {}
-        # (rows, dtype) -> (tensors it was built from, bound call, its execution report): calls of forward() that need no
-        # other work than the bound call
-        self._hot: dict[tuple[int, torch.dtype], tuple] = {}
+        # dtype -> (tensors it was built from, their versions and addresses, bound call): above the decode sizes, any row count
+        self._gemm: dict[torch.dtype, tuple] = {}
         self._native_only = False
         self._native_only_rows: frozenset[int] = frozenset()
         self._native_only_dtype: torch.dtype | None = None
         self._native_only_released_bytes = 0
-        self._last_execution: dict[str, Any] = {"implementation": "not_run", "native": False}
+        self._last_execution: tuple[str, int, torch.dtype] | None = None       # kernel, rows, dtype
 
     # ------------------------------------------------------------------ construction helpers
     @classmethod
@@ -210,7 +209,7 @@ class AWQW4A16Linear(nn.Module):
             raise ValueError(f"native-only AWQ W4A16 rows must be between 1 and {MAX_DECODE_ROWS}")
         for r in frozen:
             self.bind(rows=r, dtype=dtype)
-        self._hot.clear()
+        self._gemm.clear()
         released = self.canonical_qweight.numel() * self.canonical_qweight.element_size()
         self.canonical_qweight = None
         # the execution PackedWeight dropped its canonical bytes too
@@ -222,62 +221,52 @@ class AWQW4A16Linear(nn.Module):
         return int(released)
 
     # ------------------------------------------------------------------ forward
-    def _hot_call(self, rows: int, dtype: torch.dtype) -> tuple | None:
-        """The entry of :attr:`_hot` for ``rows`` rows, built when it is missing or a buffer has been replaced since."""
+    def _apply(self, fn, recurse=True):
+        self._gemm.clear()                                 # a module that moves leaves no copy of its buffers behind
+        return super()._apply(fn, recurse)
+
+    def _gemm_call(self, dtype: torch.dtype) -> Callable | None:
+        """The bound call for more than 16 rows, made when there is none or a buffer has changed since; None where
+        ``w4a16_linear`` has to look at the buffers itself."""
 
         buffers = self._buffers
-        zeros = buffers["weight_zero_point"]
-        made_from = (buffers["canonical_qweight"], buffers["weight_scale"], zeros, buffers["bias"])
-        canonical, scales, _, bias = made_from
-        # what the entry holds in a form of its own: the answer to "are the zero points integers", a bias of another dtype
+        canonical, scales, zeros, bias = static = (buffers["canonical_qweight"], buffers["weight_scale"], buffers["weight_zero_point"], buffers["bias"])
+        # what the call holds in a form of its own: the answer to "are the zero points integers", a bias of another dtype
         own = (zeros, None if bias is None or bias.dtype == torch.float32 else bias)
-        versions = tuple(version_of(t) for t in own)
-        hit = self._hot.get((rows, dtype))
-        if hit is not None and all(a is b for a, b in zip(hit[0], made_from)) and hit[3] == versions:
-            return hit
-        if self._native_only or canonical is None or not canonical.is_cuda or dtype not in _DTYPE_NAME or rows < 1 \
-                or any(t is not None and t.device != canonical.device for t in made_from):
+        state = tuple(version_of(t) for t in own) + tuple(None if t is None else t.data_ptr() for t in static)
+        hit = self._gemm.get(dtype)
+        if hit is not None and hit[1] == state and all(a is b for a, b in zip(hit[0], static)):
+            return hit[2]
+        if self._native_only or canonical is None or not canonical.is_cuda or dtype not in _DTYPE_NAME:
             return None
-        if rows <= MAX_DECODE_ROWS:
-            run, kernel = self.bind(rows=rows, dtype=dtype), "w4a16_decode_cl_kernel"
-        else:
-            n, k, padded_k, group, device = self.output_features, self.input_features, int(canonical.shape[1]) * 2, self.group_size, canonical.device
-            # whatever w4a16_linear converts or refuses is left to it, and what changes unseen
-            if any(t is not None and t.is_inference() for t in own) or any(t is not None and not t.is_contiguous() for t in made_from) or canonical.dtype != torch.uint8 or canonical.ndim != 2 \
-                    or canonical.shape[0] != n or scales.dtype not in native.DTYPE_CODE or tuple(scales.shape) != (n, padded_k // group) \
-                    or (zeros is not None and (zeros.dtype != scales.dtype or zeros.shape != scales.shape)) \
-                    or (bias is not None and bias.numel() != n):
-                return None
-            variant = resolve_w4a16_variant(rows, n, k, padded_k, group, zero_points=zeros)
-            nbytes = native.library().xqt_b200_w4a16_workspace_bytes(rows, n, k)
-            bias32 = None if bias is None else bias.reshape(-1).to(torch.float32).contiguous()     # a cast of the module casts the buffer
-            gemm = step("xqt_b200_w4a16_run", ((INPUT, 0), canonical, scales, zeros, bias32, 0, (OUTPUT, 0)),
-                        (rows, n, k, padded_k, group, 0, native.DTYPE_CODE[dtype], native.DTYPE_CODE[scales.dtype], native.DTYPE_CODE[dtype],
-                         0, native.VARIANT[variant]), (WORKSPACE, 0), nbytes)
-            run = bound_call([gemm], weak_method(self._forward_flat), dtype=dtype, device=device, rows=rows, k=k, n=n,
-                             workspace="run", keep=(made_from, bias32), symbols="xqt_b200_w4a16_run")
-            kernel = "w4a16 tcgen05 GEMM"
-        if len(self._hot) >= 512:
-            self._hot.clear()
-        hit = (made_from, run, self._report(kernel, rows, dtype), versions)
-        self._hot[(rows, dtype)] = hit
-        return hit
-
-    def _report(self, kernel: str, rows: int, dtype: torch.dtype) -> dict[str, Any]:
-        return {
-            "implementation": "b200_awq_w4a16", "native": True, "kernel": kernel, "rows": rows,
-            "input_features": self.input_features, "output_features": self.output_features, "dtype": _DTYPE_NAME[dtype],
-            "bias": self._has_bias, "layout": awq_ops.LANES_LAYOUT,
-        }
+        n, k, group, device = self.output_features, self.input_features, self.group_size, canonical.device
+        padded_k = int(canonical.shape[-1]) * 2
+        # whatever w4a16_linear converts or refuses is left to it, and what changes unseen
+        if any(t is not None and t.is_inference() for t in own) or any(t is not None and (t.device != device or not t.is_contiguous()) for t in static) \
+                or canonical.dtype != torch.uint8 or canonical.ndim != 2 or canonical.shape[0] != n \
+                or scales.dtype not in native.DTYPE_CODE or tuple(scales.shape) != (n, padded_k // group) \
+                or (zeros is not None and (zeros.dtype != scales.dtype or zeros.shape != scales.shape)) \
+                or (bias is not None and bias.numel() != n):
+            return None
+        integer = integer_zero_points_now(zeros)
+        if integer is None:
+            return None
+        bias32 = None if bias is None else bias.reshape(-1).to(torch.float32).contiguous()     # a cast of the module casts the buffer
+        gemm = w4a16_step((INPUT, 0), canonical, scales, zeros, bias32, (OUTPUT, 0), k=k, group_size=group, nibble_signed=False, dtype=dtype, integer=integer)
+        run = bound_layer([plan([gemm], rows=(MAX_DECODE_ROWS + 1, MANY_ROWS))], weak_method(self._forward_flat), dtype=dtype, device=device,
+                          rows=None, k=k, n=n, workspace="run", keep=(static, bias32), symbols="xqt_b200_w4a16_run")
+        self._gemm[dtype] = (static, state, run)
+        return run
 
     def forward(self, inputs: torch.Tensor) -> torch.Tensor:
         if self.training:
             raise RuntimeError("AWQ W4A16 native path requires eval mode")
-        if inputs.ndim == 2:
-            hit = self._hot_call(inputs.shape[0], inputs.dtype)
-            if hit is not None:
-                output = hit[1](inputs)
-                self._last_execution = hit[2]
+        if inputs.ndim == 2 and inputs.shape[1] == self.input_features and inputs.dtype in _DTYPE_NAME:
+            rows, dtype = inputs.shape[0], inputs.dtype
+            run = self._gemm_call(dtype) if rows > MAX_DECODE_ROWS else (self.bind(rows=rows, dtype=dtype) if rows else None)
+            if run is not None:
+                output = run(inputs)
+                self._last_execution = ("w4a16_decode_cl_kernel" if rows <= MAX_DECODE_ROWS else "w4a16 tcgen05 GEMM", rows, dtype)
                 return output
         return self._forward_flat(inputs)
 
@@ -297,13 +286,20 @@ class AWQW4A16Linear(nn.Module):
             output = w4a16_linear(flat, self.canonical_qweight, self.weight_scale, self.weight_zero_point, self.bias,
                                   group_size=self.group_size, nibble_signed=False)
             kernel = "w4a16 tcgen05 GEMM"
-        self._last_execution = self._report(kernel, rows, flat.dtype)
+        self._last_execution = (kernel, rows, flat.dtype)
         return output.reshape(*inputs.shape[:-1], self.output_features)
 
     def execution_metadata(self) -> dict[str, Any]:
         """Metadata of the most recent invocation plus the frozen-state report."""
 
-        meta = dict(self._last_execution)
+        meta: dict[str, Any] = {"implementation": "not_run", "native": False}
+        if self._last_execution is not None:
+            kernel, rows, dtype = self._last_execution
+            meta = {
+                "implementation": "b200_awq_w4a16", "native": True, "kernel": kernel, "rows": rows,
+                "input_features": self.input_features, "output_features": self.output_features, "dtype": _DTYPE_NAME[dtype],
+                "bias": self._has_bias, "layout": awq_ops.LANES_LAYOUT,
+            }
         meta.update({
             "native_only": self._native_only, "native_only_rows": sorted(self._native_only_rows),
             "native_only_dtype": None if self._native_only_dtype is None else str(self._native_only_dtype),

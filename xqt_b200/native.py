@@ -25,6 +25,7 @@ FP16, BF16, FP32 = 0, 1, 2
 ACT = {"none": 0, "relu": 1, "gelu": 2, "silu": 3}
 VARIANT = {"auto": 0, "simt": 1, "gemv": 2, "tcgen05": 3, "tcgen05_fused": 4}
 VARIANT_NAMES = {value: key for key, value in VARIANT.items()}
+AUTO_INTEGER = 5          # "auto" for a caller who knows that its zero points are integers
 DTYPE_CODE = {torch.float16: FP16, torch.bfloat16: BF16, torch.float32: FP32}
 
 _P, _I, _Z = ctypes.c_void_p, ctypes.c_int, ctypes.c_size_t
@@ -236,6 +237,6 @@ def workspace_status(device: torch.device) -> int:
 
 
 __all__ = [
-    "ACT", "BF16", "DTYPE_CODE", "FP16", "FP32", "LIBRARY_PATH", "SIGNATURES", "VARIANT", "VARIANT_NAMES",
+    "ACT", "AUTO_INTEGER", "BF16", "DTYPE_CODE", "FP16", "FP32", "LIBRARY_PATH", "SIGNATURES", "VARIANT", "VARIANT_NAMES",
     "available", "check", "host", "library", "ptr", "status_word", "stream_handle", "version", "workspace", "workspace_status",
 ]

@@ -21,9 +21,10 @@ import torch.distributed as dist
 from .. import native
 from ..contracts import PackedWeight, PackedWeightMetadata
 from ..errors import XQTBackendError
-from ..hostcall import INPUT, OUTPUT, WORKSPACE, ScratchPlan, bound_call, step, weak_method
+from ..hostcall import INPUT, MANY_ROWS, OUTPUT, ROWS, SCRATCH, WORKSPACE, bound_layer, guard, plan, step, weak_method
 from ..parallel import shard_packed_weight
-from .w4a16 import _integer_zero_points, bind_w4a16_decode, glu_row_order, prepare_decode, resolve_w4a16_variant, version_of, w4a16_linear, with_version
+from .w4a16 import (_integer_zero_points, bind_w4a16_decode, glu_row_order, integer_zero_points_now, prepare_decode, version_of, w4a16_linear,
+                    w4a16_step, with_version)
 
 
 def swiglu(gate_up: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
@@ -141,29 +142,21 @@ class _Linear:
             and self.scales.dtype in native.DTYPE_CODE and tuple(self.scales.shape) == shape \
             and (self.zeros is None or (self.zeros.dtype == self.scales.dtype and self.zeros.shape == self.scales.shape))
 
-    def decode_steps(self, m: int, source: tuple, target: tuple, *, glu: bool) -> list:
-        """The decode launches of ``m`` rows (one per 16) as steps of a bound call."""
+    def decode_step(self, first: int, rows, source: tuple, target: tuple, *, glu: bool) -> tuple:
+        """The decode launch of ``rows`` rows from row ``first`` on as a step of a bound layer."""
 
-        lib, status, params = native.library(), native.status_word(self.qweight.device), self.tiled.params
-        if not lib.xqt_b200_w4a16_decode_lanes_supported(min(m, 16), self.n, self.k, self.group):
-            raise XQTBackendError(f"B200 W4A16 decode does not cover N={self.n}, K={self.k}, group={self.group}")
+        status, params = native.status_word(self.qweight.device), self.tiled.params
         code, width = native.DTYPE_CODE[self.dtype], self.n // 2 if glu else self.n
-        return [step("xqt_b200_w4a16_decode_lanes",
-                     ((source[0], source[1] + 2 * r0 * self.k), self.tiled.weights, params[0], params[1] if self.tiled.has_zero_point else 0,
-                      0, 0, (target[0], target[1] + 2 * r0 * width), status),
-                     (min(16, m - r0), self.n, self.k, self.group, self.tiled.nibble_signed, code, native.DTYPE_CODE[params.dtype],
-                      code, 2 if glu else 0)) for r0 in range(0, m, 16)]
+        return step("xqt_b200_w4a16_decode_lanes",
+                    ((source[0], source[1] + 2 * first * self.k), self.tiled.weights, params[0], params[1] if self.tiled.has_zero_point else 0,
+                     0, 0, (target[0], target[1] + 2 * first * width), status),
+                    (rows, self.n, self.k, self.group, self.tiled.nibble_signed, code, native.DTYPE_CODE[params.dtype], code, 2 if glu else 0))
 
-    def gemm_steps(self, m: int, source: tuple, target: tuple) -> tuple[list, int]:
-        """The canonical-weight GEMM of ``m`` rows as a step of a bound call, and the workspace bytes it needs."""
+    def gemm_step(self, source: tuple, target: tuple) -> tuple:
+        """The canonical-weight GEMM of any number of rows as a step of a bound layer."""
 
-        lib = native.library()
-        variant = resolve_w4a16_variant(m, self.n, self.k, int(self.qweight.shape[1]) * 2, self.group, zero_points=self.zeros)
-        nbytes = lib.xqt_b200_w4a16_workspace_bytes(m, self.n, self.k)
-        code = native.DTYPE_CODE[self.dtype]
-        return [step("xqt_b200_w4a16_run", (source, self.qweight, self.scales, self.zeros, 0, 0, target),
-                     (m, self.n, self.k, int(self.qweight.shape[1]) * 2, self.group, self.signed, code,
-                      native.DTYPE_CODE[self.scales.dtype], code, 0, native.VARIANT[variant]), (WORKSPACE, 0), nbytes)], nbytes
+        return w4a16_step(source, self.qweight, self.scales, self.zeros, None, target, k=self.k, group_size=self.group,
+                          nibble_signed=self.signed, dtype=self.dtype, integer=_integer_zero_points(self.zeros))
 
     def partial_into(self, x: torch.Tensor, peer) -> None:
         """Decode-size fp32 partial sums of a K-sharded layer, written into the slot of ``peer`` (a counted
@@ -214,7 +207,10 @@ class W4A16SwiGLUMLP:
             up = shard_packed_weight(up, world=world, rank=rank, axis=0)
             down = shard_packed_weight(down, world=world, rank=rank, axis=1)
         self.world, self.group, self.dtype = world, group, dtype
-        self._native: dict[int, tuple] = {}       # row count -> (zero-point versions, bound call), single-GPU blocks
+        # single-GPU blocks: the bound calls by 16 rows up to CHUNKED_DECODE_MAX_ROWS, and the one above, with the state of the
+        # tensors it was built from
+        self._decode: dict[int, object] = {}
+        self._gemm: tuple | None = None
         self._can_bind = world == 1 and local_linear is None and swiglu_fn is None
         self._swiglu = swiglu_fn or swiglu
         self._fuse_gating = swiglu_fn is None and os.environ.get("XQT_B200_FUSED_SWIGLU", "1") not in {"0", ""}
@@ -239,55 +235,77 @@ class W4A16SwiGLUMLP:
 
     def __call__(self, x: torch.Tensor) -> torch.Tensor:
         if self._can_bind:
-            zeros = self._zero_versions()
-            hit = self._native.get(x.shape[0])
-            if hit is None or hit[0] != zeros:
-                if len(self._native) >= 512:
-                    self._native.clear()
-                hit = (zeros, self._bind(int(x.shape[0])))
-                self._native[x.shape[0]] = hit
-            return hit[1](x)
+            m = x.shape[0]
+            if m <= CHUNKED_DECODE_MAX_ROWS:
+                run = self._decode.get((m + 15) // 16)
+                if run is None:
+                    run = self._decode[(m + 15) // 16] = self._bind_decode((m + 15) // 16)
+                return run(x)
+            run = self._gemm_call()
+            if run is not None:
+                return run(x)
         return self._forward(x)
 
-    def _zero_versions(self) -> tuple:
-        return (version_of(self.gate_up.zeros), version_of(self.down.zeros))
+    def _bound(self, plans: list, keep: tuple = ()):
+        return bound_layer(plans, weak_method(self._forward), dtype=self.dtype, device=self.gate_up.qweight.device, rows=None, k=self.gate_up.k,
+                           n=self.hidden, workspace="run", keep=(self.gate_up, self.down, *keep), symbols="bound W4A16 SwiGLU MLP")
 
-    def _bind(self, m: int):
-        """The block for ``m`` rows as one bound call: the launches of :meth:`_forward` with their arguments resolved."""
+    def _bind_decode(self, chunks: int):
+        """The launches of :meth:`_forward` for decode sizes of ``chunks`` times 16 rows (the last chunk may have fewer) as one
+        bound layer."""
 
-        device, scratch, nbytes = self.gate_up.qweight.device, ScratchPlan(), 0
-        inter, lanes = self.inter_local, self.down.tiled.layout == "lanes"
-        served = self.gate_up.glu and lanes if m <= CHUNKED_DECODE_MAX_ROWS else self.gate_up.canonical_served and self.down.canonical_served
-        if m < 1 or device.type != "cuda" or not served:
+        gate_up, down, device = self.gate_up, self.down, self.gate_up.qweight.device
+        if device.type != "cuda" or not gate_up.glu or down.tiled.layout != "lanes" or chunks < 1:
             return weak_method(self._forward)
-        if m <= CHUNKED_DECODE_MAX_ROWS:
-            h = scratch.take(2 * m * inter)
-            steps = self.gate_up.decode_steps(m, (INPUT, 0), h, glu=True) + self.down.decode_steps(m, h, (OUTPUT, 0), glu=False)
-        elif self._one_entry(m):
-            nbytes = native.library().xqt_b200_w4a16_swiglu_mlp_workspace_bytes(m, self.hidden, inter)
-            gu, dn = self.gate_up, self.down
-            steps = [step("xqt_b200_w4a16_swiglu_mlp", ((INPUT, 0), gu.qweight, gu.scales, gu.zeros, dn.qweight, dn.scales, dn.zeros, (OUTPUT, 0)),
-                          (m, self.hidden, inter, gu.group, dn.group, gu.signed, dn.signed, native.DTYPE_CODE[self.dtype],
-                           native.DTYPE_CODE[gu.scales.dtype], native.DTYPE_CODE[dn.scales.dtype]), (WORKSPACE, 0), nbytes)]
-        else:
-            h = scratch.take(2 * m * inter)
-            both = scratch.take(4 * m * inter)
-            first, need = self.gate_up.gemm_steps(m, (INPUT, 0), both)
-            last, more = self.down.gemm_steps(m, h, (OUTPUT, 0))
-            steps = first + [step("xqt_b200_swiglu", (both, h), (m, inter, native.DTYPE_CODE[self.dtype]))] + last
-            nbytes = max(need, more)
-        return bound_call(steps, weak_method(self._forward), dtype=self.dtype, device=device, rows=m, k=self.gate_up.k, n=self.hidden,
-                          scratch_bytes=scratch.nbytes, workspace="run" if nbytes else None,
-                          keep=(self.gate_up, self.down, native.status_word(device)), symbols="bound W4A16 SwiGLU MLP")
+        h, last = (SCRATCH, 0), 16 * (chunks - 1)
+        parts = [(first, 16) for first in range(0, last, 16)] + [(last, (-last, 1))]
+        steps = [gate_up.decode_step(first, rows, (INPUT, 0), h, glu=True) for first, rows in parts]
+        steps += [down.decode_step(first, rows, h, (OUTPUT, 0), glu=False) for first, rows in parts]
+        served = tuple(guard("xqt_b200_w4a16_decode_lanes_supported", rows, layer.n, layer.k, layer.group)
+                       for layer in (gate_up, down) for rows in {rows for _, rows in parts})
+        return self._bound([plan(steps, rows=(last + 1, last + 16), guards=served, scratch=(0, 2 * self.inter_local))], (native.status_word(device),))
+
+    def _gemm_call(self):
+        """The launches of :meth:`_forward` above the decode sizes as one bound layer, made when there is none or a tensor has changed
+        since; None where ``w4a16_linear`` has to look at the tensors itself."""
+
+        gu, dn = self.gate_up, self.down
+        static = (gu.qweight, gu.scales, gu.zeros, dn.qweight, dn.scales, dn.zeros)
+        state = (version_of(gu.zeros), version_of(dn.zeros), *(None if t is None else t.data_ptr() for t in static))
+        if self._gemm is not None and self._gemm[0] == state:
+            return self._gemm[1]
+        if gu.qweight.device.type != "cuda" or not (gu.canonical_served and dn.canonical_served) \
+                or any(t is not None and t.is_inference() for t in (gu.zeros, dn.zeros)) \
+                or integer_zero_points_now(gu.zeros) is None or integer_zero_points_now(dn.zeros) is None:
+            return None
+        plans, inter = [], self.inter_local
+        if self._fuse_gating and self._one_entry_form():
+            code = native.DTYPE_CODE
+            entry = step("xqt_b200_w4a16_swiglu_mlp", ((INPUT, 0), gu.qweight, gu.scales, gu.zeros, dn.qweight, dn.scales, dn.zeros, (OUTPUT, 0)),
+                         (ROWS, self.hidden, inter, gu.group, dn.group, gu.signed, dn.signed, code[self.dtype], code[gu.scales.dtype], code[dn.scales.dtype]),
+                         (WORKSPACE, 0), ("xqt_b200_w4a16_swiglu_mlp_workspace_bytes", self.hidden, inter))
+            plans.append(plan([entry], rows=(CHUNKED_DECODE_MAX_ROWS + 1, MANY_ROWS),
+                              guards=(guard("xqt_b200_w4a16_swiglu_mlp_supported", ROWS, self.hidden, inter, gu.group, dn.group),)))
+        both, h = (SCRATCH, 0), (SCRATCH, 0, 4 * inter)          # [rows, 2 * inter], then [rows, inter]
+        plans.append(plan([gu.gemm_step((INPUT, 0), both), step("xqt_b200_swiglu", (both, h), (ROWS, inter, native.DTYPE_CODE[self.dtype])),
+                           dn.gemm_step(h, (OUTPUT, 0))], rows=(CHUNKED_DECODE_MAX_ROWS + 1, MANY_ROWS), scratch=(0, 6 * inter)))
+        self._gemm = (state, self._bound(plans, static))
+        return self._gemm[1]
+
+    def _one_entry_form(self) -> bool:
+        """Both weights are what the single library call of the block takes: unpadded, integer zero points."""
+
+        gu, dn = self.gate_up, self.down
+        exact = 2 * int(gu.qweight.shape[1]) == gu.k == self.hidden and 2 * int(dn.qweight.shape[1]) == dn.k and gu.n == 2 * self.inter_local
+        return exact and _integer_zero_points(gu.zeros) and _integer_zero_points(dn.zeros)
 
     def _one_entry(self, m: int) -> bool:
         """Both projections take the CTA-pair GEMM: the block is then one library call with the gating in the gate/up epilogue
         (unless ``XQT_B200_FUSED_SWIGLU=0`` turned the fused gating off when the block was built)."""
 
         gu, dn = self.gate_up, self.down
-        exact = 2 * int(gu.qweight.shape[1]) == gu.k == self.hidden and 2 * int(dn.qweight.shape[1]) == dn.k and gu.n == 2 * self.inter_local
-        return self._fuse_gating and exact and bool(native.library().xqt_b200_w4a16_swiglu_mlp_supported(m, self.hidden, self.inter_local, gu.group, dn.group)) \
-            and _integer_zero_points(gu.zeros) and _integer_zero_points(dn.zeros)
+        return self._fuse_gating and self._one_entry_form() and bool(
+            native.library().xqt_b200_w4a16_swiglu_mlp_supported(m, self.hidden, self.inter_local, gu.group, dn.group))
 
     def _forward(self, x: torch.Tensor) -> torch.Tensor:
         h = self.gate_up.gated(x) if isinstance(self.gate_up, _Linear) else None     # decode sizes: one launch

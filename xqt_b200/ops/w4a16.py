@@ -11,7 +11,7 @@ from __future__ import annotations
 import torch
 
 from .. import native
-from ..hostcall import INPUT, OUTPUT, RESIDUAL, WORKSPACE, bound_call, step
+from ..hostcall import INPUT, OUTPUT, RESIDUAL, ROWS, WORKSPACE, bound_call, step
 from ..errors import XQTBackendError
 from ..weakid import WeakIdDict
 
@@ -182,6 +182,18 @@ def w4a16_linear(
             native.VARIANT[variant], stream)
     native.check(code, "xqt_b200_w4a16_run")
     return out
+
+
+def w4a16_step(source: tuple, qweight: torch.Tensor, scales: torch.Tensor, zero_points: torch.Tensor | None, bias32: torch.Tensor | None,
+               target: tuple, *, k: int, group_size: int, nibble_signed: bool, dtype: torch.dtype, integer: bool) -> tuple:
+    """:func:`w4a16_linear` (``variant="auto"``, output in the activation dtype) of any number of rows as a step of a bound layer.
+    The tensors are what it takes unconverted; ``integer``: :func:`_integer_zero_points`."""
+
+    n, code = int(qweight.shape[0]), native.DTYPE_CODE[dtype]
+    return step("xqt_b200_w4a16_run", (source, qweight, scales, zero_points, bias32, 0, target),
+                (ROWS, n, k, int(qweight.shape[1]) * 2, group_size, nibble_signed, code, native.DTYPE_CODE[scales.dtype], code, 0,
+                 native.AUTO_INTEGER if integer else native.VARIANT["auto"]),
+                (WORKSPACE, 0), ("xqt_b200_w4a16_workspace_bytes", n, k))
 
 
 def bind_w4a16_linear(
