@@ -2,9 +2,12 @@
 
 from __future__ import annotations
 
+import copy
+import gc
 import os
 import subprocess
 import sys
+import weakref
 
 import pytest
 
@@ -44,3 +47,22 @@ def test_fake_tensors_raise_in_python():
     child = subprocess.run([sys.executable, "-c", _SCRIPT], cwd=ROOT, capture_output=True, text=True, timeout=300,
                            env={**os.environ, "PYTHONPATH": str(ROOT)})
     assert child.returncode == 0 and "survived" in child.stdout, child.stderr[-2000:]
+
+
+def test_bound_objects_behave_like_closures():
+    host = pytest.importorskip("xqt_b200._host")
+    import torch
+
+    run = host.Bound(((1, 1, (), (), 0, 0),), lambda *args: args, None, torch.bfloat16, torch.bfloat16, 0, 1, 8, 8, keep=("kept",))
+    run.label = "x"
+    assert copy.copy(run) is run and copy.deepcopy(run) is run and run.label == "x" and run.__dict__ == {"label": "x"}
+    for wrong in (lambda: delattr(run, "slow"), lambda: setattr(run, "slow", None), lambda: delattr(run, "keep"), lambda: setattr(run, "keep", ())):
+        with pytest.raises((TypeError, AttributeError)):
+            wrong()
+    run.slow = lambda *args: "replaced"
+    assert run(1) == "replaced"
+    gone, cycle = weakref.ref(run), [run]
+    run.cycle = cycle
+    del run, cycle
+    gc.collect()
+    assert gone() is None

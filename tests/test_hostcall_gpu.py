@@ -2,6 +2,7 @@
 
 from __future__ import annotations
 
+import copy
 import gc
 import weakref
 
@@ -181,3 +182,43 @@ def test_weights_first_seen_inside_a_graph_capture():
     torch.cuda.synchronize()
     assert torch.equal(one, want) and torch.equal(two, want)
     assert torch.equal(module(x), w4a16_linear(x, w.qweight, w.scales, w.zero_points, group_size=128, nibble_signed=False, variant="tcgen05_fused"))
+
+
+def test_copies_and_saved_layers(tmp_path):
+    """A layer that has run can be copied and saved; what comes back is a layer of its own."""
+    n, k = 256, 512
+    module = AWQW4A16Linear(_layer(n, k, 50), bias=torch.randn((n,), generator=seeded(51)).to(DEV)).eval()
+    frozen = AWQW4A16Linear(_layer(n, k, 52)).eval()
+    frozen.freeze_native_inference(device=DEV, dtype=torch.bfloat16, rows=(1,))
+    block = W4A16SwiGLUMLP(_layer(256, k, 53), _layer(256, k, 54), _layer(k, 256, 55), device=DEV)
+    x = torch.randn((300, k), generator=seeded(56)).to(DEV, torch.bfloat16)
+    sizes = (1, 16, 20, 40, 300)
+    want, want_block, want_frozen = [module(x[:m]) for m in sizes], [block(x[:m]) for m in sizes], frozen(x[:1])
+    block.gate_up.gated(x[:4])
+    torch.save((module, frozen, block), tmp_path / "layers.pt")
+    for other, other_frozen, other_block in (copy.deepcopy((module, frozen, block)), torch.load(tmp_path / "layers.pt", weights_only=False)):
+        assert other._execution_weight is not module._execution_weight and not other._bound and not other_block._decode
+        assert all(torch.equal(other(x[:m]), y) for m, y in zip(sizes, want))
+        assert all(torch.equal(other_block(x[:m]), y) for m, y in zip(sizes, want_block))
+        assert torch.equal(other_frozen(x[:1]), want_frozen)
+        with pytest.raises(RuntimeError):
+            other_frozen(x[:2])
+        other.weight_scale.zero_()                          # its own scales
+        other_block.down.scales.zero_()
+        assert not other_block(x[:40]).any() and torch.equal(other(x[:40]), other.bias.to(torch.bfloat16).expand(40, n))
+        assert torch.equal(module(x[:40]), want[3]) and torch.equal(block(x[:40]), want_block[3])
+    # saved before the present fields existed
+    old, old_block = module.__getstate__(), block.__getstate__()
+    for name in ("_gemm", "_decode", "_can_bind", "_fuse_gating"):
+        old.pop(name, None), old_block.pop(name, None)
+    old["_last_execution"] = {"implementation": "not_run", "native": False}
+    for kind, state, y in ((AWQW4A16Linear, old, want), (W4A16SwiGLUMLP, old_block, want_block)):
+        back = kind.__new__(kind)
+        back.__setstate__(state)
+        assert torch.equal(back(x[:300]), y[4]) and torch.equal(back(x[:1]), y[0])
+    run = module.bind(rows=1, dtype=torch.bfloat16)
+    run.note = "attributes and weak references, as the closures took them"
+    assert copy.deepcopy(run) is run and weakref.ref(run)() is run and run.note
+    for wrong in ("delattr(run, 'slow')", "setattr(run, 'slow', 3)", "delattr(run, 'keep')"):
+        with pytest.raises((TypeError, AttributeError)):
+            eval(wrong)

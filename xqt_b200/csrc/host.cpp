@@ -129,6 +129,7 @@ struct Bound {
   int tag;               // the workspace's
   std::vector<Plan>* plans;
   Resolved last;
+  PyObject *dict, *weakrefs;      // like the closures it stands for, it takes attributes and weak references
 };
 
 const Resolved* resolve(Bound* b, int m) {
@@ -414,6 +415,7 @@ int bound_traverse(PyObject* self, visitproc visit, void* arg) {
   Py_VISIT(b->on_error);
   Py_VISIT(b->workspace);
   Py_VISIT(b->keep);
+  Py_VISIT(b->dict);
   return 0;
 }
 int bound_clear(PyObject* self) {
@@ -422,11 +424,13 @@ int bound_clear(PyObject* self) {
   Py_CLEAR(b->on_error);
   Py_CLEAR(b->workspace);
   Py_CLEAR(b->keep);
+  Py_CLEAR(b->dict);
   return 0;
 }
 void bound_dealloc(PyObject* self) {
   Bound* b = reinterpret_cast<Bound*>(self);
   PyObject_GC_UnTrack(self);
+  if (b->weakrefs != nullptr) PyObject_ClearWeakRefs(self);
   bound_clear(self);
   delete b->plans;
   Py_TYPE(self)->tp_free(self);
@@ -486,9 +490,36 @@ PyObject* bound_new(PyTypeObject* type, PyObject* args, PyObject* kwargs) {
   }
 }
 
-PyMemberDef bound_members[] = {{"keep", T_OBJECT, offsetof(Bound, keep), 0, "the objects whose memory the calls use"},
-                               {"slow", T_OBJECT, offsetof(Bound, slow), 0, "the callable that gets what the native path does not take"},
+PyMemberDef bound_members[] = {{"keep", T_OBJECT, offsetof(Bound, keep), READONLY, "the objects whose memory the calls use"},
                                {nullptr, 0, 0, 0, nullptr}};
+
+PyObject* get_slow(PyObject* self, void*) {
+  PyObject* slow = reinterpret_cast<Bound*>(self)->slow;
+  if (slow == nullptr) slow = Py_None;
+  Py_INCREF(slow);
+  return slow;
+}
+int set_slow(PyObject* self, PyObject* value, void*) {
+  if (value == nullptr || !PyCallable_Check(value)) {
+    PyErr_SetString(PyExc_TypeError, "Bound.slow must be callable");
+    return -1;
+  }
+  Py_INCREF(value);
+  PyObject* before = reinterpret_cast<Bound*>(self)->slow;
+  reinterpret_cast<Bound*>(self)->slow = value;
+  Py_XDECREF(before);
+  return 0;
+}
+PyGetSetDef bound_getset[] = {{"slow", get_slow, set_slow, "the callable that gets what the native path does not take", nullptr},
+                              {"__dict__", PyObject_GenericGetDict, PyObject_GenericSetDict, nullptr, nullptr},
+                              {nullptr, nullptr, nullptr, nullptr, nullptr}};
+
+// As for a closure, a copy is the object itself (the addresses it holds are those of tensors that `keep` shares).
+PyObject* copy_self(PyObject* self, PyObject*) {
+  Py_INCREF(self);
+  return self;
+}
+PyMethodDef bound_methods[] = {{"__copy__", copy_self, METH_NOARGS, nullptr}, {"__deepcopy__", copy_self, METH_O, nullptr}, {nullptr, nullptr, 0, nullptr}};
 PyTypeObject bound_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
 
 // set_workspace(device, stream, tag, tensor): the pool's buffer from now on; the one before it is released
@@ -554,6 +585,10 @@ PyMODINIT_FUNC PyInit__host(void) {
   bound_type.tp_call = PyVectorcall_Call;
   bound_type.tp_vectorcall_offset = offsetof(Bound, vectorcall);
   bound_type.tp_members = bound_members;
+  bound_type.tp_getset = bound_getset;
+  bound_type.tp_methods = bound_methods;
+  bound_type.tp_dictoffset = offsetof(Bound, dict);
+  bound_type.tp_weaklistoffset = offsetof(Bound, weakrefs);
   if (PyType_Ready(&bound_type) < 0) return nullptr;
   PyObject* m = PyModule_Create(&host_module);
   if (m == nullptr) return nullptr;

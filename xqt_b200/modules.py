@@ -225,6 +225,15 @@ class AWQW4A16Linear(nn.Module):
         self._gemm.clear()                                 # a module that moves leaves no copy of its buffers behind
         return super()._apply(fn, recurse)
 
+    def __getstate__(self) -> dict[str, Any]:
+        # bound calls hold addresses of this module's tensors: a copy or a saved module makes its own
+        return {**self.__dict__, "_bound": {}, "_residual_bound": {}, "_gemm": {}}
+
+    def __setstate__(self, state: dict[str, Any]) -> None:
+        # a module saved before these fields existed
+        last = state.get("_last_execution")
+        super().__setstate__({**state, "_gemm": {}, "_last_execution": last if isinstance(last, tuple) else None})
+
     def _gemm_call(self, dtype: torch.dtype) -> Callable | None:
         """The bound call for more than 16 rows, made when there is none or a buffer has changed since; None where
         ``w4a16_linear`` has to look at the buffers itself."""

@@ -87,6 +87,10 @@ class _Linear:
         if self.tiled is None:
             self.tiled = prepare_decode(self.qweight, self.scales, self.zeros, group_size=self.group, nibble_signed=self.signed)
 
+    def __getstate__(self) -> dict:
+        # bound calls hold addresses of this layer's tensors: a copy makes its own
+        return {**self.__dict__, "_bound": {}, "_gated": {}}
+
     def gated(self, x: torch.Tensor) -> torch.Tensor | None:
         """``silu(gate) * up`` of a fused gate/up layer in one decode launch per 16 rows, or None where that form does
         not apply (not a glu layer, too many rows)."""
@@ -232,6 +236,15 @@ class W4A16SwiGLUMLP:
 
             # on the lanes layout the reduction is the counted (graph-safe) form: the call number lives on the device
             self._peer = PeerAllReduce(device, 16 * self.hidden, group, counted=self.down.tiled.layout == "lanes")
+
+    def __getstate__(self) -> dict:
+        return {**self.__dict__, "_decode": {}, "_gemm": None}
+
+    def __setstate__(self, state: dict) -> None:
+        # a block saved before these fields existed
+        gate_up = state["gate_up"]
+        self.__dict__.update({"_can_bind": state["world"] == 1 and isinstance(gate_up, _Linear) and state["_swiglu"] is swiglu,
+                              "_fuse_gating": getattr(gate_up, "glu", False), **state, "_decode": {}, "_gemm": None})
 
     def __call__(self, x: torch.Tensor) -> torch.Tensor:
         if self._can_bind:
