@@ -46,3 +46,22 @@ def test_int8_gemm_is_exact(m, n, k, dtype):
     magnitude = plain.double().abs() + bias.double().abs() + la[:, :32].double().abs() @ up[:, :32].double().abs().t()
     assert ((got - want).abs() <= eps * want.abs() + 2.0 ** -18 * magnitude + 2.0 ** -24).all()
     assert native.workspace_status(DEV) == 0
+
+
+@pytest.mark.parametrize("m,n,k", [(5, 136, 256), (300, 4096, 512)])         # the single and the pair form
+def test_scales_and_bias_at_any_address(m, n, k):
+    gen = seeded(m + n)
+    a, b = (torch.randint(-128, 128, s, generator=gen, dtype=torch.int8).to(DEV) for s in ((m, k), (n, k)))
+    a_scale = (torch.rand(m, generator=gen) * 0.01).to(DEV)
+    lib, scratch, stream = native.library(), native.workspace(DEV, 256, "gemm"), native.stream_handle(DEV)
+    values = torch.rand(2 * n + 8, generator=gen).to(DEV)
+
+    def run(scale, bias):
+        out = torch.empty((m, n), device=DEV, dtype=torch.bfloat16)
+        native.check(lib.xqt_b200_w8a8_gemm(a.data_ptr(), b.data_ptr(), a_scale.data_ptr(), scale.data_ptr(), native.ptr(bias), out.data_ptr(), m, n, k,
+                                            native.BF16, scratch.data_ptr(), scratch.numel(), stream), "xqt_b200_w8a8_gemm")
+        return out
+
+    for at, bias_at in ((1, None), (2, 0), (0, 3), (3, 1)):
+        scale, bias = values[at:at + n], None if bias_at is None else values[n + bias_at:2 * n + bias_at]
+        assert torch.equal(run(scale, bias), run(scale.clone(), None if bias is None else bias.clone()))

@@ -73,7 +73,9 @@ __device__ __forceinline__ void gs_store16(const ScaledParams& p, int row, int c
   }
 }
 
-template <int CG, typename T, bool LOW>
+// QUADS: column scales and bias lie on 16 bytes.  A caller's slices may not: then one load per column (a form of its own: a test
+// in the epilogue cost the smallest layers 2 %).
+template <int CG, typename T, bool LOW, bool QUADS>
 __global__ void __launch_bounds__(gs::kThreads, 1)
 gemm_scaled_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b, const __grid_constant__ CUtensorMap tm_l,
                    const __grid_constant__ CUtensorMap tm_u, const __grid_constant__ ScaledParams p) {
@@ -234,10 +236,18 @@ gemm_scaled_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const bool in = col + 4 * j < p.n;
-          const float4 v = in ? __ldg(reinterpret_cast<const float4*>(p.col_scale + col) + j) : make_float4(0.f, 0.f, 0.f, 0.f);
-          cs[4 * j] = v.x; cs[4 * j + 1] = v.y; cs[4 * j + 2] = v.z; cs[4 * j + 3] = v.w;
-          const float4 b = in && p.bias != nullptr ? __ldg(reinterpret_cast<const float4*>(p.bias + col) + j) : make_float4(0.f, 0.f, 0.f, 0.f);
-          add[4 * j] = b.x; add[4 * j + 1] = b.y; add[4 * j + 2] = b.z; add[4 * j + 3] = b.w;
+          if constexpr (!QUADS) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              cs[4 * j + e] = in ? __ldg(p.col_scale + col + 4 * j + e) : 0.f;
+              add[4 * j + e] = in && p.bias != nullptr ? __ldg(p.bias + col + 4 * j + e) : 0.f;
+            }
+          } else {
+            const float4 v = in ? __ldg(reinterpret_cast<const float4*>(p.col_scale + col) + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+            cs[4 * j] = v.x; cs[4 * j + 1] = v.y; cs[4 * j + 2] = v.z; cs[4 * j + 3] = v.w;
+            const float4 b = in && p.bias != nullptr ? __ldg(reinterpret_cast<const float4*>(p.bias + col) + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+            add[4 * j] = b.x; add[4 * j + 1] = b.y; add[4 * j + 2] = b.z; add[4 * j + 3] = b.w;
+          }
         }
       };
       fetch(n0 + c0);
@@ -391,7 +401,7 @@ ScaledPlan scaled_plan(int m, int n, int k, bool low) {
   return best;
 }
 
-template <int CG, typename T, bool LOW>
+template <int CG, typename T, bool LOW, bool QUADS>
 int launch_scaled(const void* a, const void* b, const void* low_a, const void* low_b, ScaledParams p, int k, cudaStream_t stream) {
   using namespace gs;
   CUtensorMap tm_a, tm_b, tm_l, tm_u;
@@ -410,7 +420,7 @@ int launch_scaled(const void* a, const void* b, const void* low_a, const void* l
   int stages = (kSmemBudget - 1024 - reduce) / stage_bytes;
   p.stages = stages > kMaxStages ? kMaxStages : stages;
   const size_t smem = (size_t)p.stages * stage_bytes + reduce + 1024;
-  auto kern = gemm_scaled_kernel<CG, T, LOW>;
+  auto kern = gemm_scaled_kernel<CG, T, LOW, QUADS>;
   XQT_SMEM_OPT_IN(kern, kSmemBudget);
   const int tiles = p.mtiles * p.ntiles;
   int grid, cluster;
@@ -438,7 +448,7 @@ int gemm_scaled_launch(const void* a, const void* b, const float* row_scale, con
   XQT_REQUIRE(m > 0 && n > 0 && k > 0 && k % 16 == 0 && n % 8 == 0 && ((uintptr_t)addend & 15) == 0);
   XQT_REQUIRE(out_dtype == XQT_B200_BF16 || out_dtype == XQT_B200_FP16);
   XQT_REQUIRE(a != nullptr && b != nullptr && row_scale != nullptr && col_scale != nullptr && out != nullptr && status != nullptr);
-  XQT_REQUIRE(((uintptr_t)out & 15) == 0 && ((uintptr_t)col_scale & 15) == 0 && ((uintptr_t)bias & 15) == 0);
+  XQT_REQUIRE(((uintptr_t)out & 15) == 0 && ((uintptr_t)row_scale & 3) == 0 && ((uintptr_t)col_scale & 3) == 0 && ((uintptr_t)bias & 3) == 0);
   XQT_REQUIRE((low_a != nullptr) == (low_b != nullptr));
   const bool low = low_a != nullptr;
   ScaledPlan plan = scaled_plan(m, n, k, low);
@@ -448,12 +458,14 @@ int gemm_scaled_launch(const void* a, const void* b, const float* row_scale, con
   // rows past the last token are not fetched (a box past the matrix costs the copy engine as much as one inside); what the
   // tile holds there reaches only sums that are not stored
   p.a_rows = plan.cg == 1 && m < gs::kBM ? (m + 7) / 8 * 8 : gs::kBM;
+  const bool quads = ((uintptr_t)col_scale & 15) == 0 && ((uintptr_t)bias & 15) == 0;
   p.wide = n % 16 == 0 && ((uintptr_t)out & 31) == 0;
   p.row_scale = row_scale; p.col_scale = col_scale; p.bias = bias; p.addend = addend; p.out = out; p.status = status;
-#define XQT_GS(T) (plan.cg == 2 ? (low ? launch_scaled<2, T, true>(a, b, low_a, low_b, p, k, stream) : launch_scaled<2, T, false>(a, b, low_a, low_b, p, k, stream)) \
-                                : (low ? launch_scaled<1, T, true>(a, b, low_a, low_b, p, k, stream) : launch_scaled<1, T, false>(a, b, low_a, low_b, p, k, stream)))
+#define XQT_GSQ(CG, T, LOW) (quads ? launch_scaled<CG, T, LOW, true>(a, b, low_a, low_b, p, k, stream) : launch_scaled<CG, T, LOW, false>(a, b, low_a, low_b, p, k, stream))
+#define XQT_GS(T) (plan.cg == 2 ? (low ? XQT_GSQ(2, T, true) : XQT_GSQ(2, T, false)) : (low ? XQT_GSQ(1, T, true) : XQT_GSQ(1, T, false)))
   return out_dtype == XQT_B200_BF16 ? XQT_GS(__nv_bfloat16) : XQT_GS(__half);
 #undef XQT_GS
+#undef XQT_GSQ
 }
 
 }  // namespace xqt_b200
