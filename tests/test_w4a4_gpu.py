@@ -3,6 +3,8 @@ and scales bit-exact; output rel-L2 <= 1e-3 against fp32((q_a s_a) @ (q_w s_w)^T
 
 from __future__ import annotations
 
+import dataclasses
+
 import pytest
 import torch
 
@@ -159,3 +161,30 @@ def test_config3_full_size(factors):
     torch.cuda.synchronize()
     assert native.workspace_status(DEV) == 0
     assert o16.rel_l2(dense.cpu(), ref) <= 1.5e-3
+
+
+def test_inputs_at_any_address_and_workspaces_that_do_not_fit():
+    from xqt_b200 import quantize
+    from xqt_b200.errors import XQTBackendError
+    from xqt_b200.ops import w4a4 as op
+    m, n, k, rank = 70, 256, 512, 16
+    w = torch.randn((n, k), generator=seeded(80)) * 0.02
+    down, up, residual = quantize.svd_split(w, rank)
+    codes, scale, _ = quantize.quantize_residual_int4(residual, group_size=64)
+    packed = op.pack_svdq_w4a4_linear(None, down.to(DEV, torch.bfloat16), up.to(DEV, torch.bfloat16), None, packed_residual=codes.to(DEV),
+                                      residual_scale=scale.to(DEV), rotation=quantize.regular_rotation(64))
+    x = torch.randn((m, k), generator=seeded(81)).to(DEV, torch.bfloat16)
+    odd = torch.empty(m * k + 1, device=DEV, dtype=torch.bfloat16)[1:].view(m, k).copy_(x)
+    want = op.svdq_w4a4_linear(x, packed)
+    # the separate kernels, which serve such an input, round the low-rank sums in another order
+    for y in (op.svdq_w4a4_linear(odd, packed), op.bind_svdq_w4a4_linear(packed, rows=m)(odd)):
+        assert (y.float() - want.float()).norm() <= 1e-3 * want.float().norm()
+    ws = op.allocate_w4a4_workspace(m, packed, with_lora_rank=rank)
+    assert torch.equal(op.svdq_w4a4_linear(x, packed, workspace=ws), want) and torch.equal(op.bind_svdq_w4a4_linear(packed, ws, rows=m)(x), want)
+    for field, wrong in (("quantized_activation", ws.quantized_activation.float()), ("activation_scales", ws.activation_scales[:m]),
+                         ("activation_scales", ws.activation_scales.half()), ("rotated_activation", ws.rotated_activation.half())):
+        bad = dataclasses.replace(ws, **{field: wrong})
+        with pytest.raises(XQTBackendError):
+            op.svdq_w4a4_linear(x, packed, workspace=bad)
+        with pytest.raises(XQTBackendError):
+            op.bind_svdq_w4a4_linear(packed, bad, rows=m)(x)

@@ -239,6 +239,7 @@ PyObject* call(PyObject* self, PyObject* const* args, size_t nargsf, PyObject* k
   if (dim < 1 || shape[dim - 1] != b->k || b->k < 1 || (!b->any_rank && dim != 2)) return slow();
   const int64_t rows = x.numel() / b->k;
   if (b->rows >= 0 ? rows != b->rows : rows < 1 || rows > INT32_MAX) return slow();
+  if ((reinterpret_cast<uintptr_t>(x.data_ptr()) & 15) != 0) return slow();      // the entries' loads are 16 bytes wide
   const Resolved* found = resolve(b, (int)rows);
   if (found == nullptr) return slow();
   const Resolved how = *found;                   // another thread may resolve another count while this one launches

@@ -206,6 +206,17 @@ def native_w4a4_version() -> str:
     return native.version()
 
 
+def _buffers_fit(workspace: W4A4Workspace, m: int, k: int, dtype: torch.dtype) -> bool:
+    """Whether the workspace's buffers are what :func:`rotate_quantize` takes for ``m`` rows with tile-major scales (where they are
+    not, it is called and raises), at addresses the fused prologue takes."""
+
+    tiles = -(-m // TILE) * TILE
+    want = ((workspace.quantized_activation, torch.int8, m, k), (workspace.activation_scales, torch.float32, tiles, k // GROUP),
+            (workspace.rotated_activation, dtype, m, k))
+    return all(t is not None and t.dtype == dt and t.ndim == 2 and t.shape[0] >= rows and t.shape[1] == columns and t[:rows].is_contiguous()
+               and t.data_ptr() % 16 == 0 for t, dt, rows, columns in want)
+
+
 def svdq_w4a4_linear(inputs: torch.Tensor, packed: PackedSVDQW4A4Linear, *, workspace: W4A4Workspace | None = None, lora_scale: float = 1.0,
                      return_parts: bool = False, form: str = "auto"):
     """Full forward: rotation (``packed.rotation``; None = input already rotated), int4 activations
@@ -240,6 +251,7 @@ def svdq_w4a4_linear(inputs: torch.Tensor, packed: PackedSVDQW4A4Linear, *, work
     kind, block = _KIND[None if rot is None else rot.kind], 0 if rot is None else rot.block
     # one kernel for rotation, quantisation and down projection where it serves the options
     fused = direct and packed.act_granularity == "group" and x.dtype == packed.dtype and x.is_cuda and bool(packed.rank) \
+        and x.data_ptr() % 16 == 0 and (workspace is None or _buffers_fit(workspace, m, k, packed.dtype)) \
         and bool(lib.xqt_b200_act_prologue_supported(k, kind, block, 6))
     if fused:
         if buffers is None:
@@ -346,7 +358,7 @@ def bind_svdq_w4a4_linear(packed: PackedSVDQW4A4Linear, workspace: W4A4Workspace
         return svdq_w4a4_linear(inputs, packed, workspace=workspace, lora_scale=lora_scale)
 
     if lora_scale != 1.0 or k % (1 if packed.rotation is None else packed.rotation.block) or rows < 1 \
-            or int(workspace.quantized_activation.shape[1]) != k or workspace.rotated_activation is None:
+            or not _buffers_fit(workspace, rows, k, dtype):
         run.keep = (packed, workspace)
         return run
     # the calls of the unbound form with every argument resolved: prologue with tile-major scales, down projection into
