@@ -54,3 +54,45 @@ def test_bound_call_reuses_its_workspace():
     assert torch.equal(bound(x), svdq_w8a8_linear(x, packed))
     with pytest.raises(Exception):
         bound(x[:10])
+
+
+def test_workspace_fields_and_inputs_at_any_address():
+    from xqt_b200.errors import XQTBackendError
+    from xqt_b200.ops import svdq_w8a8 as op
+    m, n, k = 20, 264, 512
+    w, down, up = _layer(n, k, 16, 70, torch.bfloat16)
+    packed, plain = op.pack_svdq_w8a8_linear(w.to(DEV), down.to(DEV), up.to(DEV)), op.pack_svdq_w8a8_linear(w.to(DEV), None, None)
+    x = torch.randn((m, k), generator=seeded(71)).to(DEV, torch.bfloat16)
+    odd = torch.empty(m * k + 1, device=DEV, dtype=torch.bfloat16)[1:].view(m, k).copy_(x)        # two bytes past a 16-byte boundary
+    want, want_plain = op.svdq_w8a8_linear(x, packed), op.w8a8_linear(x, packed)
+    assert torch.equal(op.w8a8_linear(odd, packed), want_plain) and torch.equal(op.svdq_w8a8_linear(odd, plain), op.svdq_w8a8_linear(x, plain))
+    assert torch.equal(op.bind_svdq_w8a8_linear(plain, rows=m)(odd), op.svdq_w8a8_linear(x, plain))
+    # the workspace by its fields, as callers build it
+    ws = op.allocate_svdq_w8a8_workspace(m, packed)
+    assert tuple(ws.lora_activation.shape) == (m, 32) and tuple(ws.low_rank_output.shape) == (m, n)
+    assert ws.lora_activation.dtype == ws.low_rank_output.dtype == torch.float32 and ws.low_rank_output is ws.low_rank_output
+    again = op.W8A8SVDQWorkspace(ws.quantized_activation, ws.activation_scales, ws.lora_activation, ws.lora_activation16, ws.low_rank_output)
+    assert torch.equal(op.svdq_w8a8_linear(x, packed, workspace=again), want)
+    other = op.allocate_svdq_w8a8_workspace(m, op.pack_svdq_w8a8_linear(w[:128].contiguous().to(DEV), down.to(DEV), up[:128].to(DEV)))
+    with pytest.raises(ValueError):
+        op.svdq_w8a8_linear(x, packed, workspace=other)                      # another layer's N
+    for field, wrong in (("quantized_activation", ws.quantized_activation.float()), ("activation_scales", ws.activation_scales.half()),
+                         ("activation_scales", ws.activation_scales[: m // 2]), ("quantized_activation", torch.empty((k, m), device=DEV, dtype=torch.int8).t())):
+        bad = op.W8A8SVDQWorkspace(**{**ws.__dict__, field: wrong})
+        with pytest.raises((XQTBackendError, ValueError)):
+            op.svdq_w8a8_linear(x, packed, workspace=bad)
+        with pytest.raises((XQTBackendError, ValueError)):
+            op.bind_svdq_w8a8_linear(packed, bad, rows=m)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_up_projection_entry(dtype):
+    """``xqt_b200_lowrank_up``, the fp32 product of a caller's own low-rank activations."""
+    from xqt_b200 import native
+    m, n = 130, 264
+    la, up = (torch.randn(s, generator=seeded(sum(s))).to(DEV, dtype) for s in ((m, 64), (n, 64)))
+    out, scratch = torch.empty((m, n), device=DEV), native.workspace(DEV, 256, "gemm")
+    native.check(native.library().xqt_b200_lowrank_up(la.data_ptr(), up.data_ptr(), out.data_ptr(), m, n, 64, native.DTYPE_CODE[dtype], scratch.data_ptr(),
+                                                      scratch.numel(), native.stream_handle(DEV)), "xqt_b200_lowrank_up")
+    # exact products, 64 of them summed in fp32: 2^-24 of the partial sums for each addition
+    assert ((out.double() - la.double() @ up.double().t()).abs() <= 64 * 2.0 ** -24 * (la.double().abs() @ up.double().abs().t())).all()

@@ -18,6 +18,7 @@ import torch
 from .. import native
 from ..errors import XQTBackendError
 from ..hostcall import INPUT, OUTPUT, WORKSPACE, bound_call, float_bits, step
+from .activation import rotate_quantize
 
 RANK_PAD = 32          # the down projection's width
 UP_PAD = 64            # the up projection's K extent (one 64-element tensor-core K block)
@@ -40,15 +41,53 @@ class PackedSVDQW8A8Linear:
         return RANK_PAD
 
 
+@dataclass(frozen=True)
+class _Unallocated:
+    """A workspace field that the layer's own kernels do not use: allocated when somebody reads it."""
+
+    shape: tuple[int, int]
+    dtype: torch.dtype
+    device: torch.device
+
+
+class _OnDemand:
+    def __set_name__(self, owner, name: str) -> None:
+        self.name = name
+
+    def __get__(self, instance, owner=None) -> torch.Tensor:
+        if instance is None:
+            raise AttributeError(self.name)          # to the dataclass: a field without a default
+        value = instance.__dict__[self.name]
+        if isinstance(value, _Unallocated):
+            value = instance.__dict__[self.name] = torch.empty(value.shape, dtype=value.dtype, device=value.device)
+        return value
+
+    def __set__(self, instance, value) -> None:
+        instance.__dict__[self.name] = value
+
+
 @dataclass
 class W8A8SVDQWorkspace:
     quantized_activation: torch.Tensor     # int8 [rows, K]
     activation_scales: torch.Tensor        # fp32 [rows]
+    lora_activation: torch.Tensor = _OnDemand()        # fp32 [rows, 32]: for callers of xqt_b200_lowrank_down / _up of their own
     lora_activation16: torch.Tensor        # dtype [rows, 64], columns past 32 stay zero
+    low_rank_output: torch.Tensor = _OnDemand()        # fp32 [rows, N], likewise
 
     @property
     def padded_rows(self) -> int:
         return int(self.quantized_activation.shape[0])
+
+    def _check(self, packed: PackedSVDQW8A8Linear, rows: int, low_rank: bool) -> None:
+        k, n = packed.input_features, packed.output_features
+        if self.padded_rows < rows or int(self.quantized_activation.shape[1]) != k or int(self.__dict__["low_rank_output"].shape[1]) != n:
+            raise ValueError("workspace extent does not match inputs")
+        for tensor, dtype, shape in ((self.quantized_activation, torch.int8, (rows, k)), (self.activation_scales, torch.float32, (rows,)),
+                                     (self.lora_activation16, packed.dtype, (rows, UP_PAD))):
+            if tensor is self.lora_activation16 and not low_rank:
+                continue
+            if tensor.dtype != dtype or tuple(tensor[:rows].shape) != shape or not tensor[:rows].is_contiguous():
+                raise XQTBackendError("SVDQ W8A8: workspace buffers do not match the layer")
 
 
 def native_svdq_w8a8_shape_supported(input_features: int, output_features: int, rank: int) -> bool:
@@ -100,11 +139,13 @@ def pack_svdq_w8a8_linear(residual_weight: torch.Tensor, down_weight: torch.Tens
 
 
 def allocate_svdq_w8a8_workspace(rows: int, packed: PackedSVDQW8A8Linear) -> W8A8SVDQWorkspace:
-    rows, k, device = int(rows), packed.input_features, packed.qweight.device
+    rows, k, n, device = int(rows), packed.input_features, packed.output_features, packed.qweight.device
     return W8A8SVDQWorkspace(
         quantized_activation=torch.empty((rows, k), dtype=torch.int8, device=device),
         activation_scales=torch.empty((rows,), dtype=torch.float32, device=device),
-        lora_activation16=torch.zeros((rows, UP_PAD), dtype=packed.dtype, device=device))
+        lora_activation=_Unallocated((rows, RANK_PAD), torch.float32, device),
+        lora_activation16=torch.zeros((rows, UP_PAD), dtype=packed.dtype, device=device),
+        low_rank_output=_Unallocated((rows, n), torch.float32, device))
 
 
 def _forward(inputs: torch.Tensor, packed: PackedSVDQW8A8Linear, workspace: W8A8SVDQWorkspace | None, lora_scale: float,
@@ -121,16 +162,17 @@ def _forward(inputs: torch.Tensor, packed: PackedSVDQW8A8Linear, workspace: W8A8
     if m == 0:
         return out
     ws = workspace or allocate_svdq_w8a8_workspace(m, packed)
-    if ws.padded_rows < m or int(ws.quantized_activation.shape[1]) != k:
-        raise ValueError("workspace extent does not match inputs")
+    low_rank = low_rank and bool(packed.rank)
+    ws._check(packed, m, low_rank)
     codes, scales, la = ws.quantized_activation[:m], ws.activation_scales[:m], ws.lora_activation16[:m]
     lib, stream, dcode = native.library(), native.stream_handle(device), native.DTYPE_CODE[packed.dtype]
-    low_rank = low_rank and bool(packed.rank)
     with torch.cuda.device(device):
         scratch = native.workspace(device, 256, "gemm")
-        native.check(lib.xqt_b200_act_prologue(x.data_ptr(), 0, codes.data_ptr(), scales.data_ptr(), packed.down.data_ptr() if low_rank else 0,
-                                               la.data_ptr() if low_rank else 0, lora_scale, m, k, 0, 0, 9, 3 if low_rank else 0, dcode, stream),
-                     "xqt_b200_act_prologue")
+        if low_rank:
+            native.check(lib.xqt_b200_act_prologue(x.data_ptr(), 0, codes.data_ptr(), scales.data_ptr(), packed.down.data_ptr(), la.data_ptr(),
+                                                   lora_scale, m, k, 0, 0, 9, 3, dcode, stream), "xqt_b200_act_prologue")
+        else:                                                # serves an input at any address
+            rotate_quantize(x, None, bits=8, out=(ws.quantized_activation, ws.activation_scales), scale_in_act_dtype=True)
         head = (codes.data_ptr(), packed.qweight.data_ptr(), scales.data_ptr(), packed.weight_scales.data_ptr(), native.ptr(packed.bias))
         tail = (out.data_ptr(), m, n, k, dcode, scratch.data_ptr(), scratch.numel(), stream)
         if low_rank:
@@ -166,8 +208,11 @@ def bind_svdq_w8a8_linear(packed: PackedSVDQW8A8Linear, workspace: W8A8SVDQWorks
     if workspace.padded_rows < rows:
         raise ValueError("workspace row extent does not match rows")
     k, n, dtype, device, scale = packed.input_features, packed.output_features, packed.dtype, packed.qweight.device, float(lora_scale)
-    if int(workspace.quantized_activation.shape[1]) != k:
-        raise ValueError("workspace extent does not match the packed layer")
+    # a workspace may be shared by layers of several sizes: its memory is what counts here
+    for tensor, held, count in ((workspace.quantized_activation, torch.int8, rows * k), (workspace.activation_scales, torch.float32, rows),
+                                (workspace.lora_activation16, dtype, rows * UP_PAD if packed.rank else 0)):
+        if count and (tensor.dtype != held or not tensor.is_contiguous() or tensor.numel() < count):
+            raise ValueError("workspace extent does not match the packed layer")
     native.workspace(device, 256, "gemm")            # the current stream's status word, made now
     dcode = native.DTYPE_CODE[dtype]
     codes, scales, la = workspace.quantized_activation, workspace.activation_scales, workspace.lora_activation16
