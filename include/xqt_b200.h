@@ -254,7 +254,9 @@ int xqt_b200_w4a16_decode_static_status(unsigned int* host_status, xqt_b200_stre
  * quantize_w4a4_act_fuse_lora (svdq_w4a4_sm89_kernel.cu:24-328).
  *
  *   activation    [M, K] act_dtype
- *   rot_kind      0 none, 1 regular Hadamard (rot_block a power of 4), 2 Sylvester (power of 2)
+ *   rot_kind      0 none, 1 regular Hadamard (rot_block a power of 4), 2 Sylvester (power of 2); with
+ *                 XQT_B200_ROT_FACTORS_READY added: column_scale was complete before this call was made (a synchronisation
+ *                 since it was written), so the kernel may read it while the one before it in the stream still runs
  *   column_scale  [rot_block] fp32 = signs / sqrt(rot_block) (NULL when rot_kind == 0)
  *   quant_bits    8: per-token scale max(amax,1e-8)/127, codes in [-128,127], scales [M]
  *                 4: per (token, group_size) scale max(amax/7,1e-6), codes in [-8,7], scales [M, K/group_size];
@@ -269,6 +271,7 @@ int xqt_b200_w4a16_decode_static_status(unsigned int* host_status, xqt_b200_stre
  *   codes         one byte per element [M, K] in every mode (int8 for 8 and 4);  rotated: [M, K] act_dtype or
  *                 NULL (the rotated, rounded activation, input of the W4A4 low-rank branch)
  */
+#define XQT_B200_ROT_FACTORS_READY 256
 int xqt_b200_rotate_quantize(const void* activation, const float* column_scale, void* codes,
                              float* scales, void* rotated, int m, int k, int rot_kind, int rot_block,
                              int quant_bits, int group_size, int act_dtype, xqt_b200_stream_t stream);
@@ -281,7 +284,8 @@ int xqt_b200_rotate_quantize(const void* activation, const float* column_scale, 
  *   la_form  1: fp32 [M, 32];  2: the operand images xqt_b200_w4a4_gemm takes with flag 2 (ceil(M/128) x 16 KiB);
  *            3: act_dtype [M, 64], columns 0..31 written (rounded once)
  * xqt_b200_act_prologue_supported: rotation none or of 16..256 features (regular: 16, 64, 256), K a multiple of 16 (64 for
- * mode 6), and for the int8 modes K at most about 20000. */
+ * mode 6), and for the int8 modes K at most 169984 (a cluster of eight CTAs holds a token).  rot_kind takes
+ * XQT_B200_ROT_FACTORS_READY too. */
 int xqt_b200_act_prologue_supported(int k, int rot_kind, int rot_block, int mode);
 int xqt_b200_act_prologue(const void* activation, const float* column_scale, void* codes, float* scales, const void* down,
                           void* la, float lora_scale, int m, int k, int rot_kind, int rot_block, int mode, int la_form,

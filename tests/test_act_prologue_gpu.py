@@ -38,13 +38,13 @@ def test_matches_the_separate_kernels(m, k, rotation, mode, dtype):
     want_la = 0.5 * rotated.float() @ down.float().t()
     # the MMA's fp32 sums of K exact products: the error of a sum of K terms in fp32 is below K * 2^-24 of the sum of magnitudes
     bound = 0.5 * k * 2.0 ** -24 * (rotated.float().abs() @ down.float().abs().t()) + 1e-30
-    for form in (0, 1, 2, 3):
+    for form, ready in ((0, 0), (1, 0), (2, 256), (3, 256), (0, 256)):       # column factors read after and before the wait
         codes = torch.full((m, k), 99, device=DEV, dtype=torch.int8)
         scales = torch.full_like(want_scales, -1.0)
         la = torch.zeros({0: (1,), 1: (m, 32), 2: (-(-m // 128) * 128, 32), 3: (m, 64)}[form], device=DEV, dtype=dtype if form == 3 else torch.float32)
         native.check(lib.xqt_b200_act_prologue(
             x.data_ptr(), native.ptr(column_scale), codes.data_ptr(), scales.data_ptr(), down.data_ptr() if form else 0, la.data_ptr() if form else 0,
-            0.5, m, k, kind, block, mode, form, native.DTYPE_CODE[dtype], native.stream_handle(DEV)), "xqt_b200_act_prologue")
+            0.5, m, k, kind | (ready if kind else 0), block, mode, form, native.DTYPE_CODE[dtype], native.stream_handle(DEV)), "xqt_b200_act_prologue")
         assert torch.equal(codes, want_codes)
         if mode == 6:                                      # tile-major: only the rows below M are written
             order = lambda s: s.reshape(-1, k // 64, 128).permute(0, 2, 1).reshape(-1, k // 64)[:m]

@@ -40,6 +40,7 @@ constexpr float kSeventh = 1.0f / 7.0f;
 struct ProloguePar {
   const void* x;
   const float* column_scale;   // [rot_block] or null
+  int factors_ready;           // the caller vouches that no earlier kernel is writing them: read before griddepcontrol.wait
   int8_t* codes;               // [M, K]
   float* scales;               // int8: [M]; int4: tile-major [ceil(M/128)][K/64][128]
   const void* down;            // [32, K] or null
@@ -405,6 +406,8 @@ __device__ __forceinline__ void apro_store_down(const ProloguePar& p, float* par
   }
 }
 
+// Read after the wait they cost every CTA a memory latency on its critical path (0.4 of 9.4 us at 77 tokens x 2048, 0.7 of 43.7
+// at 2048 x 4096; a prefetch into L2 or loads of x ahead of them do not hide it), read before it nothing.
 template <int ROT>
 __device__ __forceinline__ void apro_column_scale(const ProloguePar& p, float* cs) {
   if constexpr (ROT != 0)
@@ -430,10 +433,14 @@ act_prologue_i8_kernel(const ProloguePar p) {
   const int row0 = (int)(blockIdx.x / p.split) * p.rows;
   if (p.split > 1) cluster_arrive_relaxed();           // "this CTA runs"; waited for before the first remote store
   if (threadIdx.x < 17) s_top[threadIdx.x & 15] = s_nan[threadIdx.x] = 0;
-  apro_column_scale<ROT>(p, cs);
+  if (p.factors_ready) apro_column_scale<ROT>(p, cs);
   __syncthreads();
   grid_dependency_wait();
   grid_launch_dependents();
+  if (ROT != 0 && !p.factors_ready) {
+    apro_column_scale<ROT>(p, cs);
+    __syncthreads();
+  }
   int chunk = warp;
   for (int ur = 0; ur < p.rows; ur += kUnitRows, chunk -= own) {
     // consecutive units of the CTA go to consecutive warps, also where a token has fewer chunks than there are warps
@@ -516,10 +523,14 @@ act_prologue_i4_kernel(const ProloguePar p) {
   float* xpose = reinterpret_cast<float*>(tile + p.rows * stride);
   const int row0 = (int)(blockIdx.x / p.split) * p.rows, groups = p.k / 64;
   if (p.split > 1) cluster_arrive_relaxed();
-  apro_column_scale<ROT>(p, cs);
+  if (p.factors_ready) apro_column_scale<ROT>(p, cs);
   __syncthreads();
   grid_dependency_wait();
   grid_launch_dependents();
+  if (ROT != 0 && !p.factors_ready) {
+    apro_column_scale<ROT>(p, cs);
+    __syncthreads();
+  }
   float acc[4][4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
@@ -633,11 +644,14 @@ static int apro_dispatch(ProloguePar p, int rot_kind, int mode, cudaStream_t str
 
 int act_prologue_launch(const void* x, const float* column_scale, void* codes, float* scales, const void* down, void* la, float lora_scale,
                         int m, int k, int rot_kind, int rot_block, int mode, int la_form, int act_dtype, cudaStream_t stream) {
+  const int factors_ready = (rot_kind & XQT_B200_ROT_FACTORS_READY) != 0;
+  rot_kind &= ~XQT_B200_ROT_FACTORS_READY;
   XQT_REQUIRE(m > 0 && act_prologue_supported(k, rot_kind, rot_block, mode) && la_form >= 0 && la_form <= 3);
   XQT_REQUIRE(down == nullptr || k % 32 == 0);
   XQT_REQUIRE((down != nullptr) == (la_form != 0) && (down == nullptr || la != nullptr) && (rot_kind == 0 || column_scale != nullptr));
   XQT_REQUIRE(((uintptr_t)x & 15) == 0 && ((uintptr_t)codes & 15) == 0 && ((uintptr_t)down & 15) == 0 && ((uintptr_t)la & 15) == 0);
   ProloguePar p{};
+  p.factors_ready = factors_ready;
   p.x = x; p.column_scale = column_scale; p.codes = (int8_t*)codes; p.scales = scales; p.down = down; p.la = la;
   p.lora_scale = lora_scale; p.la_form = la_form; p.m = m; p.k = k; p.rot_block = rot_block;
   if (act_dtype == XQT_B200_BF16) return apro_dispatch<__nv_bfloat16>(p, rot_kind, mode, stream);

@@ -53,7 +53,8 @@ inline int sm_count() {
 }
 
 // Launch with programmatic stream serialisation: the kernel may start while the one before it in the stream drains.  It
-// has to execute griddepcontrol.wait (in every CTA) before it touches memory that an earlier kernel writes or reads.
+// has to execute griddepcontrol.wait (in every CTA) before it touches memory that an earlier kernel writes or reads, unless the
+// caller vouches that it was complete before the launch.
 template <typename... Params, typename... Args>
 inline int launch_pdl_cluster(void (*kern)(Params...), dim3 grid, dim3 block, int cluster, size_t smem, cudaStream_t stream, Args&&... args) {
   cudaLaunchConfig_t cfg = {};

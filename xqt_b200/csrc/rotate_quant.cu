@@ -332,10 +332,12 @@ int act_prologue_launch(const void* x, const float* column_scale, void* codes, f
 int rotate_quant_launch(const void* x, const float* column_scale, void* codes, float* scales, void* x_rot, int m, int k,
                         int rot_kind, int rot_block, int mode, int group, int act_dtype, cudaStream_t stream) {
   XQT_REQUIRE(m > 0 && k > 0 && (mode == 8 || mode == 9 || mode == 4 || mode == 5 || mode == 6));
+  const int factors_ready = rot_kind & XQT_B200_ROT_FACTORS_READY;
+  rot_kind &= ~XQT_B200_ROT_FACTORS_READY;
   // act_prologue.cu has the same codes and scales from fewer instructions where nobody wants the rotated activation
   if (x_rot == nullptr && (mode == 8 || mode == 9 || (mode == 6 && group == 64)) && act_prologue_supported(k, rot_kind, rot_block, mode) &&
       (rot_kind == 0 || column_scale != nullptr) && ((uintptr_t)x & 15) == 0 && ((uintptr_t)codes & 15) == 0)
-    return act_prologue_launch(x, column_scale, codes, scales, nullptr, nullptr, 1.f, m, k, rot_kind, rot_block, mode, 0, act_dtype, stream);
+    return act_prologue_launch(x, column_scale, codes, scales, nullptr, nullptr, 1.f, m, k, rot_kind | factors_ready, rot_block, mode, 0, act_dtype, stream);
   // modes 5, 6: the int4 codes of mode 4 written as sign-magnitude bytes; mode 6 also orders the scales tile-major;
   // mode 9: mode 8 with the scale rounded to the activation dtype
   const int signmag = mode == 5 ? 1 : (mode == 6 ? 3 : (mode == 9 ? 4 : 0));

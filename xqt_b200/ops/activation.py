@@ -9,19 +9,32 @@ from ..errors import XQTBackendError
 from ..quantize import Rotation
 
 _KIND = {None: 0, "regular": 1, "sylvester": 2}
-_scale_cache: dict[tuple, torch.Tensor] = {}
+_FACTORS_READY = 256                 # XQT_B200_ROT_FACTORS_READY
+_scale_cache: dict[tuple, tuple] = {}
 
 
 def _column_scale(rotation: Rotation, device: torch.device) -> torch.Tensor:
     """The rotation's column factors on ``device``, cached per Rotation object (the entry keeps the object alive, so
     its id cannot be reused; building a key from the sign vector on every call cost more host time than the launch)."""
 
+    return _factors(rotation, device)[0]
+
+
+def _factors(rotation: Rotation | None, device: torch.device) -> tuple[torch.Tensor | None, int, int]:
+    """Column factors, and the kind (with the flag that says that the factors are complete) and block size the library takes."""
+
+    if rotation is None:
+        return None, 0, 0
     key = (id(rotation), device.type, device.index)
     cached = _scale_cache.get(key)
     if cached is None or cached[0] is not rotation:
-        cached = (rotation, rotation.column_scale.to(device).contiguous())
+        scale, kind = rotation.column_scale.to(device).contiguous(), _KIND[rotation.kind]
+        if scale.is_cuda and not torch.cuda.is_current_stream_capturing():
+            torch.cuda.current_stream(device).synchronize()       # once per rotation: the kernels may read them early, on any stream
+            kind |= _FACTORS_READY
+        cached = (rotation, scale, kind)
         _scale_cache[key] = cached
-    return cached[1]
+    return cached[1], cached[2], rotation.block
 
 
 def rotate_quantize(x: torch.Tensor, rotation: Rotation | None, *, bits: int, group_size: int = 64,
@@ -75,11 +88,11 @@ def rotate_quantize(x: torch.Tensor, rotation: Rotation | None, *, bits: int, gr
                 or (rotated is not None and (rotated.dtype != x.dtype or tuple(rotated.shape) != (m, k) or not rotated.is_contiguous())):
             raise XQTBackendError("rotate_quantize: workspace buffers do not match the activation")
     if m:
-        cs = None if rotation is None else _column_scale(rotation, device)
+        cs, kind, block = _factors(rotation, device)
         with torch.cuda.device(device):
             code = native.library().xqt_b200_rotate_quantize(
                 x.data_ptr(), native.ptr(cs), codes.data_ptr(), scales.data_ptr(), native.ptr(rotated), m, k,
-                _KIND[None if rotation is None else rotation.kind], 0 if rotation is None else rotation.block,
+                kind, block,
                 (6 if tiled_scales else 5) if sign_magnitude else (9 if scale_in_act_dtype else bits), int(group_size), native.DTYPE_CODE[x.dtype], native.stream_handle(device))
         native.check(code, "xqt_b200_rotate_quantize")
     return (codes, scales, rotated) if return_rotated else (codes, scales)

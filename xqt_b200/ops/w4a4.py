@@ -29,7 +29,7 @@ from .. import native
 from ..errors import XQTBackendError
 from ..hostcall import INPUT, OUTPUT, WORKSPACE, bound_call, float_bits, step
 from ..quantize import Rotation, quantize_residual_int4
-from .activation import _KIND, _column_scale, rotate_quantize
+from .activation import _KIND, _factors, rotate_quantize
 
 GROUP = 64
 RANK_PAD = 32
@@ -277,7 +277,7 @@ def svdq_w4a4_linear(inputs: torch.Tensor, packed: PackedSVDQW4A4Linear, *, work
         scratch = native.workspace(device, lib.xqt_b200_w4a4_dense_workspace_bytes(m, n, k) if dense else
                                    lib.xqt_b200_w4a4_workspace_bytes(m, n, k), "gemm")
         if fused:
-            column_scale = None if rot is None else _column_scale(rot, device)
+            column_scale, kind, block = _factors(rot, device)
             native.check(lib.xqt_b200_act_prologue(x.data_ptr(), native.ptr(column_scale), codes.data_ptr(), scales.data_ptr(), packed.down.data_ptr(),
                                                    la.data_ptr(), 1.0, m, k, kind, block, 6, 2, native.DTYPE_CODE[packed.dtype], stream),
                          "xqt_b200_act_prologue")
@@ -367,10 +367,9 @@ def bind_svdq_w4a4_linear(packed: PackedSVDQW4A4Linear, workspace: W4A4Workspace
     la = workspace.lora_activation if packed.rank else None
     if la is None:
         la = torch.zeros((-(-rows // TILE) * TILE, RANK_PAD), device=device, dtype=torch.float32)
-    column_scale = None if rot is None else _column_scale(rot, device)
+    column_scale, kind, block = _factors(rot, device)
     codes, scales, rotated = workspace.quantized_activation, workspace.activation_scales, workspace.rotated_activation
-    kind, block = _KIND[None if rot is None else rot.kind], 0 if rot is None else rot.block
-    if packed.act_granularity == "group" and lib.xqt_b200_act_prologue_supported(k, kind, block, 6):
+    if packed.act_granularity == "group" and lib.xqt_b200_act_prologue_supported(k, _KIND[None if rot is None else rot.kind], block, 6):
         steps = [step("xqt_b200_act_prologue", ((INPUT, 0), column_scale, codes, scales, packed.down if packed.rank else 0,
                                                 la if packed.rank else 0),
                       (float_bits(1.0), rows, k, kind, block, 6, 2 if packed.rank else 0, dcode))]

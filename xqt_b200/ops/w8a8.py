@@ -297,16 +297,15 @@ def bind_convrot_w8a8_linear(packed: PackedConvRotW8A8Linear, workspace: ConvRot
         raise XQTBackendError("the rotated dimension must be a multiple of the rotation block")
     # every pointer and code of the two library calls is resolved here; a call checks its input, allocates its output
     # and makes the two calls (the general entry's per-call validation costs about as much host time as the kernels run)
-    from .activation import _KIND, _column_scale
+    from .activation import _factors
 
     lib = native.library()
     codes, scales = workspace.quantized_activation[:rows], workspace.activation_scales[:rows]
-    column_scale = None if rot is None else _column_scale(rot, device)
+    column_scale, kind, block = _factors(rot, device)
     index = device.index if device.index is not None else torch.cuda.current_device()
     native.workspace(device, 256, "gemm")            # the current stream's status word, made now
     dcode = native.DTYPE_CODE[dtype]
-    prologue = (native.ptr(column_scale), codes.data_ptr(), scales.data_ptr(), 0, rows, k, _KIND[None if rot is None else rot.kind],
-                0 if rot is None else rot.block, 8, 0, dcode)
+    prologue = (native.ptr(column_scale), codes.data_ptr(), scales.data_ptr(), 0, rows, k, kind, block, 8, 0, dcode)
     gemm_head = (codes.data_ptr(), packed.qweight.data_ptr(), scales.data_ptr(), packed.weight_scales.data_ptr(), native.ptr(packed.bias))
     gemm_tail = (rows, n, k, dcode)
 
