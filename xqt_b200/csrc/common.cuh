@@ -81,6 +81,30 @@ inline int launch_pdl(void (*kern)(Params...), dim3 grid, dim3 block, size_t sme
   return launch_pdl_cluster(kern, grid, block, 1, smem, stream, args...);
 }
 
+// Clusters of two CTAs of `Kern` that are resident together with a CTA per SM, asked for once per kernel and device.
+template <auto Kern>
+inline int resident_pairs(int threads, size_t smem) {
+  static int cached[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return sm_count() / 2;
+  if (cached[dev] == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(sm_count() & ~1));
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int v = 0;
+    if (cudaOccupancyMaxActiveClusters(&v, Kern, &cfg) != cudaSuccess || v <= 0) v = sm_count() / 2;
+    cached[dev] = v < sm_count() / 2 ? v : sm_count() / 2;
+  }
+  return cached[dev];
+}
+
 __host__ __device__ constexpr int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
 template <typename T>

@@ -348,30 +348,6 @@ struct ScaledPlan {
   int cg, tile_n, split;
 };
 
-// Clusters of two CTAs that are resident together with a CTA per SM (asked for once per device).
-template <typename Kern>
-int resident_pairs(Kern kern, size_t smem) {
-  static int cached[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return sm_count() / 2;
-  if (cached[dev] == 0) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(sm_count() & ~1));
-    cfg.blockDim = dim3(gs::kThreads);
-    cfg.dynamicSmemBytes = smem;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int v = 0;
-    if (cudaOccupancyMaxActiveClusters(&v, kern, &cfg) != cudaSuccess || v <= 0) v = sm_count() / 2;
-    cached[dev] = v < sm_count() / 2 ? v : sm_count() / 2;
-  }
-  return cached[dev];
-}
-
 // Estimated SM clocks of a form; the constants were fitted to sweeps of tile_n and split on a B200.
 ScaledPlan scaled_plan(int m, int n, int k, bool low) {
   const int sms = sm_count(), kblocks = ceil_div(k, gs::kRowBytes), widest = low ? 160 : 256;
@@ -420,12 +396,12 @@ int launch_scaled(const void* a, const void* b, const void* low_a, const void* l
   int stages = (kSmemBudget - 1024 - reduce) / stage_bytes;
   p.stages = stages > kMaxStages ? kMaxStages : stages;
   const size_t smem = (size_t)p.stages * stage_bytes + reduce + 1024;
-  auto kern = gemm_scaled_kernel<CG, T, LOW, QUADS>;
+  constexpr auto kern = gemm_scaled_kernel<CG, T, LOW, QUADS>;
   XQT_SMEM_OPT_IN(kern, kSmemBudget);
   const int tiles = p.mtiles * p.ntiles;
   int grid, cluster;
   if (CG == 2) {
-    const int pairs = resident_pairs(kern, kSmemBudget);
+    const int pairs = resident_pairs<kern>(kThreads, kSmemBudget);
     grid = 2 * (tiles < pairs ? tiles : pairs);
     cluster = 2;
   } else if (p.split > 1) {

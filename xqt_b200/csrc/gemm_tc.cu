@@ -150,7 +150,7 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
           if (sn == ns) { sn = 0; pn ^= 1; }
           // four 32-byte K steps, the commit that frees the stage, and the poll of the next stage's
           // barrier in one go: the poll's round trip is hidden behind the MMA issue
-          ready = umma_ss_x4_commit_poll<false>(d_tmem, adesc, bdesc, kIdesc, kb != 0 ? 1u : 0u, empty_bar(s), full_bar(sn), pn);
+          ready = umma_ss_x4_commit_poll(d_tmem, adesc, bdesc, kIdesc, kb != 0 ? 1u : 0u, empty_bar(s), full_bar(sn), pn);
           if (last_tile && kb == p.kblocks - 1) ready = false;
           s = sn;
           phase = pn;

@@ -204,7 +204,7 @@ gemm_w4a16_fused_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_c
           const uint32_t a_addr = smem_addr(tiles + (size_t)s * kStageBytes);
           const uint64_t adesc = umma_desc_sw128(a_addr), bdesc = umma_desc_sw128(a_addr + kABytes);
 #pragma unroll
-          for (int q = 0; q < 4; ++q) umma_ss<false>(tmem_base + buf * kTileCols, adesc + 2 * q, bdesc + 2 * q, kIdesc, (kb != 0 || q != 0) ? 1u : 0u);
+          for (int q = 0; q < 4; ++q) umma_ss(tmem_base + buf * kTileCols, adesc + 2 * q, bdesc + 2 * q, kIdesc, (kb != 0 || q != 0) ? 1u : 0u);
           umma_commit(bar(kBarEmpty + s));
           // the next stage's barriers, tested without blocking after this stage's MMAs are on their way
           ready = mbar_test_wait(bar(kBarReady + nxt.slot), nxt.phase) && mbar_test_wait(bar(kBarFull + nxt.slot), nxt.phase);

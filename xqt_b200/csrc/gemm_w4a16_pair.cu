@@ -484,29 +484,6 @@ PairPlan pair_plan(int m, int n, int k, int max_splits = 8) {
   return best;
 }
 
-template <typename Kern>
-int resident_pairs(Kern kern, size_t smem) {
-  static int cached[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return sm_count() / 2;
-  if (cached[dev] == 0) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(sm_count() & ~1));
-    cfg.blockDim = dim3(w4p::kThreads);
-    cfg.dynamicSmemBytes = smem;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int v = 0;
-    if (cudaOccupancyMaxActiveClusters(&v, kern, &cfg) != cudaSuccess || v <= 0) v = sm_count() / 2;
-    cached[dev] = v < sm_count() / 2 ? v : sm_count() / 2;
-  }
-  return cached[dev];
-}
-
 template <int MB, typename T, bool GLU>
 int launch_pair(const void* x, const void* qw, W4PairParams p, int k, cudaStream_t stream) {
   using namespace w4p;
@@ -518,9 +495,9 @@ int launch_pair(const void* x, const void* qw, W4PairParams p, int k, cudaStream
   p.raw_bufs = ring.raws;
   const int stage_bytes = MB * kABlockBytes + p.tile_n / 2 * 128, raw_bytes = p.tile_n / 2 * (kBK / 2);
   const size_t smem_bytes = (size_t)p.stages * stage_bytes + (size_t)p.raw_bufs * raw_bytes + 1024;
-  auto kern = gemm_w4a16_pair_kernel<MB, T, GLU>;
+  constexpr auto kern = gemm_w4a16_pair_kernel<MB, T, GLU>;
   XQT_SMEM_OPT_IN(kern, kSmemBudget);
-  const int tiles = p.mchunks * p.ntiles * p.splits, pairs = resident_pairs(kern, kSmemBudget);
+  const int tiles = p.mchunks * p.ntiles * p.splits, pairs = resident_pairs<kern>(kThreads, kSmemBudget);
   const int rc = launch_pdl_cluster(kern, dim3((unsigned)(2 * (tiles < pairs ? tiles : pairs))), dim3(kThreads), 2, smem_bytes, stream, tm_a, tm_w, p);
   if (rc != 0 || p.splits == 1) return rc;
   const size_t threads = (size_t)p.m * (p.n / 8);

@@ -396,12 +396,12 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
           tc_fence_after();
           const uint64_t ladesc = umma_desc_sw128(smem_addr(la_base)), updesc = umma_desc_sw128(smem_addr(up_base));
           const uint32_t d_tmem = tmem_base + pb * (2 * kBN);
-          umma_ss<false>(d_tmem, ladesc + 0, updesc + 0, kIdescLora, 0u);     // hi x hi
-          umma_ss<false>(d_tmem, ladesc + 2, updesc + 2, kIdescLora, 1u);
-          umma_ss<false>(d_tmem, ladesc + 4, updesc + 0, kIdescLora, 1u);     // lo x hi
-          umma_ss<false>(d_tmem, ladesc + 6, updesc + 2, kIdescLora, 1u);
-          umma_ss<false>(d_tmem, ladesc + 0, updesc + 4, kIdescLora, 1u);     // hi x lo
-          umma_ss<false>(d_tmem, ladesc + 2, updesc + 6, kIdescLora, 1u);
+          umma_ss(d_tmem, ladesc + 0, updesc + 0, kIdescLora, 0u);     // hi x hi
+          umma_ss(d_tmem, ladesc + 2, updesc + 2, kIdescLora, 1u);
+          umma_ss(d_tmem, ladesc + 4, updesc + 0, kIdescLora, 1u);     // lo x hi
+          umma_ss(d_tmem, ladesc + 6, updesc + 2, kIdescLora, 1u);
+          umma_ss(d_tmem, ladesc + 0, updesc + 4, kIdescLora, 1u);     // hi x lo
+          umma_ss(d_tmem, ladesc + 2, updesc + 6, kIdescLora, 1u);
           umma_commit(bar(kBarPairFull + pb));
           umma_commit(bar(kBarEpiEmpty));                                      // the two images may be overwritten
           ++pair;

@@ -278,22 +278,13 @@ __host__ __device__ constexpr uint32_t umma_idesc(uint32_t acc_fmt, uint32_t a_f
   return (acc_fmt << 4) | (a_fmt << 7) | (b_fmt << 10) | ((n >> 3) << 17) | ((m >> 4) << 24);
 }
 
-// D[tmem] (+)= A[smem] * B[smem]; issued by ONE thread
-template <bool I8>
+// D[tmem] (+)= A[smem] * B[smem], 16-bit operands; issued by ONE thread
 __device__ __forceinline__ void umma_ss(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  if (I8) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-  } else {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-  }
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
 }
 // D[tmem] (+)= A[smem] * B[smem] with 8-bit floating operands (kind::f8f6f4; formats in the descriptor:
 // E4M3 = 0, E5M2 = 1), fp32 accumulators; issued by ONE thread
@@ -334,48 +325,27 @@ __device__ __forceinline__ unsigned long long f32x2_add(unsigned long long a, un
 // issued first, consumed last -- one poll of `next_bar` (a non-blocking test_wait: try_wait would suspend the issuer
 // when the next stage has not landed yet): the 150-cycle round trip of the poll runs while the MMAs are being issued.  Returns whether `next_bar` had completed `next_parity`.
 // `first_accumulate` is the accumulate flag of the first step; the other three always accumulate.
-template <bool I8>
 __device__ __forceinline__ bool umma_ss_x4_commit_poll(uint32_t d_tmem, uint64_t a0, uint64_t b0, uint32_t idesc,
                                                         uint32_t first_accumulate, uint32_t done_bar, uint32_t next_bar,
                                                         uint32_t next_parity) {
   uint32_t ok;
-  if (I8) {
-    asm volatile(
-        "{\n\t.reg .pred p, q, t;\n\t.reg .b64 a, b;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 q, [%6], %7;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "setp.eq.b32 t, 0, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%1], %2, %3, %8, p;\n\t"
-        "add.u64 a, %2, 2;\n\tadd.u64 b, %3, 2;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%1], a, b, %8, t;\n\t"
-        "add.u64 a, %2, 4;\n\tadd.u64 b, %3, 4;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%1], a, b, %8, t;\n\t"
-        "add.u64 a, %2, 6;\n\tadd.u64 b, %3, 6;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%1], a, b, %8, t;\n\t"
-        "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%5];\n\t"
-        "selp.u32 %0, 1, 0, q;\n\t}\n"
-        : "=r"(ok)
-        : "r"(d_tmem), "l"(a0), "l"(b0), "r"(first_accumulate), "r"(done_bar), "r"(next_bar), "r"(next_parity), "r"(idesc)
-        : "memory");
-  } else {
-    asm volatile(
-        "{\n\t.reg .pred p, q, t;\n\t.reg .b64 a, b;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 q, [%6], %7;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "setp.eq.b32 t, 0, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%1], %2, %3, %8, p;\n\t"
-        "add.u64 a, %2, 2;\n\tadd.u64 b, %3, 2;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%1], a, b, %8, t;\n\t"
-        "add.u64 a, %2, 4;\n\tadd.u64 b, %3, 4;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%1], a, b, %8, t;\n\t"
-        "add.u64 a, %2, 6;\n\tadd.u64 b, %3, 6;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%1], a, b, %8, t;\n\t"
-        "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%5];\n\t"
-        "selp.u32 %0, 1, 0, q;\n\t}\n"
-        : "=r"(ok)
-        : "r"(d_tmem), "l"(a0), "l"(b0), "r"(first_accumulate), "r"(done_bar), "r"(next_bar), "r"(next_parity), "r"(idesc)
-        : "memory");
-  }
+  asm volatile(
+      "{\n\t.reg .pred p, q, t;\n\t.reg .b64 a, b;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 q, [%6], %7;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.eq.b32 t, 0, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%1], %2, %3, %8, p;\n\t"
+      "add.u64 a, %2, 2;\n\tadd.u64 b, %3, 2;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%1], a, b, %8, t;\n\t"
+      "add.u64 a, %2, 4;\n\tadd.u64 b, %3, 4;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%1], a, b, %8, t;\n\t"
+      "add.u64 a, %2, 6;\n\tadd.u64 b, %3, 6;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%1], a, b, %8, t;\n\t"
+      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%5];\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}\n"
+      : "=r"(ok)
+      : "r"(d_tmem), "l"(a0), "l"(b0), "r"(first_accumulate), "r"(done_bar), "r"(next_bar), "r"(next_parity), "r"(idesc)
+      : "memory");
   return ok != 0;
 }
 // D[tmem] (+)= A[tmem] * B[smem]
@@ -429,7 +399,7 @@ __device__ __forceinline__ void umma_commit_cg(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n" ::"r"(bar), "h"((uint16_t)3)
                  : "memory");
 }
-enum : int { kMmaI8 = 0, kMmaF16 = 1, kMmaF8 = 2 };
+enum : int { kMmaI8 = 0, kMmaF16 = 1 };
 template <int CG, int KIND>
 __device__ __forceinline__ void umma_ss_cg(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
 #define XQT_UMMA(GROUP, NAME)                                                                                   \
@@ -439,10 +409,8 @@ __device__ __forceinline__ void umma_ss_cg(uint32_t d_tmem, uint64_t adesc, uint
                : "memory")
   if constexpr (CG == 1 && KIND == kMmaI8) XQT_UMMA("1", "i8");
   if constexpr (CG == 1 && KIND == kMmaF16) XQT_UMMA("1", "f16");
-  if constexpr (CG == 1 && KIND == kMmaF8) XQT_UMMA("1", "f8f6f4");
   if constexpr (CG == 2 && KIND == kMmaI8) XQT_UMMA("2", "i8");
   if constexpr (CG == 2 && KIND == kMmaF16) XQT_UMMA("2", "f16");
-  if constexpr (CG == 2 && KIND == kMmaF8) XQT_UMMA("2", "f8f6f4");
 #undef XQT_UMMA
 }
 // arrive on a barrier of another CTA of the cluster (address from cluster_map)
