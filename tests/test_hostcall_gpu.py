@@ -154,6 +154,11 @@ def test_one_bound_layer_serves_every_row_count():
             assert torch.equal(got, want) if layer is module or m <= 128 else (got - want).norm() <= 4e-3 * want.norm()
     assert len(module._gemm) == 1 and len(blocks[0]._decode) == 2
     kept = {id(module._gemm[torch.bfloat16][2]), *(id(run) for block in blocks for run in (*block._decode.values(), block._gemm[1]))}
+    first = W4A16SwiGLUMLP(_layer(640, k, 32), _layer(640, k, 33), _layer(k, 640, 34), device=DEV)
+    for m in (300, 64, 300, 33, 400):                              # the single library call first, then the separate launches
+        assert torch.equal(first(x[:m]), blocks[0](x[:m]))
+    with pytest.raises(XQTBackendError):
+        first(x[:300, :128])
     baseline = None
     for m in range(17, 700, 3):
         module(x[:m]), blocks[0](x[:m])
@@ -181,6 +186,17 @@ def test_weights_first_seen_inside_a_graph_capture():
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(one, want) and torch.equal(two, want)
+    # and the small layer that never asks: above 512 rows two passes whatever its zero points are
+    small = AWQW4A16Linear(_layer(256, k, 42)).eval()
+    stream.wait_stream(torch.cuda.current_stream(DEV))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        one = small(x)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert small._gemm[torch.bfloat16][3] is None and torch.equal(small(x), one)
+    want_small = w4a16_linear(x[:300], small.canonical_qweight, small.weight_scale, small.weight_zero_point, group_size=128, nibble_signed=False)
+    assert torch.equal(small(x[:300]), want_small) and small._gemm[torch.bfloat16][3] is True
     assert torch.equal(module(x), w4a16_linear(x, w.qweight, w.scales, w.zero_points, group_size=128, nibble_signed=False, variant="tcgen05_fused"))
 
 

@@ -26,7 +26,7 @@ from .errors import XQTBackendError
 from .hostcall import INPUT, MANY_ROWS, OUTPUT, bound_layer, plan, weak_method
 from .layout import signed_storage_to_unsigned
 from .ops import awq as awq_ops
-from .ops.w4a16 import integer_zero_points_now, version_of, w4a16_linear, w4a16_step, with_version
+from .ops.w4a16 import fused_preferred, integer_zero_points_now, version_of, w4a16_linear, w4a16_step, with_version
 
 _DTYPE_NAME = {torch.float16: "fp16", torch.bfloat16: "bf16"}
 MAX_DECODE_ROWS = 16
@@ -61,7 +61,8 @@ class AWQW4A16Linear(nn.Module):
         self._prepared: dict[torch.dtype, tuple] = {}
         self._bound: dict[tuple[int, torch.dtype], Callable] = {}
         self._residual_bound: dict[tuple[int, torch.dtype], Callable] = {}
-        # dtype -> (tensors it was built from, their versions and addresses, bound call): above the decode sizes, any row count
+        # dtype -> (tensors it was built from, their versions and addresses, bound call, "zero points are integers"): above the
+        # decode sizes, any row count
         self._gemm: dict[torch.dtype, tuple] = {}
         self._native_only = False
         self._native_only_rows: frozenset[int] = frozenset()
@@ -234,9 +235,10 @@ class AWQW4A16Linear(nn.Module):
         last = state.get("_last_execution")
         super().__setstate__({**state, "_gemm": {}, "_last_execution": last if isinstance(last, tuple) else None})
 
-    def _gemm_call(self, dtype: torch.dtype) -> Callable | None:
+    def _gemm_call(self, dtype: torch.dtype, rows: int) -> Callable | None:
         """The bound call for more than 16 rows, made when there is none or a buffer has changed since; None where
-        ``w4a16_linear`` has to look at the buffers itself."""
+        ``w4a16_linear`` has to look at the buffers itself.  Whether the zero points are integers, a copy from the device, is
+        asked when the first row count comes for which it matters; until then (and in a graph capture) it is left open."""
 
         buffers = self._buffers
         canonical, scales, zeros, bias = static = (buffers["canonical_qweight"], buffers["weight_scale"], buffers["weight_zero_point"], buffers["bias"])
@@ -244,12 +246,13 @@ class AWQW4A16Linear(nn.Module):
         own = (zeros, None if bias is None or bias.dtype == torch.float32 else bias)
         state = tuple(version_of(t) for t in own) + tuple(None if t is None else t.data_ptr() for t in static)
         hit = self._gemm.get(dtype)
+        n, k, group = self.output_features, self.input_features, self.group_size
         if hit is not None and hit[1] == state and all(a is b for a, b in zip(hit[0], static)):
-            return hit[2]
+            if hit[3] is not None or not fused_preferred(rows, n, k, int(canonical.shape[1]) * 2, group) or integer_zero_points_now(zeros) is None:
+                return hit[2]
         if self._native_only or canonical is None or not canonical.is_cuda or dtype not in _DTYPE_NAME:
             return None
-        n, k, group, device = self.output_features, self.input_features, self.group_size, canonical.device
-        padded_k = int(canonical.shape[-1]) * 2
+        device, padded_k = canonical.device, int(canonical.shape[-1]) * 2
         # whatever w4a16_linear converts or refuses is left to it, and what changes unseen
         if any(t is not None and t.is_inference() for t in own) or any(t is not None and (t.device != device or not t.is_contiguous()) for t in static) \
                 or canonical.dtype != torch.uint8 or canonical.ndim != 2 or canonical.shape[0] != n \
@@ -257,14 +260,12 @@ class AWQW4A16Linear(nn.Module):
                 or (zeros is not None and (zeros.dtype != scales.dtype or zeros.shape != scales.shape)) \
                 or (bias is not None and bias.numel() != n):
             return None
-        integer = integer_zero_points_now(zeros)
-        if integer is None:
-            return None
+        integer = integer_zero_points_now(zeros) if fused_preferred(rows, n, k, padded_k, group) else None
         bias32 = None if bias is None else bias.reshape(-1).to(torch.float32).contiguous()     # a cast of the module casts the buffer
         gemm = w4a16_step((INPUT, 0), canonical, scales, zeros, bias32, (OUTPUT, 0), k=k, group_size=group, nibble_signed=False, dtype=dtype, integer=integer)
         run = bound_layer([plan([gemm], rows=(MAX_DECODE_ROWS + 1, MANY_ROWS))], weak_method(self._forward_flat), dtype=dtype, device=device,
                           rows=None, k=k, n=n, workspace="run", keep=(static, bias32), symbols="xqt_b200_w4a16_run")
-        self._gemm[dtype] = (static, state, run)
+        self._gemm[dtype] = (static, state, run, integer)
         return run
 
     def forward(self, inputs: torch.Tensor) -> torch.Tensor:
@@ -272,7 +273,7 @@ class AWQW4A16Linear(nn.Module):
             raise RuntimeError("AWQ W4A16 native path requires eval mode")
         if inputs.ndim == 2 and inputs.shape[1] == self.input_features and inputs.dtype in _DTYPE_NAME:
             rows, dtype = inputs.shape[0], inputs.dtype
-            run = self._gemm_call(dtype) if rows > MAX_DECODE_ROWS else (self.bind(rows=rows, dtype=dtype) if rows else None)
+            run = self._gemm_call(dtype, rows) if rows > MAX_DECODE_ROWS else (self.bind(rows=rows, dtype=dtype) if rows else None)
             if run is not None:
                 output = run(inputs)
                 self._last_execution = ("w4a16_decode_cl_kernel" if rows <= MAX_DECODE_ROWS else "w4a16 tcgen05 GEMM", rows, dtype)

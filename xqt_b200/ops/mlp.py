@@ -23,7 +23,7 @@ from ..contracts import PackedWeight, PackedWeightMetadata
 from ..errors import XQTBackendError
 from ..hostcall import INPUT, MANY_ROWS, OUTPUT, ROWS, SCRATCH, WORKSPACE, bound_layer, guard, plan, step, weak_method
 from ..parallel import shard_packed_weight
-from .w4a16 import (_integer_zero_points, bind_w4a16_decode, glu_row_order, integer_zero_points_now, prepare_decode, version_of, w4a16_linear,
+from .w4a16 import (_integer_zero_points, bind_w4a16_decode, fused_preferred, glu_row_order, integer_zero_points_now, prepare_decode, version_of, w4a16_linear,
                     w4a16_step, with_version)
 
 
@@ -156,11 +156,14 @@ class _Linear:
                      0, 0, (target[0], target[1] + 2 * first * width), status),
                     (rows, self.n, self.k, self.group, self.tiled.nibble_signed, code, native.DTYPE_CODE[params.dtype], code, 2 if glu else 0))
 
-    def gemm_step(self, source: tuple, target: tuple) -> tuple:
+    def fused_preferred(self, m: int) -> bool:
+        return fused_preferred(m, self.n, self.k, int(self.qweight.shape[1]) * 2, self.group)
+
+    def gemm_step(self, source: tuple, target: tuple, integer: bool | None) -> tuple:
         """The canonical-weight GEMM of any number of rows as a step of a bound layer."""
 
         return w4a16_step(source, self.qweight, self.scales, self.zeros, None, target, k=self.k, group_size=self.group,
-                          nibble_signed=self.signed, dtype=self.dtype, integer=_integer_zero_points(self.zeros))
+                          nibble_signed=self.signed, dtype=self.dtype, integer=integer)
 
     def partial_into(self, x: torch.Tensor, peer) -> None:
         """Decode-size fp32 partial sums of a K-sharded layer, written into the slot of ``peer`` (a counted
@@ -254,13 +257,19 @@ class W4A16SwiGLUMLP:
                 if run is None:
                     run = self._decode[(m + 15) // 16] = self._bind_decode((m + 15) // 16)
                 return run(x)
-            run = self._gemm_call()
+            run = self._gemm_call(m)
             if run is not None:
                 return run(x)
         return self._forward(x)
 
-    def _bound(self, plans: list, keep: tuple = ()):
-        return bound_layer(plans, weak_method(self._forward), dtype=self.dtype, device=self.gate_up.qweight.device, rows=None, k=self.gate_up.k,
+    def _separate(self, x: torch.Tensor, *rest) -> torch.Tensor:
+        """A call that the single library call's bound layer does not take."""
+
+        run = self._gemm_call(x.shape[0], every=True) if not rest and x.ndim == 2 and x.shape[0] > CHUNKED_DECODE_MAX_ROWS else None
+        return self._forward(x, *rest) if run is None else run(x)
+
+    def _bound(self, plans: list, keep: tuple = (), slow=None):
+        return bound_layer(plans, weak_method(slow or self._forward), dtype=self.dtype, device=self.gate_up.qweight.device, rows=None, k=self.gate_up.k,
                            n=self.hidden, workspace="run", keep=(self.gate_up, self.down, *keep), symbols="bound W4A16 SwiGLU MLP")
 
     def _bind_decode(self, chunks: int):
@@ -278,31 +287,40 @@ class W4A16SwiGLUMLP:
                        for layer in (gate_up, down) for rows in {rows for _, rows in parts})
         return self._bound([plan(steps, rows=(last + 1, last + 16), guards=served, scratch=(0, 2 * self.inter_local))], (native.status_word(device),))
 
-    def _gemm_call(self):
+    def _gemm_call(self, m: int, every: bool = False):
         """The launches of :meth:`_forward` above the decode sizes as one bound layer, made when there is none or a tensor has changed
-        since; None where ``w4a16_linear`` has to look at the tensors itself."""
+        since; None where ``w4a16_linear`` has to look at the tensors itself.  Whether the zero points are integers is asked when
+        the first row count comes for which it matters; until then (and in a graph capture) it is left open.  A block whose first
+        row count is one for the single library call has the separate launches bound when a row count needs them (``every``)."""
 
         gu, dn = self.gate_up, self.down
         static = (gu.qweight, gu.scales, gu.zeros, dn.qweight, dn.scales, dn.zeros)
         state = (version_of(gu.zeros), version_of(dn.zeros), *(None if t is None else t.data_ptr() for t in static))
-        if self._gemm is not None and self._gemm[0] == state:
+
+        def integers() -> list | None:
+            answers = [integer_zero_points_now(layer.zeros) for layer in (gu, dn)] if gu.fused_preferred(m) or dn.fused_preferred(m) else [None]
+            return None if None in answers else answers
+
+        if self._gemm is not None and self._gemm[0] == state and not every and (self._gemm[2] or integers() is None):
             return self._gemm[1]
         if gu.qweight.device.type != "cuda" or not (gu.canonical_served and dn.canonical_served) \
-                or any(t is not None and t.is_inference() for t in (gu.zeros, dn.zeros)) \
-                or integer_zero_points_now(gu.zeros) is None or integer_zero_points_now(dn.zeros) is None:
+                or any(t is not None and t.is_inference() for t in (gu.zeros, dn.zeros)):
             return None
-        plans, inter = [], self.inter_local
-        if self._fuse_gating and self._one_entry_form():
+        plans, inter, known = [], self.inter_local, integers()
+        if known and self._fuse_gating and self._one_entry_form():
             code = native.DTYPE_CODE
             entry = step("xqt_b200_w4a16_swiglu_mlp", ((INPUT, 0), gu.qweight, gu.scales, gu.zeros, dn.qweight, dn.scales, dn.zeros, (OUTPUT, 0)),
                          (ROWS, self.hidden, inter, gu.group, dn.group, gu.signed, dn.signed, code[self.dtype], code[gu.scales.dtype], code[dn.scales.dtype]),
                          (WORKSPACE, 0), ("xqt_b200_w4a16_swiglu_mlp_workspace_bytes", self.hidden, inter))
             plans.append(plan([entry], rows=(CHUNKED_DECODE_MAX_ROWS + 1, MANY_ROWS),
                               guards=(guard("xqt_b200_w4a16_swiglu_mlp_supported", ROWS, self.hidden, inter, gu.group, dn.group),)))
+            if not every and native.library().xqt_b200_w4a16_swiglu_mlp_supported(m, self.hidden, inter, gu.group, dn.group):
+                self._gemm = (state, self._bound(plans, static, slow=self._separate), True)
+                return self._gemm[1]
         both, h = (SCRATCH, 0), (SCRATCH, 0, 4 * inter)          # [rows, 2 * inter], then [rows, inter]
-        plans.append(plan([gu.gemm_step((INPUT, 0), both), step("xqt_b200_swiglu", (both, h), (ROWS, inter, native.DTYPE_CODE[self.dtype])),
-                           dn.gemm_step(h, (OUTPUT, 0))], rows=(CHUNKED_DECODE_MAX_ROWS + 1, MANY_ROWS), scratch=(0, 6 * inter)))
-        self._gemm = (state, self._bound(plans, static))
+        plans.append(plan([gu.gemm_step((INPUT, 0), both, known and known[0]), step("xqt_b200_swiglu", (both, h), (ROWS, inter, native.DTYPE_CODE[self.dtype])),
+                           dn.gemm_step(h, (OUTPUT, 0), known and known[1])], rows=(CHUNKED_DECODE_MAX_ROWS + 1, MANY_ROWS), scratch=(0, 6 * inter)))
+        self._gemm = (state, self._bound(plans, static), known is not None)
         return self._gemm[1]
 
     def _one_entry_form(self) -> bool:

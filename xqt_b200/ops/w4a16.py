@@ -72,6 +72,12 @@ def integer_zero_points_now(zero_points: torch.Tensor | None) -> bool | None:
     return _integer_zero_points(zero_points)
 
 
+def fused_preferred(m: int, n: int, k: int, padded_k: int, group_size: int) -> bool:
+    """Whether ``variant="auto"`` takes the single-pass GEMM where the zero points are integers (else it need not know)."""
+
+    return bool(native.library().xqt_b200_w4a16_fused_preferred(m, n, k, padded_k, group_size))
+
+
 def select_variant(m: int, n: int, k: int, padded_k: int, group_size: int, activation: str = "none",
                    has_residual: bool = False) -> str:
     code = native.library().xqt_b200_w4a16_select_variant(
@@ -185,9 +191,9 @@ def w4a16_linear(
 
 
 def w4a16_step(source: tuple, qweight: torch.Tensor, scales: torch.Tensor, zero_points: torch.Tensor | None, bias32: torch.Tensor | None,
-               target: tuple, *, k: int, group_size: int, nibble_signed: bool, dtype: torch.dtype, integer: bool) -> tuple:
+               target: tuple, *, k: int, group_size: int, nibble_signed: bool, dtype: torch.dtype, integer: bool | None) -> tuple:
     """:func:`w4a16_linear` (``variant="auto"``, output in the activation dtype) of any number of rows as a step of a bound layer.
-    The tensors are what it takes unconverted; ``integer``: :func:`_integer_zero_points`."""
+    The tensors are what it takes unconverted; ``integer``: :func:`_integer_zero_points`, None where it is not known."""
 
     n, code = int(qweight.shape[0]), native.DTYPE_CODE[dtype]
     return step("xqt_b200_w4a16_run", (source, qweight, scales, zero_points, bias32, 0, target),
