@@ -230,7 +230,11 @@ struct WithoutGil {
 PyObject* call(PyObject* self, PyObject* const* args, size_t nargsf, PyObject* kwnames) {
   Bound* b = reinterpret_cast<Bound*>(self);
   const Py_ssize_t nargs = PyVectorcall_NARGS(nargsf);
-  auto slow = [&]() { return PyObject_Vectorcall(b->slow, args, nargsf, kwnames); };
+  auto slow = [&]() {
+    Py_INCREF(b->slow);                          // it may be replaced while it runs
+    THPObjectPtr held(b->slow);
+    return PyObject_Vectorcall(held.get(), args, nargsf, kwnames);
+  };
   if (kwnames != nullptr || nargs < 1 || nargs > 3 || !THPVariable_Check(args[0])) return slow();
   const at::Tensor& x = THPVariable_Unpack(args[0]);
   if (!plain(x, b->dtype, b->device) || c10::cuda::current_device() != b->device) return slow();
