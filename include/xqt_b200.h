@@ -302,7 +302,8 @@ int xqt_b200_quantize_per_tensor(const void* activation, void* codes, float* row
 /* W8A8 GEMM: output[m,n] = int32(sum_k a[m,k] w[n,k]) * act_scale[m] * weight_scale[n] (+ bias[n]).
  * Replaces xqt_convrot_w8a8_sm89_gemm / _small_gemm (convrot_w8a8_sm89_kernel.cu:506-755; the
  * Nunchaku main loop jit/include/nunchaku/gemm_w8a8.cuh:11-61).  act_codes int8 [M,K], weight_codes
- * int8 [N,K] (both K-major), K a multiple of 16, N a multiple of 8, output [M,N] out_dtype.
+ * int8 [N,K] (both K-major), K a multiple of 16, N a multiple of 8, output [M,N] out_dtype (16-byte aligned;
+ * scales and bias at any fp32 address).
  * workspace: at least 256 bytes, zero before first use (status word). */
 int xqt_b200_w8a8_gemm(const void* act_codes, const void* weight_codes, const float* act_scale,
                        const float* weight_scale, const float* bias, void* output, int m, int n,

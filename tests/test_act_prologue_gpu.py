@@ -99,3 +99,13 @@ def test_values_that_are_not_finite(m, k, rotation, mode, dtype):
         assert torch.equal(codes, want_codes)
         order = (lambda s: s.reshape(-1, k // 64, 128).permute(0, 2, 1).reshape(-1, k // 64)[:m]) if mode == 6 else (lambda s: s)
         assert torch.equal(order(scales), order(want_scales))        # no scale is NaN
+
+
+@pytest.mark.parametrize("k", [51200, 169984])             # the longest token of the separate kernels, and of the cluster form
+def test_longest_tokens(k):
+    lib, x = native.library(), (torch.randn((5, k), generator=seeded(k)) * 3).to(DEV, torch.bfloat16)
+    assert lib.xqt_b200_act_prologue_supported(k, 0, 0, 8) and not lib.xqt_b200_act_prologue_supported(169984 + 16, 0, 0, 8)
+    codes, scales = rotate_quantize(x, None, bits=8)
+    want_scales = x.float().abs().amax(dim=1) / torch.full((5,), 127.0, device=DEV)      # by a scalar, torch multiplies by its reciprocal
+    assert torch.equal(scales, want_scales)
+    assert torch.equal(codes, torch.round(x.float() / want_scales[:, None]).clamp(-128, 127).to(torch.int8))

@@ -64,8 +64,9 @@ def test_mlp_with_the_gating_in_the_epilogue(m, hidden, inter, group, dtype):
 
 # 160-column tiles of two token blocks (the narrowest that leave room for four stages only), in one wave, two waves and a
 # partial last tile; K short enough for the rings never to wrap, and long; token counts past 1000
-@pytest.mark.parametrize("m,n,k", [(300, 11008, 512), (512, 22016, 320), (512, 11000, 4096), (1024, 5120, 5120), (1024, 5112, 2304)])
-def test_tiles_of_160_columns(m, n, k):
+@pytest.mark.parametrize("m,n,k", [(300, 11008, 512), (512, 22016, 320), (512, 11000, 4096), (1024, 5120, 5120), (1024, 5112, 2304),
+                                   (2600, 4096, 6144)])             # and 256 columns, eleven chunks of which the last is ragged
+def test_wide_tiles_and_many_chunks(m, n, k):
     gen = seeded(m + n + k)
     pw = quantize.quantize_w4_asymmetric(torch.randn((n, k), generator=gen) * 0.02, group_size=64, param_dtype=torch.float16)
     weight = (pw.qweight.to(DEV), pw.scales.to(DEV), pw.zero_points.to(DEV))

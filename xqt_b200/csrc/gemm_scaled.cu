@@ -5,7 +5,8 @@
 //   pair (CG = 2)  persistent; the two CTAs of a cluster run 256 x tile_n tiles with cta_group::2 MMAs.  Each loads its 128
 //                  rows of A and half of the B rows, so a stage moves a quarter less through L2 than two single-CTA tiles of
 //                  the same area: at int8 rates (8192 multiply-adds per SM and clock) L2 -> SM bandwidth is what bounds
-//                  128 x 256 tiles (393 MB in 24 us for 2048 x 4096 x 4096).
+//                  128 x 256 tiles (393 MB in 24 us for 2048 x 4096 x 4096).  With pairs the tensor pipe is busy 52 % of a
+//                  cold launch, L2 32 %: the rest is the pipeline's ramp per tile and the last wave.
 //   single (CG = 1) one 128 x tile_n tile per CTA, its K range split over the CTAs of a cluster when the tiles alone leave
 //                  SMs idle: int32 partial sums are exact, so they meet in distributed shared memory in any order.  For few
 //                  tokens the layer is bound by streaming the weights, which takes as many SMs as possible.

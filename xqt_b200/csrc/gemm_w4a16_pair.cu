@@ -12,7 +12,7 @@
 // saves 7 %, its parameter loads 7 %), the tensor rate under the power cap, and the last wave.
 //
 // tile_n is a run-time multiple of 32 and K may be split: the plan takes the pair with the cheapest waves (28672 channels
-// are 1.51 waves of 256-wide tiles on 74 pairs, but 1.86 of 208-wide ones).  A split writes fp32 partial sums [split][M][N]
+// at 512 tokens are 1.51 waves of 256-wide tiles on 74 pairs, but 1.73 of 224-wide ones).  A split writes fp32 partial sums [split][M][N]
 // which a second kernel, on all SMs, adds in split order (bit-reproducible); letting the last CTA of a tile add them
 // took 128 threads of one SM 14 us for 512 KiB.
 //

@@ -100,11 +100,10 @@ __global__ void __launch_bounds__(256) dequant_w4_f16_kernel(const uint8_t* __re
   }
 }
 
-// From this M on the weights are dequantised once per call into an fp16 scratch and multiplied by the
-// dense tcgen05 GEMM.  Measured on the 4096 x 14336 MLP block the two passes beat the fused
-// single-pass kernel at every M above the decode range (261 vs 328 us at M = 64, 342 vs 474 us at
-// M = 512, 1250 vs 2560 us at M = 4096), so the default threshold is the first M the decode kernels do
-// not serve; the single-pass kernel stays reachable as its own variant (no N*K*2 scratch).
+// From this M on the two-pass form is available: weights dequantised once per call into an fp16 scratch (any zero point) and
+// multiplied by the dense tcgen05 GEMM.  The default is the first M the decode kernels do not serve.  Where the zero points
+// are integers the single-pass kernels are ahead of it up to 512 tokens and for large layers beyond: the figures are at
+// w4a16_gemm_fused_preferred.
 // XQT_B200_TWO_PASS_MIN_M in the environment moves the threshold (read once; tuning and tests).
 static int dense_min_m() {
   static int v = -1;
