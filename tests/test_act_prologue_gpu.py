@@ -38,13 +38,13 @@ def test_matches_the_separate_kernels(m, k, rotation, mode, dtype):
     want_la = 0.5 * rotated.float() @ down.float().t()
     # the MMA's fp32 sums of K exact products: the error of a sum of K terms in fp32 is below K * 2^-24 of the sum of magnitudes
     bound = 0.5 * k * 2.0 ** -24 * (rotated.float().abs() @ down.float().abs().t()) + 1e-30
-    for form, ready in ((0, 0), (1, 0), (2, 256), (3, 256), (0, 256)):       # column factors read after and before the wait
+    for form in (0, 1, 2, 3):
         codes = torch.full((m, k), 99, device=DEV, dtype=torch.int8)
         scales = torch.full_like(want_scales, -1.0)
         la = torch.zeros({0: (1,), 1: (m, 32), 2: (-(-m // 128) * 128, 32), 3: (m, 64)}[form], device=DEV, dtype=dtype if form == 3 else torch.float32)
         native.check(lib.xqt_b200_act_prologue(
             x.data_ptr(), native.ptr(column_scale), codes.data_ptr(), scales.data_ptr(), down.data_ptr() if form else 0, la.data_ptr() if form else 0,
-            0.5, m, k, kind | (ready if kind else 0), block, mode, form, native.DTYPE_CODE[dtype], native.stream_handle(DEV)), "xqt_b200_act_prologue")
+            0.5, m, k, kind, block, mode, form, native.DTYPE_CODE[dtype], native.stream_handle(DEV)), "xqt_b200_act_prologue")
         assert torch.equal(codes, want_codes)
         if mode == 6:                                      # tile-major: only the rows below M are written
             order = lambda s: s.reshape(-1, k // 64, 128).permute(0, 2, 1).reshape(-1, k // 64)[:m]
@@ -109,3 +109,20 @@ def test_longest_tokens(k):
     want_scales = x.float().abs().amax(dim=1) / torch.full((5,), 127.0, device=DEV)      # by a scalar, torch multiplies by its reciprocal
     assert torch.equal(scales, want_scales)
     assert torch.equal(codes, torch.round(x.float() / want_scales[:, None]).clamp(-128, 127).to(torch.int8))
+
+
+@pytest.mark.parametrize("m,k,rotation,mode", [(9, 768, "r256", 8), (600, 512, "s128", 8), (9, 768, "s32", 6), (1300, 512, "r64", 6)])
+def test_column_factors_read_before_and_after_the_wait(m, k, rotation, mode):
+    rot, dtype = ROTATIONS[rotation], torch.bfloat16
+    x, column_scale = torch.randn((m, k), generator=seeded(m)).to(DEV, dtype), _column_scale(rot, DEV)
+    down = torch.randn((32, k), generator=seeded(k)).to(DEV, dtype)
+    got = []
+    for ready in (0, 256):                                 # 256: XQT_B200_ROT_FACTORS_READY
+        codes, la = torch.full((m, k), 99, device=DEV, dtype=torch.int8), torch.zeros((m, 32), device=DEV)
+        scales = torch.zeros((m,) if mode == 8 else (-(-m // 128) * 128, k // 64), device=DEV)
+        native.check(native.library().xqt_b200_act_prologue(
+            x.data_ptr(), column_scale.data_ptr(), codes.data_ptr(), scales.data_ptr(), down.data_ptr(), la.data_ptr(), 1.0, m, k, _KIND[rot.kind] | ready,
+            rot.block, mode, 1, native.DTYPE_CODE[dtype], native.stream_handle(DEV)), "xqt_b200_act_prologue")
+        got.append((codes, scales, la))
+    assert all(torch.equal(a, b) for a, b in zip(*got))
+    assert torch.equal(got[0][0], rotate_quantize(x, rot, bits=4 if mode == 6 else 8, sign_magnitude=mode == 6, tiled_scales=mode == 6, return_rotated=True)[0])
